@@ -107,6 +107,19 @@ int ensure_geom(acu_ctx* c)
         CK(c, gs.lines_order.ensure(sizeof(int) * ord.size()));
         CK(c, cudaMemcpy(gs.lines_order.p, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
         gs.d.lines_order = gs.lines_order.template as<int>();
+        if (sizeof(Real) == 4) {
+            gs.h_mma = mma_angles(h.xsc_fp.data(), c->T);
+            CK(c, gs.mma.ensure(sizeof(MmaAngle) * gs.h_mma.size()));
+            CK(c, cudaMemcpy(gs.mma.p, gs.h_mma.data(), sizeof(MmaAngle) * gs.h_mma.size(), cudaMemcpyHostToDevice));
+            gs.d.mma = gs.mma.template as<MmaAngle>();
+            gs.d.h_mma = gs.h_mma.data();
+            gs.h_groups = mma_groups(gs.h_mma);
+            CK(c, gs.groups.ensure(sizeof(int) * gs.h_groups.size()));
+            CK(c, cudaMemcpy(gs.groups.p, gs.h_groups.data(), sizeof(int) * gs.h_groups.size(), cudaMemcpyHostToDevice));
+            gs.d.groups = gs.groups.template as<int>();
+            gs.d.h_groups = gs.h_groups.data();
+            gs.d.n_groups = (int)gs.h_groups.size() - 1;
+        }
     }
     gs.d.xsc_bp = gs.xsc_bp.template as<float4>();
     gs.hx_bp.resize(c->T);
@@ -163,12 +176,18 @@ enum OpKind { OP_IRADON, OP_RADON, OP_RADON_ADJ, OP_FILTER, OP_BACKPROJECT };
 
 // Runs one operator on plain-layout device arrays of S slices.
 // The single-precision 4-slice projector variant for G slice groups:
-// ACU_OPT_PROJECTOR, where 7 (automatic) takes the pixel-line projector (6)
-// when the groups fill their 8-group lines to 8/9 or more (its cost follows
-// the lines, the others' the groups), else variant 5.
+// ACU_OPT_PROJECTOR, where 7 (automatic) takes the tensor-core projector for
+// large batches at exact positions, else the pixel-line projector (6) when the
+// groups fill their 8-group lines to 8/9 or more (its cost follows the lines,
+// the others' the groups), else variant 5.
+constexpr int PROJ_MMA = 8, MMA_MIN_GROUPS = 7, MMA_MIN_SIDE = 200;
 int projector_variant(const acu_ctx* c, int G)
 {
     if (c->opt_projector != 7) return c->opt_projector;
+    // the tensor-core projector works on blocks of 64 slices, whatever part of one is filled.  Measured (ms, it / the
+    // better gather variant): 1025^2 x 600, 16 slices 9.6 / 6.6, 24 slices 9.6 / 10.0, 64 slices 9.6 / 23.4; 257^2 x
+    // 180, 20 slices 0.29 / 0.26, 32 slices 0.30 / 0.31; at 129^2 it gains nothing at any batch that fits a block
+    if (c->opt_positions == 1 && G >= MMA_MIN_GROUPS && c->N >= MMA_MIN_SIDE && mma_fits(c->N)) return PROJ_MMA;
     return 8 * ((G + 7) / 8) <= G + G / 8 ? 6 : 5;
 }
 
@@ -181,6 +200,11 @@ int ensure_projector_buffers(acu_ctx* c, int G)
     if (v == 0) {
         CK(c, c->pairP.ensure(sizeof(float) * 2 * nimg));
         CK(c, c->pairPT.ensure(sizeof(float) * 2 * nimg));
+    } else if (v == PROJ_MMA) {
+        const MmaPlan p = mma_plan(c->g32.d, G);
+        CK(c, c->mmaT.ensure(p.tile_bytes));
+        CK(c, c->mmaP.ensure(p.part_bytes));
+        CK(c, c->mmaF.ensure(2 * sizeof(int)));
     } else if (v == 6) {
         CK(c, c->lineL.ensure(sizeof(float) * lines_image_floats(c->N, G)));
         CK(c, c->lineA.ensure(sizeof(float) * lines_sums_floats(c->N, c->T, G)));
@@ -195,7 +219,10 @@ int ensure_projector_buffers(acu_ctx* c, int G)
 void radon_quads(acu_ctx* c, const DevGeom<float>& g, int G, const float* img, float* sino)
 {
     const int v = projector_variant(c, G);
-    if (v == 6)
+    if (v == PROJ_MMA)
+        launch_radon_mma(g, G, img, c->mmaT.as<unsigned char>(), c->mmaP.as<float>(), c->mmaF.as<int>(),
+                         mma_plan(g, G), sino, c->stream);
+    else if (v == 6)
         launch_radon_lines(g, G, img, c->lineL.as<float>(), c->lineA.as<float>(), sino, c->stream);
     else if (v >= 1)
         launch_radon_quads(g, G, img, c->pairPT.as<float>(), sino, c->stream, v == 2, v >= 3, v >= 4, v == 5);
@@ -490,12 +517,12 @@ int tv_iterate_v(acu_ctx* c, int nouter)
         // the key holds every device address the captured iteration uses
         // outside the solver state, so a work buffer that has grown since
         // (another call on a larger batch) forces a new capture
-        char key[400];
-        snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%p/%p/%p/%p/%p/%p", (int)sizeof(Real), V,
+        char key[480];
+        snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%p/%p/%p/%p/%p/%p/%p/%p/%p", (int)sizeof(Real), V,
                  s.G, s.ninner, s.ncg, s.lambda, s.mu, c->opt_filter, c->opt_projector, c->opt_positions,
                  c->opt_residual, c->g32.d.bp_tma * 100 + c->g32.d.bp_groups * 10 + c->g32.d.bp_param, s.uk.p, s.part.p, c->pairP.p,
-                 c->pairPT.p, c->lineL.p, c->lineA.p);
-        char key2[440];
+                 c->pairPT.p, c->lineL.p, c->lineA.p, c->mmaT.p, c->mmaP.p, c->mmaF.p);
+        char key2[520];
         snprintf(key2, sizeof key2, "%s/%d", key, c->opt_refresh);
         if (!s.graph || s.graph_key != key2) {
             for (cudaGraphExec_t* gx : {&s.graph, &s.graph_inc})
@@ -631,11 +658,12 @@ int tv_chunk(acu_ctx* c, int S, bool host_io)
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = 0;
     TvState<Real>& st = tvstate<Real>(c);
-    size_t held = c->pairP.n + c->pairPT.n + c->lineL.n + c->lineA.n + c->w_host_in.n + c->w_host_out.n;
+    size_t held = c->pairP.n + c->pairPT.n + c->lineL.n + c->lineA.n + c->mmaT.n + c->mmaP.n + c->w_host_in.n + c->w_host_out.n;
     for (const DevBuf* b : {&st.f, &st.fk, &st.ruk, &st.rp, &st.q, &st.uk, &st.ukp, &st.dx, &st.dy, &st.bx, &st.by,
                             &st.rhs, &st.r, &st.p, &st.Ap, &st.tmp, &st.bd, &st.dacc})
         held += b->n;
-    const size_t reserve = ((size_t)1 << 30) + totalb / 50;
+    // the tensor-core projector's partial sums do not grow with the batch
+    const size_t reserve = ((size_t)1 << 30) + totalb / 50 + (sizeof(Real) == 4 && c->opt_projector == 7 ? MMA_PART_CAP : 0);
     const size_t avail = freeb + held > reserve ? freeb + held - reserve : 0;
     long long smax = (long long)(avail / per);
     if (smax >= 4) smax -= smax % 4;

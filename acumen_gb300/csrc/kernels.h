@@ -15,6 +15,15 @@ struct BpTable {
     float4 v[BP_TMAX];
 };
 
+// One angle of the tensor-core projector (kernels_radon_mma.cu).
+struct MmaAngle {
+    float4 x;         // split sine and cosine, as xsc_fp
+    float c, s, t;    // cosine, sine, slope of a ray's closest approach
+    float reach;      // |c| + |s| and a margin: how far a pixel's taps reach across the rays
+    int nr, roff;     // rows (rays) of the angle's window in a tile, and the rows of the angles before it
+    int pad[2];
+};
+
 // Geometry of one reconstruction grid on the device, for one precision.
 // All tables are computed on the host (tables.cpp) with the reference's
 // arithmetic and uploaded once.
@@ -39,6 +48,11 @@ struct DevGeom {
     const float4* xsc_bp = nullptr;
     const float4* xsc_fp = nullptr;
     int exact = 0;
+    const MmaAngle* mma = nullptr;      // tensor-core projector's angles (single precision), and their host copy
+    const MmaAngle* h_mma = nullptr;
+    const int* groups = nullptr;        // first angles of its groups, n_groups + 1 of them, and their host copy
+    const int* h_groups = nullptr;
+    int n_groups = 0;
     const float4* h_xsc_bp = nullptr;   // host copy of xsc_bp (for the parameter table)
     const float4* h_sc_bp = nullptr;    // host copy of sc_bp as (sin, cos, 0, 0), single precision
     int bp_param = 1;                   // backprojection: angle table in the launch parameters when T <= BP_TMAX
@@ -72,6 +86,23 @@ size_t lines_sums_floats(int N, int T, int G);
 int lines_band_rows(int N);
 // The band launches' angle order for single-precision (sin, cos) pairs sc[2T].
 std::vector<int> lines_angle_order(const float* sc, int T);
+// Projector on the tensor cores (kernels_radon_mma.cu; exact positions):
+// 64-slice blocks of 16 x 16 pixel tiles in operand layout, partial sums of a
+// chunk of angles, two flags (not finite; a wait gave up).
+struct MmaPlan {
+    int nt = 0;        // tiles per side
+    int nblk = 0;      // 64-slice blocks of the batch
+    int nb = 0;        // of them at once
+    int ng = 0;        // groups of angles at once
+    size_t tile_bytes = 0, part_bytes = 0;
+};
+constexpr size_t MMA_PART_CAP = (size_t)4 << 30;   // bytes of partial sums at once
+std::vector<MmaAngle> mma_angles(const float* xsc, int T);
+bool mma_fits(int N);
+std::vector<int> mma_groups(const std::vector<MmaAngle>& ang);
+MmaPlan mma_plan(const DevGeom<float>& g, int G);
+void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned char* tiles, float* P, int* flags,
+                      const MmaPlan& p, float* sino, cudaStream_t st);
 // The staggered projector for one slice per thread (plain layout); IT is a
 // work buffer of N * N floats per slice.
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);

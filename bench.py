@@ -58,6 +58,34 @@ def projector_variant(option, S):
     return 6 if 8 * ((G + 7) // 8) <= G + G // 8 else 5
 
 
+def tensor_projector(option, positions, S, N):
+    """Whether the library projects on the tensor cores (csrc/api.cu projector_variant)."""
+    return option == 7 and positions == 1 and (S + 3) // 4 >= 7 and 200 <= N <= 4096
+
+
+def tensor_radon_launches(N, theta, S):
+    """Kernels of one projection on the tensor cores (csrc/kernels_radon_mma.cu
+    mma_plan): per pass over slice blocks one layout kernel, per chunk of angle
+    groups a product and a reduction, and the flagged fallback."""
+    import numpy as np
+    c = np.pi * (np.asarray(theta, np.float64) - 90.0) / 180.0
+    nr = np.minimum(25, np.floor(17.0 * (np.abs(np.cos(c)) + np.abs(np.sin(c))) + 0.002).astype(int) + 1)
+    groups, t = [], 0
+    while t < len(nr):
+        n = min(5, len(nr) - t)
+        n = 4 if n == 5 and nr[t + 4] > 24 else n
+        groups.append(int(nr[t:t + n].sum()))
+        t += n
+    row, cap, nblk = ((N + 15) // 16) ** 2 * 256, 4 << 30, (S + 63) // 64
+    nb, ng, total = min(nblk, 2), len(groups), row * sum(groups)
+    if total * nb <= cap:
+        nb = min(nblk, cap // total)
+        nb = nb & ~1 if nb > 2 else nb
+    else:
+        ng = max(1, cap // (row * 125 * nb))
+    return 1 + -(-nblk // nb) * (1 + 2 * -(-len(groups) // ng))
+
+
 def radon_launches(variant, N):
     """Kernels of one batched projection: line conversion, one launch per
     band of rows and the finish for the pixel-line projector (csrc/kernels_lines.cu
@@ -773,7 +801,8 @@ def main():
     n_ew += NINNER * NCG if carried else 0          # the sinogram updates ruk += alpha radon(p)
     n_ew += 1 if carried_res else 0                 # iradon(fk - f) += iradon(f - radon(uk))
     variant = projector_variant(t.get_option(7), S)
-    per_radon = radon_launches(variant, N)
+    tensor = tensor_projector(t.get_option(7), t.get_option(8), S, N)
+    per_radon = tensor_radon_launches(N, t.theta, S) if tensor else radon_launches(variant, N)
     kernel_launches = (per_radon * n_radon + 2 * n_iradon + n_ew) * args.steps + per_radon * n_full
     if carried_res:   # each refresh: two differences and two backprojections instead of the sum
         kernel_launches += n_full * (2 * 2 + 2 - 1)
@@ -823,17 +852,20 @@ def main():
         achieved = alg_bytes / t_radon / 1e9
         line_groups = ((S + 3) // 4 + 7) // 8
         traffic = (RADON_TRAFFIC_PER_LINE_GROUP * line_groups
-                   if (N, T) == (N_GRID, T_ANG) and variant == 6 and RADON_TRAFFIC_PER_LINE_GROUP else None)
-        kname = ("k_radon_lines (pixel lines of 32 slices, %d band launches + conversions; projector, "
+                   if (N, T) == (N_GRID, T_ANG) and variant == 6 and not tensor else None)
+        kname = ("k_mma_project + k_mma_reduce (partial sums of 16 x 16 tiles on the tensor cores; projector, "
+                 "tv_hpc.F90:137-156)" if tensor else
+                 "k_radon_lines (pixel lines of 32 slices, %d band launches + conversions; projector, "
                  "tv_hpc.F90:137-156)" % (radon_launches(6, N) - 2) if variant == 6 else
                  "k_radon_stag_reuse<4, exact, f32x2> (projector, tv_hpc.F90:137-156)")
         line["roofline"] = {"bound": "hbm", "kernel": kname,
                             "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                             "peak_kind": kind, "traffic": traffic,
                             "algorithmic_bytes": alg_bytes, "launch_ms": 1000 * t_radon,
-                            "note": "runs from L2 and L1, not from HBM (each band of rows stays in L2); traffic (from "
-                                    "one 32-slice ncu capture, scaled by 32-slice line groups) is mostly the ray "
-                                    "sums carried between the band launches, ~1.4 % of the HBM bandwidth",
+                            "note": "tensor cores: ~1.76 KB of partial sums written and read per tile, angle and 20 "
+                                    "rays of 64 slices; gather variants: runs from L2 and L1, traffic (from one "
+                                    "32-slice ncu capture, scaled by 32-slice line groups) is mostly the ray sums "
+                                    "carried between the band launches",
                             "l1_level": l1_level(16.0 * N * N * T * S / t_radon / 1e9, clocks, probe,
                                                  bytes_per_sample_slice=16,
                                                  sample_slices_per_s=N * N * T * S / t_radon)}

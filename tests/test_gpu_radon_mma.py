@@ -1,0 +1,117 @@
+"""The projector on the tensor cores (automatic from 25 slices and a side of 200
+on, exact positions) against the gather projector (variant 5) and the FP64
+oracle.
+
+Both round each sum to single precision in another order; a sum of up to 3 N
+terms of one sign stays within ~1e-6 of FP64 either way (the bar of
+test_operators_at_the_2049_grid is 5e-6), so they agree to 3e-6 in relative L2.
+"""
+import numpy as np
+import pytest
+import torch
+
+from acumen_gb300 import synthetic as syn
+from acumen_gb300.tomography import Tomography
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+def axes(T):
+    """Angles on and near the axes and the diagonals (25-row windows) among evenly spread ones."""
+    near = [0.0, 45.0, 90.0, 135.0, 180.0, 44.0, 46.5, 89.9999, 90.0001, 1e-5, 134.2]
+    return np.concatenate([syn.angles(max(T - len(near), 1)), near])[:max(T, 1)].astype(np.float32)
+
+
+def both(N, th, x):
+    t = Tomography(N, th, max(4, N // 20))
+    got = t.radon(x)
+    t.set_option(7, 5)
+    ref = t.radon(x)
+    t.close()
+    return got, ref
+
+
+# sides at and around multiples of the 16-pixel tile; slices at the rule's lower end and around blocks of 64 and pairs
+# of them; angle counts that leave a group of five partly filled
+@pytest.mark.parametrize("N, T, S", [(200, 12, 25), (208, 31, 64), (209, 33, 65), (223, 1, 128), (257, 40, 130),
+                                     (224, 13, 200)])
+def test_matches_the_gather_projector(N, T, S):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    th = axes(T) if T > 11 else np.array([33.3], np.float32)
+    for x in (torch.rand(S, N, N, device="cuda", generator=g), torch.randn(S, N, N, device="cuda", generator=g)):
+        got, ref = both(N, th, x)
+        assert not torch.equal(got, ref)     # the other path did run
+        assert rel(got, ref) < 3e-6
+
+
+def test_several_chunks_of_angles_and_same_result_twice():
+    """Partial sums of 120 angles of two 64-slice blocks exceed what is held at once."""
+    N, T, S = 1025, 120, 128
+    x = torch.rand(S, N, N, device="cuda")
+    t = Tomography(N, syn.angles(T), 50)
+    got = t.radon(x)
+    assert torch.equal(got, t.radon(x))
+    t.set_option(7, 6)
+    assert rel(got, t.radon(x)) < 3e-6
+    t.close()
+
+
+def test_against_fp64(oracle, built_lib):
+    N, T, S = 225, 40, 32
+    th = (syn.angles(T) + 0.21).astype(np.float32)
+    x = np.random.default_rng(5).random((S, N, N), dtype=np.float32)
+    got, ref = both(N, th, torch.from_numpy(x).cuda())
+    o = torch.from_numpy(oracle.radon(x[:2].astype(np.float64), th, 64))
+    assert rel(got[:2].cpu(), o) < 1e-6
+
+
+def test_scales_of_slices_and_tiles():
+    """Every tile of a slice has its own power-of-two scale: slices and regions of very different magnitude."""
+    N, T, S = 209, 20, 32
+    x = torch.rand(S, N, N, device="cuda")
+    x[0] *= 1e30
+    x[1] *= 1e-30
+    x[2, :100] *= 1e6
+    x[3] = 0
+    x[4] = 0
+    x[4, 77, 99] = 1e-20
+    got, ref = both(N, axes(T), x)
+    for s in range(6):
+        assert torch.isfinite(got[s]).all()
+        scale = float(ref[s].abs().max())
+        assert rel(got[s] / max(scale, 1e-38), ref[s] / max(scale, 1e-38)) < 3e-6 if s != 3 else not got[s].any()
+
+
+def test_values_that_are_not_finite_stay_on_their_rays():
+    """A matrix product would spread a NaN or infinity over its tile: such a call takes plain gathers."""
+    N, T, S = 209, 20, 32
+    x = torch.rand(S, N, N, device="cuda")
+    x[1, 100, 60] = float("nan")
+    x[2, 30, 150] = float("inf")
+    x[2, 31, 150] = float("-inf")
+    got, ref = both(N, axes(T), x)
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+    m = torch.isfinite(ref)
+    assert rel(got[m], ref[m]) < 3e-6
+
+
+def test_in_the_solver():
+    """TV of a batch with the tensor-core projector against the gather projector, through a captured graph."""
+    N, T, S = 209, 60, 32
+    th = syn.angles(T)
+    f = torch.stack([syn.normalised_sinogram(syn.random_ellipses(s, 0.3 * N), N, th, I0=5e3, seed=s, device="cuda")
+                     for s in range(S)])
+    t = Tomography(N, th, 10)
+    tv, _ = t.tvopt(f, 1, 3, 4, 0.05, 1.0)
+    t.set_option(3, 0)
+    tv_l, _ = t.tvopt(f, 1, 3, 4, 0.05, 1.0)
+    assert torch.equal(tv, tv_l)             # graph and launches
+    t.set_option(7, 5)
+    ref, _ = t.tvopt(f, 1, 3, 4, 0.05, 1.0)
+    mask = t.backproject(torch.ones(1, T, N, device="cuda"))[0] != 0
+    assert rel(tv[:, mask], ref[:, mask]) < 2e-5
+    t.close()
