@@ -119,6 +119,12 @@ int ensure_geom(acu_ctx* c)
             gs.d.groups = gs.groups.template as<int>();
             gs.d.h_groups = gs.h_groups.data();
             gs.d.n_groups = (int)gs.h_groups.size() - 1;
+            const std::vector<float> mask(h.cmask.begin(), h.cmask.end());
+            std::vector<int> tiles;
+            gs.d.n_tiles_in = bp_tiles(mask.data(), c->N, tiles);
+            CK(c, gs.tiles_in.ensure(sizeof(int) * tiles.size()));
+            CK(c, cudaMemcpy(gs.tiles_in.p, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice));
+            gs.d.tiles_in = gs.tiles_in.template as<int>();
         }
     }
     gs.d.xsc_bp = gs.xsc_bp.template as<float4>();
@@ -165,11 +171,41 @@ void lanes_filter(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* in, Rea
         launch_filter_direct<Real, V>(g, G, in, out, c->stream);
 }
 
+// Whether G groups are backprojected on the tensor cores (blocks of 64 slices,
+// whatever part of one is filled).  Measured (ms, there / gathers): 725^2 x 360,
+// 32 slices 1.36 / 1.28, 40 slices 1.38 / 1.63; 1025^2 x 600, 36 slices 3.99 /
+// 4.64, 64 slices 4.09 / 8.18; 257^2 x 180, 48 slices 0.18 / 0.19; 129^2 x 90,
+// 128 slices 0.12 / 0.09.
+constexpr int BP_MMA_MIN_GROUPS = 10, BP_MMA_MIN_SIDE = 200;
+bool bp_mma(const acu_ctx* c, int G)
+{
+    return c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma && G >= BP_MMA_MIN_GROUPS &&
+           c->N >= BP_MMA_MIN_SIDE;
+}
+
+// Work buffers of the single-precision backprojection of G 4-slice groups (grow-only).
+int ensure_backproject_buffers(acu_ctx* c, int G)
+{
+    if (!bp_mma(c, G)) return ACU_OK;
+    CK(c, c->bpQ.ensure(bp_mma_bins_bytes(c->N, c->T, G)));
+    CK(c, c->bpS.ensure(sizeof(unsigned) * bp_mma_scalars(G)));
+    return ACU_OK;
+}
+
+template <typename Real, int V>
+void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q, Real* img)
+{
+    if constexpr (V == 4 && sizeof(Real) == 4) {
+        if (bp_mma(c, G) && launch_backproject_mma(g, G, q, c->bpQ.p, c->bpS.as<unsigned>(), img, c->stream)) return;
+    }
+    launch_backproject<Real, V>(g, G, q, img, c->stream);
+}
+
 template <typename Real, int V>
 void lanes_iradon(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* sino, Real* q, Real* img)
 {
     lanes_filter<Real, V>(c, g, G, sino, q);
-    launch_backproject<Real, V>(g, G, q, img, c->stream);
+    lanes_backproject<Real, V>(c, g, G, q, img);
 }
 
 enum OpKind { OP_IRADON, OP_RADON, OP_RADON_ADJ, OP_FILTER, OP_BACKPROJECT };
@@ -252,6 +288,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     }
     switch (op) {
     case OP_IRADON:
+        if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
         CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * V));
         lanes_iradon<Real, V>(c, g, G, lin, c->w_q.template as<Real>(), lout);
         break;
@@ -268,7 +305,10 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
         break;
     case OP_RADON_ADJ: launch_radon_adjoint<Real, V>(g, G, lin, lout, c->stream); break;
     case OP_FILTER: lanes_filter<Real, V>(c, g, G, lin, lout); break;
-    case OP_BACKPROJECT: launch_backproject<Real, V>(g, G, lin, lout, c->stream); break;
+    case OP_BACKPROJECT:
+        if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
+        lanes_backproject<Real, V>(c, g, G, lin, lout);
+        break;
     }
     CKLAUNCH(c);
     if constexpr (V > 1) {
@@ -454,6 +494,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     if (c->opt_verbose) CK(c, s.ukp.ensure(sizeof(Real) * nimg));
     if constexpr (V == 4 && sizeof(Real) == 4) {
         CKRET(ensure_projector_buffers(c, G));
+        CKRET(ensure_backproject_buffers(c, G));
     } else if constexpr (sizeof(Real) == 4) {
         CK(c, c->pairPT.ensure(sizeof(float) * nimg));
     }
@@ -503,7 +544,10 @@ int tv_iterate_v(acu_ctx* c, int nouter)
     const int S = s.S, Sp = s.G * V;
     const bool use_graph = c->opt_graph != 0 && !run.verbose;
     // the projector option may have changed since acu_tv_begin
-    if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_projector_buffers(c, s.G));
+    if constexpr (V == 4 && sizeof(Real) == 4) {
+        CKRET(ensure_projector_buffers(c, s.G));
+        CKRET(ensure_backproject_buffers(c, s.G));
+    }
     // the residual options may have changed too: the carried backprojections
     // start from the current iterate, and lapse when not carried
     if (run.carried && !s.carried_valid) {
@@ -517,12 +561,13 @@ int tv_iterate_v(acu_ctx* c, int nouter)
         // the key holds every device address the captured iteration uses
         // outside the solver state, so a work buffer that has grown since
         // (another call on a larger batch) forces a new capture
-        char key[480];
-        snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%p/%p/%p/%p/%p/%p/%p/%p/%p", (int)sizeof(Real), V,
+        char key[560];
+        snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p", (int)sizeof(Real), V,
                  s.G, s.ninner, s.ncg, s.lambda, s.mu, c->opt_filter, c->opt_projector, c->opt_positions,
                  c->opt_residual, c->g32.d.bp_tma * 100 + c->g32.d.bp_groups * 10 + c->g32.d.bp_param, s.uk.p, s.part.p, c->pairP.p,
-                 c->pairPT.p, c->lineL.p, c->lineA.p, c->mmaT.p, c->mmaP.p, c->mmaF.p);
-        char key2[520];
+                 c->pairPT.p, c->lineL.p, c->lineA.p, c->mmaT.p, c->mmaP.p, c->mmaF.p, c->bpQ.p,
+                 c->bpS.p);
+        char key2[600];
         snprintf(key2, sizeof key2, "%s/%d", key, c->opt_refresh);
         if (!s.graph || s.graph_key != key2) {
             for (cudaGraphExec_t* gx : {&s.graph, &s.graph_inc})
@@ -658,12 +703,13 @@ int tv_chunk(acu_ctx* c, int S, bool host_io)
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = 0;
     TvState<Real>& st = tvstate<Real>(c);
-    size_t held = c->pairP.n + c->pairPT.n + c->lineL.n + c->lineA.n + c->mmaT.n + c->mmaP.n + c->w_host_in.n + c->w_host_out.n;
+    size_t held = c->pairP.n + c->pairPT.n + c->lineL.n + c->lineA.n + c->mmaT.n + c->mmaP.n + c->bpQ.n + c->w_host_in.n + c->w_host_out.n;
     for (const DevBuf* b : {&st.f, &st.fk, &st.ruk, &st.rp, &st.q, &st.uk, &st.ukp, &st.dx, &st.dy, &st.bx, &st.by,
                             &st.rhs, &st.r, &st.p, &st.Ap, &st.tmp, &st.bd, &st.dacc})
         held += b->n;
-    // the tensor-core projector's partial sums do not grow with the batch
-    const size_t reserve = ((size_t)1 << 30) + totalb / 50 + (sizeof(Real) == 4 && c->opt_projector == 7 ? MMA_PART_CAP : 0);
+    // the tensor-core operators' partial sums and bins (of 128 slices) do not grow with the batch
+    size_t reserve = ((size_t)1 << 30) + totalb / 50;
+    if (sizeof(Real) == 4) reserve += (c->opt_projector == 7 ? MMA_PART_CAP : 0) + sizeof(float) * 128 * T * N;
     const size_t avail = freeb + held > reserve ? freeb + held - reserve : 0;
     long long smax = (long long)(avail / per);
     if (smax >= 4) smax -= smax % 4;

@@ -49,7 +49,7 @@ struct DevBuf {
 template <typename Real>
 struct GeomSet {
     bool ready = false;
-    DevBuf sc_bp, sc_fp, filt, cmask, fft_h, fft_h_x, fft_tw, fft_tw16, fp_order, lines_order, xsc_bp, xsc_fp, mma, groups;
+    DevBuf sc_bp, sc_fp, filt, cmask, fft_h, fft_h_x, fft_tw, fft_tw16, fp_order, lines_order, xsc_bp, xsc_fp, mma, groups, tiles_in;
     std::vector<MmaAngle> h_mma;
     std::vector<int> h_groups;
     std::vector<float4> hx_bp;   // host copy of xsc_bp
@@ -109,6 +109,7 @@ struct acu_ctx {
     acu::DevBuf pairP, pairPT;   // pair images of the single-precision projector
     acu::DevBuf lineL, lineA;    // line image and ray sums of projector variant 6
     acu::DevBuf mmaT, mmaP, mmaF; // tiles, partial sums and flags of the tensor-core projector
+    acu::DevBuf bpQ, bpS;         // bins in operand layout and per-slice scalars of the tensor-core backprojection
     acu::DevBuf w_part;          // FP64 / int64 partial sums of the preprocessing reductions
     acu::TvState<float> tv32;
     acu::TvState<double> tv64;

@@ -53,6 +53,8 @@ struct DevGeom {
     const int* groups = nullptr;        // first angles of its groups, n_groups + 1 of them, and their host copy
     const int* h_groups = nullptr;
     int n_groups = 0;
+    const int* tiles_in = nullptr;      // 16 x 16 pixel tiles that meet the mask (n_tiles_in), then the others
+    int n_tiles_in = 0;
     const float4* h_xsc_bp = nullptr;   // host copy of xsc_bp (for the parameter table)
     const float4* h_sc_bp = nullptr;    // host copy of sc_bp as (sin, cos, 0, 0), single precision
     int bp_param = 1;                   // backprojection: angle table in the launch parameters when T <= BP_TMAX
@@ -103,6 +105,14 @@ std::vector<int> mma_groups(const std::vector<MmaAngle>& ang);
 MmaPlan mma_plan(const DevGeom<float>& g, int G);
 void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned char* tiles, float* P, int* flags,
                       const MmaPlan& p, float* sino, cudaStream_t st);
+// Backprojection on the tensor cores (kernels_bp_mma.cu; exact positions): work
+// buffers of bp_mma_bins_bytes bytes and bp_mma_scalars words.  False if the
+// driver has no tensor maps (nothing usable was written).
+int bp_tiles(const float* cmask, int N, std::vector<int>& list);
+size_t bp_mma_bins_bytes(int N, int T, int G);
+size_t bp_mma_scalars(int G);
+bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
+                            cudaStream_t st);
 // The staggered projector for one slice per thread (plain layout); IT is a
 // work buffer of N * N floats per slice.
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);

@@ -81,6 +81,19 @@ __device__ __forceinline__ void tmem_ld_wait(float2 (&v)[4], float2 (&x)[4])
                    "+f"(x[3].x), "+f"(x[3].y)::"memory");
 }
 
+__device__ __forceinline__ void tmem_ld_wait(float2 (&v)[4])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[3].x),
+                   "+f"(v[3].y)::"memory");
+}
+
+// registers a thread of this warpgroup may use from here on
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---- mbarriers --------------------------------------------------------------
 __device__ __forceinline__ void bar_init(uint64_t* b, int count)
 {
@@ -149,6 +162,15 @@ __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t 
                  "r"(bytes)
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// box of a 3-d tensor map at (c0, c1, c2); c0 times the element size is a multiple of 16 bytes
+__device__ __forceinline__ void tensor_load_3d(void* dst, const void* map, int c0, int c1, int c2, uint64_t* bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];" ::"r"(smem_addr(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(bar))
+        : "memory");
 }
 // an empty group, so that groups stay in step
 __device__ __forceinline__ void bulk_store_none() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }

@@ -86,6 +86,16 @@ def tensor_radon_launches(N, theta, S):
     return 1 + -(-nblk // nb) * (1 + 2 * -(-len(groups) // ng))
 
 
+def iradon_launches(positions, S, N):
+    """Kernels of one filtered backprojection: the filter, then the gather
+    kernel, or on the tensor cores (csrc/kernels_bp_mma.cu) the largest
+    magnitudes, layout and product per pass of up to 128 slices, the tiles
+    outside the mask and the flagged fallback."""
+    if positions != 1 or (S + 3) // 4 < 10 or N < 200:
+        return 2
+    return 1 + 1 + 2 * -(-S // 128) + 2
+
+
 def radon_launches(variant, N):
     """Kernels of one batched projection: line conversion, one launch per
     band of rows and the finish for the pixel-line projector (csrc/kernels_lines.cu
@@ -803,9 +813,10 @@ def main():
     variant = projector_variant(t.get_option(7), S)
     tensor = tensor_projector(t.get_option(7), t.get_option(8), S, N)
     per_radon = tensor_radon_launches(N, t.theta, S) if tensor else radon_launches(variant, N)
-    kernel_launches = (per_radon * n_radon + 2 * n_iradon + n_ew) * args.steps + per_radon * n_full
+    per_iradon = iradon_launches(t.get_option(8), S, N)
+    kernel_launches = (per_radon * n_radon + per_iradon * n_iradon + n_ew) * args.steps + per_radon * n_full
     if carried_res:   # each refresh: two differences and two backprojections instead of the sum
-        kernel_launches += n_full * (2 * 2 + 2 - 1)
+        kernel_launches += n_full * (2 * per_iradon + 2 - 1)
 
     # solver state: 10 image-sized and 5 sinogram-sized FP32 arrays per slice
     state_gb = S * (10 * N * N + 5 * T * N) * 4 / 1e9
@@ -913,12 +924,12 @@ def main():
         # the other hot kernel: the backprojection (8 bytes per update at L1 level)
         t_bp = cuda_time(lambda: t.backproject(f), 2)
         line["roofline_backprojection"] = {
-            "kernel": "k_backproject_exact_ct<4, 1> (tv_hpc.F90:107-123)", "launch_ms": 1000 * t_bp,
+            "kernel": ("k_bp_mma (tensor cores" if iradon_launches(t.get_option(8), S, N) > 2 else
+                       "k_backproject_exact_ct<4, 1> (gathers") + "; tv_hpc.F90:107-123)", "launch_ms": 1000 * t_bp,
             "updates_per_s": N * N * T * S / t_bp,
             "l1_level": l1_level(8.0 * N * N * T * S / t_bp / 1e9, clocks, probe, bytes_per_update=8),
-            "note": "neighbouring pixels' taps often fall in the same bins and are broadcast within a "
-                    "quarter-warp, so bytes delivered to registers can exceed the data path's 128 B/clk; "
-                    "ncu: 84 % of L1 data-pipe wavefronts, 73 % issue; launch includes the lane-layout "
+            "note": "8 bytes per update at L1 level is the gather kernel's unit; on the tensor cores the bins are "
+                    "read once per 256 pixels (profiles/ has both); launch includes the lane-layout "
                     "conversions"}
         # ragged batch: 64 problems, grids {363,725,1449,2173,2897},
         # 180-1500 angles; one outer iteration timed as [tvopt(6) - tvopt(1)] / 5

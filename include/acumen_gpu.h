@@ -85,10 +85,12 @@ int acu_set_stream(acu_ctx *ctx, void *cuda_stream);
                                  Bregman updates and recomputed with radon(uk) every ACU_OPT_RADON_REFRESH
                                  outer iterations (default; as 1 when radon(uk) is not carried),
                                  1 one backprojection of fk - radon(uk), or 0 the reference's two */
-#define ACU_OPT_BP_GROUPS 10  /* 4-slice groups per backprojection thread: 0 auto (default: 1 with the
-                                 angle table in the launch parameters, else 2 where the groups divide),
-                                 1, 2 or 4; the groups share the angle's table entry and sample
-                                 position, the sums are unchanged */
+#define ACU_OPT_BP_GROUPS 10  /* 4-slice groups per backprojection thread: 0 auto (default: exact positions,
+                                 37 slices or more and a side of 200 or more on the tensor cores, the
+                                 same sums to single-precision rounding; else 1 with the angle table in
+                                 the launch parameters, else 2 where the groups divide), 1, 2 or 4; the
+                                 groups share the angle's table entry and sample position, the sums are
+                                 the same for 1, 2 and 4 */
 #define ACU_OPT_RADON_REFRESH 11 /* batched TV: radon(uk) for the Bregman update recomputed every outer
                                  iteration (1, the reference), or carried through the CG updates
                                  (radon(uk + a p) = radon(uk) + a radon(p)) and recomputed every K-th
