@@ -49,85 +49,74 @@ int ensure_geom(acu_ctx* c)
     if (c->N <= 0) return set_err(c, ACU_ERR_INVALID, "context has no reconstruction grid (nimage = 0)");
     HostTables<Real> h;
     make_tables<Real>(c->N, c->T, c->theta.data(), c->wpu, h);
-    CK(c, gs.sc_bp.ensure(sizeof(Real) * h.sc_bp.size()));
-    CK(c, gs.sc_fp.ensure(sizeof(Real) * h.sc_fp.size()));
-    CK(c, gs.filt.ensure(sizeof(Real) * (h.filt.size() + 8)));
     CK(c, gs.cmask.ensure(sizeof(Real) * h.cmask.size()));
-    CK(c, gs.fft_h.ensure(sizeof(Real) * h.fft_h.size()));
-    CK(c, gs.fft_h_x.ensure(sizeof(Real) * h.fft_h_x.size()));
-    std::vector<float> tw32(h.fft_tw.begin(), h.fft_tw.end());
-    CK(c, gs.fft_tw.ensure(sizeof(double) * h.fft_tw.size()));
-    CK(c, cudaMemcpy(gs.sc_bp.p, h.sc_bp.data(), sizeof(Real) * h.sc_bp.size(), cudaMemcpyHostToDevice));
-    CK(c, cudaMemcpy(gs.sc_fp.p, h.sc_fp.data(), sizeof(Real) * h.sc_fp.size(), cudaMemcpyHostToDevice));
-    CK(c, gs.xsc_bp.ensure(sizeof(float) * h.xsc_bp.size()));
-    CK(c, gs.xsc_fp.ensure(sizeof(float) * h.xsc_fp.size()));
-    CK(c, cudaMemcpy(gs.xsc_bp.p, h.xsc_bp.data(), sizeof(float) * h.xsc_bp.size(), cudaMemcpyHostToDevice));
-    CK(c, cudaMemcpy(gs.xsc_fp.p, h.xsc_fp.data(), sizeof(float) * h.xsc_fp.size(), cudaMemcpyHostToDevice));
-    CK(c, cudaMemset(gs.filt.p, 0, sizeof(Real) * (h.filt.size() + 8)));
-    CK(c, cudaMemcpy(gs.filt.p, h.filt.data(), sizeof(Real) * h.filt.size(), cudaMemcpyHostToDevice));
     CK(c, cudaMemcpy(gs.cmask.p, h.cmask.data(), sizeof(Real) * h.cmask.size(), cudaMemcpyHostToDevice));
-    CK(c, cudaMemcpy(gs.fft_h.p, h.fft_h.data(), sizeof(Real) * h.fft_h.size(), cudaMemcpyHostToDevice));
-    CK(c, cudaMemcpy(gs.fft_h_x.p, h.fft_h_x.data(), sizeof(Real) * h.fft_h_x.size(), cudaMemcpyHostToDevice));
-    if (sizeof(Real) == 4)
-        CK(c, cudaMemcpy(gs.fft_tw.p, tw32.data(), sizeof(float) * tw32.size(), cudaMemcpyHostToDevice));
-    else
-        CK(c, cudaMemcpy(gs.fft_tw.p, h.fft_tw.data(), sizeof(double) * h.fft_tw.size(), cudaMemcpyHostToDevice));
     gs.d.N = c->N;
     gs.d.T = c->T;
     gs.d.mid = h.mid;
-    gs.d.sc_bp = gs.sc_bp.template as<Real>();
-    gs.d.sc_fp = gs.sc_fp.template as<Real>();
-    gs.d.filt = gs.filt.template as<Real>();
     gs.d.cmask = gs.cmask.template as<Real>();
-    gs.d.fft_h = gs.fft_h.template as<Real>();
-    gs.d.fft_h_x = gs.fft_h_x.template as<Real>();
-    if (sizeof(Real) == 4 && !h.fft_tw16.empty()) {
-        const std::vector<float> t16(h.fft_tw16.begin(), h.fft_tw16.end());
-        CK(c, gs.fft_tw16.ensure(sizeof(float) * t16.size()));
-        CK(c, cudaMemcpy(gs.fft_tw16.p, t16.data(), sizeof(float) * t16.size(), cudaMemcpyHostToDevice));
-        gs.d.fft_tw16 = gs.fft_tw16.template as<float2>();
-    }
-    gs.d.fft_tw = gs.fft_tw.template as<float2>();
-    gs.d.fft_tw64 = gs.fft_tw.template as<double2>();
-    {
-        // angle order of the pair projector: angles read through the x-pair
-        // image (|sin| >= |cos|) first, then the transposed ones
-        std::vector<int> ord;
-        for (int pass = 0; pass < 2; ++pass)
-            for (int t = 0; t < c->T; ++t) {
-                const bool tr = std::fabs((double)h.sc_fp[2 * t + 1]) > std::fabs((double)h.sc_fp[2 * t]);
-                if (tr == (pass == 1)) ord.push_back(t);
-            }
-        CK(c, gs.fp_order.ensure(sizeof(int) * ord.size()));
-        CK(c, cudaMemcpy(gs.fp_order.p, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
-        gs.d.fp_order = gs.fp_order.template as<int>();
-        // projector variant 6: chunks of neighbouring angles, longest blocks first
-        const std::vector<float> s32(h.sc_fp.begin(), h.sc_fp.end());
-        ord = lines_angle_order(s32.data(), c->T);
-        CK(c, gs.lines_order.ensure(sizeof(int) * ord.size()));
-        CK(c, cudaMemcpy(gs.lines_order.p, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
-        gs.d.lines_order = gs.lines_order.template as<int>();
-        if (sizeof(Real) == 4) {
-            gs.h_mma = mma_angles(h.xsc_fp.data(), c->T);
-            CK(c, gs.mma.ensure(sizeof(MmaAngle) * gs.h_mma.size()));
-            CK(c, cudaMemcpy(gs.mma.p, gs.h_mma.data(), sizeof(MmaAngle) * gs.h_mma.size(), cudaMemcpyHostToDevice));
-            gs.d.mma = gs.mma.template as<MmaAngle>();
-            gs.d.h_mma = gs.h_mma.data();
-            gs.h_groups = mma_groups(gs.h_mma);
-            CK(c, gs.groups.ensure(sizeof(int) * gs.h_groups.size()));
-            CK(c, cudaMemcpy(gs.groups.p, gs.h_groups.data(), sizeof(int) * gs.h_groups.size(), cudaMemcpyHostToDevice));
-            gs.d.groups = gs.groups.template as<int>();
-            gs.d.h_groups = gs.h_groups.data();
-            gs.d.n_groups = (int)gs.h_groups.size() - 1;
-            const std::vector<float> mask(h.cmask.begin(), h.cmask.end());
-            std::vector<int> tiles;
-            gs.d.n_tiles_in = bp_tiles(mask.data(), c->N, tiles);
-            CK(c, gs.tiles_in.ensure(sizeof(int) * tiles.size()));
-            CK(c, cudaMemcpy(gs.tiles_in.p, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice));
-            gs.d.tiles_in = gs.tiles_in.template as<int>();
+    // the other tables share one allocation and one copy: either costs a new
+    // context some 10 us, and there are 16 of them
+    std::vector<char> pack;
+    struct Place {
+        size_t at;
+        const void** to;
+    };
+    std::vector<Place> places;
+    auto put = [&](auto& to, const void* p, size_t bytes) {
+        const size_t at = pack.size();
+        pack.resize((at + bytes + 255) / 256 * 256);
+        if (bytes) std::memcpy(pack.data() + at, p, bytes);
+        places.push_back({at, (const void**)&to});
+    };
+    put(gs.d.sc_bp, h.sc_bp.data(), sizeof(Real) * h.sc_bp.size());
+    put(gs.d.sc_fp, h.sc_fp.data(), sizeof(Real) * h.sc_fp.size());
+    h.filt.resize(h.filt.size() + 8);
+    put(gs.d.filt, h.filt.data(), sizeof(Real) * h.filt.size());
+    put(gs.d.fft_h, h.fft_h.data(), sizeof(Real) * h.fft_h.size());
+    put(gs.d.fft_h_x, h.fft_h_x.data(), sizeof(Real) * h.fft_h_x.size());
+    put(gs.d.xsc_bp, h.xsc_bp.data(), sizeof(float) * h.xsc_bp.size());
+    put(gs.d.xsc_fp, h.xsc_fp.data(), sizeof(float) * h.xsc_fp.size());
+    if (sizeof(Real) == 4) {
+        const std::vector<float> tw32(h.fft_tw.begin(), h.fft_tw.end());
+        put(gs.d.fft_tw, tw32.data(), sizeof(float) * tw32.size());
+        if (!h.fft_tw16.empty()) {
+            const std::vector<float> t16(h.fft_tw16.begin(), h.fft_tw16.end());
+            put(gs.d.fft_tw16, t16.data(), sizeof(float) * t16.size());
         }
+    } else {
+        put(gs.d.fft_tw64, h.fft_tw.data(), sizeof(double) * h.fft_tw.size());
     }
-    gs.d.xsc_bp = gs.xsc_bp.template as<float4>();
+    // angle order of the pair projector: angles read through the x-pair
+    // image (|sin| >= |cos|) first, then the transposed ones
+    std::vector<int> ord;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int t = 0; t < c->T; ++t) {
+            const bool tr = std::fabs((double)h.sc_fp[2 * t + 1]) > std::fabs((double)h.sc_fp[2 * t]);
+            if (tr == (pass == 1)) ord.push_back(t);
+        }
+    put(gs.d.fp_order, ord.data(), sizeof(int) * ord.size());
+    // projector variant 6: chunks of neighbouring angles, longest blocks first
+    const std::vector<float> s32(h.sc_fp.begin(), h.sc_fp.end());
+    ord = lines_angle_order(s32.data(), c->T);
+    put(gs.d.lines_order, ord.data(), sizeof(int) * ord.size());
+    if constexpr (sizeof(Real) == 4) {
+        gs.h_mma = mma_angles(h.xsc_fp.data(), c->T);
+        put(gs.d.mma, gs.h_mma.data(), sizeof(MmaAngle) * gs.h_mma.size());
+        gs.d.h_mma = gs.h_mma.data();
+        gs.h_groups = mma_groups(gs.h_mma);
+        put(gs.d.groups, gs.h_groups.data(), sizeof(int) * gs.h_groups.size());
+        gs.d.h_groups = gs.h_groups.data();
+        gs.d.n_groups = (int)gs.h_groups.size() - 1;
+        const std::vector<FxAngle> fx = fx_angles(h.xsc_fp.data(), c->T);
+        put(gs.d.fx_fp, fx.data(), sizeof(FxAngle) * fx.size());
+        std::vector<int> tiles;
+        gs.d.n_tiles_in = bp_tiles(h.cmask.data(), c->N, tiles);
+        put(gs.d.tiles_in, tiles.data(), sizeof(int) * tiles.size());
+    }
+    CK(c, gs.tables.ensure(pack.size()));
+    CK(c, cudaMemcpy(gs.tables.p, pack.data(), pack.size(), cudaMemcpyHostToDevice));
+    for (const Place& p : places) *p.to = gs.tables.template as<char>() + p.at;
     gs.hx_bp.resize(c->T);
     std::memcpy(gs.hx_bp.data(), h.xsc_bp.data(), sizeof(float4) * c->T);
     gs.d.h_xsc_bp = gs.hx_bp.data();
@@ -137,7 +126,6 @@ int ensure_geom(acu_ctx* c)
             gs.hs_bp[t] = make_float4((float)h.sc_bp[2 * t], (float)h.sc_bp[2 * t + 1], 0.f, 0.f);
         gs.d.h_sc_bp = gs.hs_bp.data();
     }
-    gs.d.xsc_fp = gs.xsc_fp.template as<float4>();
     gs.d.exact = (sizeof(Real) == 4) ? c->opt_positions : 0;
     gs.d.fft_L = h.fft_L;
     gs.d.fft_log2L = h.fft_log2L;
@@ -201,9 +189,21 @@ void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q,
     launch_backproject<Real, V>(g, G, q, img, c->stream);
 }
 
+// Floats per bin of the filtered sinogram's buffer: single slices are
+// backprojected from pairs (bin, next bin).
+template <typename Real, int V>
+constexpr size_t q_width() { return V == 1 && sizeof(Real) == 4 ? 2 : 1; }
+
 template <typename Real, int V>
 void lanes_iradon(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* sino, Real* q, Real* img)
 {
+    if constexpr (V == 1 && sizeof(Real) == 4) {
+        if (g.exact && c->opt_filter == 0 && g.fft_L > 0 && fft_fits<Real>(g.fft_L)) {
+            launch_filter_fft<Real, V>(g, G, sino, q, c->stream, true);
+            launch_backproject_fx(g, G, reinterpret_cast<const float2*>(q), img, c->stream);
+            return;
+        }
+    }
     lanes_filter<Real, V>(c, g, G, sino, q);
     lanes_backproject<Real, V>(c, g, G, q, img);
 }
@@ -289,7 +289,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     switch (op) {
     case OP_IRADON:
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
-        CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * V));
+        CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * V * q_width<Real, V>()));
         lanes_iradon<Real, V>(c, g, G, lin, c->w_q.template as<Real>(), lout);
         break;
     case OP_RADON:
@@ -307,6 +307,14 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     case OP_FILTER: lanes_filter<Real, V>(c, g, G, lin, lout); break;
     case OP_BACKPROJECT:
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
+        if constexpr (V == 1 && sizeof(Real) == 4) {
+            if (g.exact) {
+                CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * 2));
+                launch_pairs(lin, c->w_q.template as<float2>(), N, nsino * G, c->stream);
+                launch_backproject_fx(g, G, c->w_q.template as<float2>(), lout, c->stream);
+                break;
+            }
+        }
         lanes_backproject<Real, V>(c, g, G, lin, lout);
         break;
     }
@@ -488,7 +496,8 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     TvState<Real>& s = tvstate<Real>(c);
     const int N = c->N, T = c->T, G = (S + V - 1) / V;
     const size_t nimg = (size_t)N * N * G * V, nsino = (size_t)T * N * G * V;
-    for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp, &s.q}) CK(c, b->ensure(sizeof(Real) * nsino));
+    for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CK(c, b->ensure(sizeof(Real) * nsino));
+    CK(c, s.q.ensure(sizeof(Real) * nsino * q_width<Real, V>()));
     for (DevBuf* b : {&s.uk, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap, &s.tmp})
         CK(c, b->ensure(sizeof(Real) * nimg));
     if (c->opt_verbose) CK(c, s.ukp.ensure(sizeof(Real) * nimg));

@@ -19,16 +19,17 @@
 #include "batch.h"
 #include "common.cuh"
 #include "ctx.h"
+#include "fixed.cuh"
 #include "tables.h"
 
 namespace acu {
 
-// One staggered ray of the single-slice projector (as radon_stag_ray<1> in
-// kernels_radon.cu), through the image (TR = false) or its transpose, over the
-// warp's steps i0..i1.
-template <bool EX, bool TR>
+// One staggered ray of the single-slice projector at the reference's positions
+// (as radon_stag_ray<1> in kernels_radon.cu), through the image (TR = false) or its
+// transpose, over the warp's steps i0..i1.  Exact positions: fx_ray (fixed.cuh).
+template <bool TR>
 __device__ __forceinline__ void radon_stag_ray_v1(const float* __restrict__ base, int N, int kb, int i0, int i1,
-                                                  const ProjRay<float, EX>& ray, float mid, int jy,
+                                                  const ProjRay<float, false>& ray, float mid, int jy,
                                                   float (&acc)[1])
 {
     constexpr bool transposed = TR;
@@ -70,7 +71,8 @@ template <bool EX>
 __global__ void __launch_bounds__(512) k_batch_radon(const ProbDesc* __restrict__ pd, int nprob,
                                                      const float* __restrict__ img, const float* __restrict__ IT,
                                                      float* __restrict__ sino, const float* __restrict__ sc,
-                                                     const float4* __restrict__ xsc, long long total, int* counter)
+                                                     const float4* __restrict__ xsc, const FxAngle* __restrict__ fx,
+                                                     long long total, int* counter)
 {
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -86,6 +88,12 @@ __global__ void __launch_bounds__(512) k_batch_radon(const ProbDesc* __restrict_
         const int N = d.N;
         const float s = sc[d.sc + 2 * t], c = sc[d.sc + 2 * t + 1];
         const ProjRay<float, EX> ray(sc + d.sc, xsc + d.sc / 2, t, jy, d.mid, nullptr);
+        if constexpr (EX) {
+            const FxAngle a = fx[d.sc / 2 + t];
+            const float v = llabs(a.c) > llabs(a.s) ? fx_ray<true>(IT + d.img, N, a, ray, jy, lane)
+                                                    : fx_ray<false>(img + d.img, N, a, ray, jy, lane);
+            if (jy <= N) sino[d.sino + (size_t)t * N + (jy - 1)] = v / (float)N;
+        } else {
         const bool transposed = fabsf(c) > fabsf(s);
         const float ratio = transposed ? -s / c : c / s;
         const int kb = __float2int_rn((float)lane * ratio);
@@ -101,10 +109,11 @@ __global__ void __launch_bounds__(512) k_batch_radon(const ProbDesc* __restrict_
         const int i1 = min(N + max(0, kend), __reduce_max_sync(0xffffffffu, hi + kb));
         float acc[1] = {0.f};
         if (transposed)
-            radon_stag_ray_v1<EX, true>(IT + d.img, N, kb, i0, i1, ray, d.mid, jy, acc);
+            radon_stag_ray_v1<true>(IT + d.img, N, kb, i0, i1, ray, d.mid, jy, acc);
         else
-            radon_stag_ray_v1<EX, false>(img + d.img, N, kb, i0, i1, ray, d.mid, jy, acc);
+            radon_stag_ray_v1<false>(img + d.img, N, kb, i0, i1, ray, d.mid, jy, acc);
         if (jy <= N) sino[d.sino + (size_t)t * N + (jy - 1)] = acc[0] / (float)N;
+        }
     }
 }
 
@@ -132,12 +141,10 @@ __global__ void __launch_bounds__(256) k_batch_transpose(const ProbDesc* __restr
     }
 }
 
-// ---- backprojection: one block item = a 32 x R pixel tile of one problem ----
-template <bool EX>
+// ---- backprojection: one block item = a 32-pixel-wide tile of one problem; here at the reference's positions ----
 __global__ void __launch_bounds__(512) k_batch_backproject(const ProbDesc* __restrict__ pd, int nprob,
                                                            const float* __restrict__ q, float* __restrict__ img,
                                                            const float* __restrict__ sc,
-                                                           const float4* __restrict__ xsc,
                                                            const float* __restrict__ cmask, long long total,
                                                            int* counter)
 {
@@ -165,20 +172,11 @@ __global__ void __launch_bounds__(512) k_batch_backproject(const ProbDesc* __res
             const float dx = (float)jx - mid, dy = (float)jy - mid;
             const float* qq = q + d.sino;
             const float* sct = sc + d.sc;
-            const float4* xst = xsc + d.sc / 2;
             for (int t = 0; t < d.T; ++t) {
-                float y1f, wl, wh;
-                if constexpr (EX) {
-                    const float4 x = __ldg(xst + t);
-                    exact_coord(x.x, x.y, x.z, x.w, dx, dy, mid, y1f, wh);
-                    wl = 1.f - wh;
-                } else {
-                    const float s = sct[2 * t], c = sct[2 * t + 1];
-                    const float yr = add_rn(add_rn(mul_rn(s, dx), mul_rn(c, dy)), mid);
-                    y1f = floorf(yr);
-                    wl = add_rn(y1f, 1.f) - yr;
-                    wh = yr - y1f;
-                }
+                const float s = sct[2 * t], c = sct[2 * t + 1];
+                const float yr = add_rn(add_rn(mul_rn(s, dx), mul_rn(c, dy)), mid);
+                const float y1f = floorf(yr);
+                const float wl = add_rn(y1f, 1.f) - yr, wh = yr - y1f;
                 const int y1 = (int)y1f;
                 if (y1 > 1 && y1 < N) {
                     const float* row = qq + (size_t)t * N + (y1 - 1);
@@ -187,6 +185,42 @@ __global__ void __launch_bounds__(512) k_batch_backproject(const ProbDesc* __res
             }
         }
         img[d.img + pix] = cm * acc;
+    }
+}
+
+// Exact positions: the same items, R pixel rows a thread, bins as pairs (fixed.cuh).
+template <int R>
+__global__ void __launch_bounds__(512) k_batch_backproject_fx(const ProbDesc* __restrict__ pd, int nprob,
+                                                              const float2* __restrict__ q, float* __restrict__ img,
+                                                              const float4* __restrict__ xsc,
+                                                              const float* __restrict__ cmask, long long total,
+                                                              int* counter)
+{
+    __shared__ int s_it;
+    __shared__ int4 tab[FX_CHUNK];
+    for (;;) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) s_it = atomicAdd(counter, 1);
+        __syncthreads();
+        const int it = s_it;
+        __syncthreads();
+        if (it >= total) break;
+        const ProbDesc d = pd[find_prob<&ProbDesc::it_bp>(pd, nprob, it)];
+        const int N = d.N, ntx = (N + 31) / 32, h = R * blockDim.y;
+        const int local = (int)(it - d.it_bp);
+        const int x0 = (local % ntx) * 32 + 1, y0 = (local / ntx) * h + 1;
+        const int x = x0 + threadIdx.x - 1, y = y0 + threadIdx.y * R - 1;   // 0-based
+        float cm[R], v[R];
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            v[r] = 0.f;
+            cm[r] = x < N && y + r < N ? cmask[d.cm + (size_t)(y + r) * N + x] : 0.f;
+            any |= cm[r] != 0.f;
+        }
+        if (__syncthreads_or(any)) fx_backproject<R>(q + d.sino, xsc + d.sc / 2, N, d.T, d.mid, x0, y0, tab, v);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (x < N && y + r < N) img[d.img + (size_t)(y + r) * N + x] = cm[r] != 0.f ? cm[r] * v[r] : 0.f;
     }
 }
 
@@ -232,7 +266,7 @@ __device__ float2* fft_ragged(float2* d0, float2* d1, const float2* __restrict__
 __global__ void __launch_bounds__(256) k_batch_filter(const ProbDesc* __restrict__ pd, int nprob,
                                                       const float* __restrict__ sino, float* __restrict__ out,
                                                       const float* __restrict__ H, const float2* __restrict__ tw,
-                                                      int Lmax)
+                                                      int Lmax, bool pairs)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const long long it = blockIdx.x;
@@ -257,6 +291,16 @@ __global__ void __launch_bounds__(256) k_batch_filter(const ProbDesc* __restrict
     __syncthreads();
     float2* y = fft_ragged(res, other, tw, Lmax / L, L);
     float* o = out + d.sino + (size_t)t0 * N;
+    if (pairs) {   // (bin, next bin), zeros in the first and the last
+        float2* o2 = reinterpret_cast<float2*>(out) + d.sino + (size_t)t0 * N;
+        for (int n = threadIdx.x; n < N; n += blockDim.x) {
+            const bool in = n > 0 && n < N - 1;
+            const float2 v = y[n], w = y[in ? n + 1 : n];
+            o2[n] = in ? make_float2(v.x, w.x) : make_float2(0.f, 0.f);
+            if (has_b) o2[N + n] = in ? make_float2(-v.y, -w.y) : make_float2(0.f, 0.f);
+        }
+        return;
+    }
     for (int n = threadIdx.x; n < N; n += blockDim.x) {
         o[n] = y[n].x;
         if (has_b) o[N + n] = -y[n].y;
@@ -472,30 +516,36 @@ void batch_radon(const BatchDev& b, const float* img, float* sino, int slot, cud
     const int threads = 32 * b.radon_warps;
     const int blocks = sm_count() * (2048 / threads);
     if (b.exact)
-        k_batch_radon<true><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.n_radon,
-                                                        b.counter + slot);
+        k_batch_radon<true><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.fx_fp,
+                                                        b.n_radon, b.counter + slot);
     else
-        k_batch_radon<false><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.n_radon,
-                                                         b.counter + slot);
+        k_batch_radon<false><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.fx_fp,
+                                                         b.n_radon, b.counter + slot);
 }
+// pixel rows per thread of the exact backprojection: tiles of 16 or 32 rows
+static int batch_bp_pixels(int rows) { return rows == 16 ? 2 : 4; }
+
 void batch_backproject(const BatchDev& b, const float* q, float* img, int slot, cudaStream_t st)
 {
     cudaMemsetAsync(b.counter + slot, 0, sizeof(int), st);
     dim3 blk(32, b.bp_rows);
     const int blocks = sm_count() * (2048 / (32 * b.bp_rows));
-    if (b.exact)
-        k_batch_backproject<true><<<blocks, blk, 0, st>>>(b.pd, b.nprob, q, img, b.sc_bp, b.xsc_bp, b.cmask, b.n_bp,
+    const float2* q2 = reinterpret_cast<const float2*>(q);
+    if (b.exact && batch_bp_pixels(b.bp_rows) == 4)
+        k_batch_backproject_fx<4><<<blocks, blk, 0, st>>>(b.pd, b.nprob, q2, img, b.xsc_bp, b.cmask, b.n_bp,
+                                                          b.counter + slot);
+    else if (b.exact)
+        k_batch_backproject_fx<2><<<blocks, blk, 0, st>>>(b.pd, b.nprob, q2, img, b.xsc_bp, b.cmask, b.n_bp,
                                                           b.counter + slot);
     else
-        k_batch_backproject<false><<<blocks, blk, 0, st>>>(b.pd, b.nprob, q, img, b.sc_bp, b.xsc_bp, b.cmask, b.n_bp,
-                                                           b.counter + slot);
+        k_batch_backproject<<<blocks, blk, 0, st>>>(b.pd, b.nprob, q, img, b.sc_bp, b.cmask, b.n_bp, b.counter + slot);
 }
 void batch_filter(const BatchDev& b, const float* sino, float* out, cudaStream_t st)
 {
     max_dynamic_smem<k_batch_filter>();
     const float* H = (b.exact && b.fft_h_x) ? b.fft_h_x : b.fft_h;   // exact positions: FP64 taps
     k_batch_filter<<<(unsigned)b.n_fft, 256, 2 * (size_t)b.Lmax * sizeof(float2), st>>>(b.pd, b.nprob, sino, out, H,
-                                                                                         b.tw, b.Lmax);
+                                                                                         b.tw, b.Lmax, b.exact != 0);
 }
 void batch_rhs(const BatchDev& b, float mu, float lambda, const float* ifkt, const float* dx, const float* bx,
                const float* dy, const float* by, float* rhs, cudaStream_t st)
@@ -558,7 +608,7 @@ struct acu_batch {
     std::vector<ProbDesc> desc;       // in caller order
     std::vector<int> order;           // execution order (largest work first) -> caller index
     BatchDev dev;
-    DevBuf d_pd, d_sc_bp, d_sc_fp, d_xsc_bp, d_xsc_fp, d_cm, d_fh, d_fhx, d_tw, d_counter;
+    DevBuf d_pd, d_sc_bp, d_sc_fp, d_xsc_bp, d_xsc_fp, d_fx_fp, d_cm, d_fh, d_fhx, d_tw, d_counter;
     DevBuf f, fk, ruk, rp, q, uk, dx, dy, bx, by, rhs, r, p, Ap, tmp, part, rsold, alpha, beta, it_img;
     DevBuf io_in, io_out;
     cudaGraphExec_t graph = nullptr, graph_inc = nullptr;
@@ -764,6 +814,8 @@ int acu_batch_create(acu_batch** out, int nprob, const int* nimage, const int* n
     CKRET(up(b->d_sc_fp, sc_fp.data(), sizeof(float) * sc_fp.size()));
     CKRET(up(b->d_xsc_bp, xsc_bp.data(), sizeof(float) * xsc_bp.size()));
     CKRET(up(b->d_xsc_fp, xsc_fp.data(), sizeof(float) * xsc_fp.size()));
+    const std::vector<FxAngle> fx = fx_angles(xsc_fp.data(), (int)(xsc_fp.size() / 4));
+    CKRET(up(b->d_fx_fp, fx.data(), sizeof(FxAngle) * fx.size()));
     CKRET(up(b->d_cm, cm.data(), sizeof(float) * cm.size()));
     CKRET(up(b->d_fh, fh.data(), sizeof(float) * fh.size()));
     CKRET(up(b->d_fhx, fhx.data(), sizeof(float) * fhx.size()));
@@ -776,6 +828,7 @@ int acu_batch_create(acu_batch** out, int nprob, const int* nimage, const int* n
     d.sc_fp = b->d_sc_fp.as<float>();
     d.xsc_bp = b->d_xsc_bp.as<float4>();
     d.xsc_fp = b->d_xsc_fp.as<float4>();
+    d.fx_fp = b->d_fx_fp.as<FxAngle>();
     d.cmask = b->d_cm.as<float>();
     d.fft_h = b->d_fh.as<float>();
     d.fft_h_x = b->d_fhx.as<float>();
@@ -819,12 +872,13 @@ namespace {
 int set_bp_rows(acu_batch* b, int rows)
 {
     b->dev.bp_rows = rows;
+    const int height = rows * (b->dev.exact ? batch_bp_pixels(rows) : 1);
     std::vector<ProbDesc> ex(b->nprob);
     long long ib = 0;
     for (int k = 0; k < b->nprob; ++k) {
         ProbDesc d = b->desc[b->order[k]];
         d.it_bp = ib;
-        ib += (long long)((d.N + 31) / 32) * ((d.N + rows - 1) / rows);
+        ib += (long long)((d.N + 31) / 32) * ((d.N + height - 1) / height);
         ex[k] = d;
         b->desc[b->order[k]].it_bp = d.it_bp;
     }
@@ -837,7 +891,8 @@ int ensure_state(acu_batch* b)
 {
     acu_ctx* c = b->ctx;
     const size_t ni = sizeof(float) * (size_t)b->dev.img_total, ns = sizeof(float) * (size_t)b->dev.sino_total;
-    for (DevBuf* x : {&b->f, &b->fk, &b->ruk, &b->rp, &b->q}) CK(c, x->ensure(ns));
+    for (DevBuf* x : {&b->f, &b->fk, &b->ruk, &b->rp}) CK(c, x->ensure(ns));
+    CK(c, b->q.ensure(2 * ns));   // exact positions: pairs of bins
     for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->rhs, &b->r, &b->p, &b->Ap, &b->tmp, &b->it_img})
         CK(c, x->ensure(ni));
     b->dev.IT = b->it_img.as<float>();
@@ -851,7 +906,7 @@ int tune_all(acu_batch* b)
     if (b->tuned) return ACU_OK;
     CKRET(ensure_state(b));
     CK(b->ctx, cudaMemsetAsync(b->uk.p, 0, sizeof(float) * b->dev.img_total, b->ctx->stream));
-    CK(b->ctx, cudaMemsetAsync(b->q.p, 0, sizeof(float) * b->dev.sino_total, b->ctx->stream));
+    CK(b->ctx, cudaMemsetAsync(b->q.p, 0, 2 * sizeof(float) * b->dev.sino_total, b->ctx->stream));
     // the backprojection work list must match the tile height while timing
     cudaStream_t st = b->ctx->stream;
     cudaEvent_t e0, e1;
@@ -1004,6 +1059,7 @@ int acu_batch_set_option(acu_batch* b, int option, int value)
     if (option != ACU_OPT_POSITIONS)
         return berr(b, ACU_ERR_INVALID, "acu_batch_set_option: only ACU_OPT_POSITIONS and ACU_OPT_RADON_REFRESH");
     if (value != 0 && value != 1) return berr(b, ACU_ERR_INVALID, "ACU_OPT_POSITIONS must be 0 or 1");
+    if (b->dev.exact != value) b->tuned = false;   // the backprojection's tiles differ
     b->dev.exact = value;
     return ACU_OK;
 }

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
+
 namespace acu {
 
 // One problem of a ragged batch.  Offsets are in elements of the
@@ -32,6 +34,7 @@ struct BatchDev {
     const float* sc_fp = nullptr;
     const float4* xsc_bp = nullptr;   // exact-position tables, [angle][4] (index ProbDesc::sc / 2)
     const float4* xsc_fp = nullptr;
+    const FxAngle* fx_fp = nullptr;   // projector's angles in fixed point (index ProbDesc::sc / 2)
     int exact = 1;                    // 1: exact sample positions (default), 0: the reference's (acu_batch_set_option)
     const float* cmask = nullptr;
     const float* fft_h = nullptr;

@@ -49,7 +49,7 @@ struct DevBuf {
 template <typename Real>
 struct GeomSet {
     bool ready = false;
-    DevBuf sc_bp, sc_fp, filt, cmask, fft_h, fft_h_x, fft_tw, fft_tw16, fp_order, lines_order, xsc_bp, xsc_fp, mma, groups, tiles_in;
+    DevBuf cmask, tables;
     std::vector<MmaAngle> h_mma;
     std::vector<int> h_groups;
     std::vector<float4> hx_bp;   // host copy of xsc_bp

@@ -1,0 +1,173 @@
+// Sample positions in fixed point for the kernels that carry one slice per
+// thread, which are held by the instructions a position takes (exact positions,
+// sides up to FX_MAX_SIDE).
+//
+// Along a ray both coordinates advance by a constant, so they are kept as
+// 64-bit integers with 32 fraction bits: the cell is the high word, the fraction
+// the low word's leading 23 bits, and a step is an addition.  A sine or cosine is
+// rounded to 2^-33 and multiplied by at most FX_MAX_SIDE / 2 from the middle of
+// the grid, so a coordinate is within 2.4e-7 of double precision at a side of
+// 2049 (6e-8 rms) and exact at grid-aligned angles, as with split tables
+// (common.cuh), at five instructions in place of thirteen.
+#pragma once
+#include <type_traits>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace acu {
+
+__device__ __forceinline__ int fx_cell(long long v) { return (int)(v >> 32); }
+__device__ __forceinline__ float fx_frac(long long v)
+{
+    return __uint_as_float(((unsigned)v >> 9) | 0x3f800000u) - 1.f;
+}
+constexpr long long FX_HALF = 1ll << 8;   // half of the fraction's last kept bit: fractions are rounded, not cut
+
+// One ray (bin jy) of the single-slice projector: the sum of its samples.  The
+// rays of a warp are staggered so that the 32 samples of a step lie in one or two
+// rows of the copy read.  TR: through the transpose (rows follow x), else the
+// image (rows follow y).
+template <bool TR>
+__device__ __forceinline__ float fx_ray(const float* __restrict__ base, int N, FxAngle a,
+                                        const ProjRay<float, true>& ray, int jy, int lane)
+{
+    const int m = (N + 1) / 2;
+    const float s = (float)a.s * 0x1p-32f, c = (float)a.c * 0x1p-32f;
+    // |c| <= |s| without TR and the other way round with it
+    const float ratio = TR ? -s / c : c / s;
+    const int kb = __float2int_rn((float)lane * ratio);
+    long long xm = ((long long)m << 32) - a.s * (jy - m) + FX_HALF, ym = ((long long)m << 32) + a.c * (jy - m) + FX_HALF;
+    bool some = jy <= N;
+    // The ray's steps whose cell is valid are an interval.  It is estimated with a margin and narrowed by the fixed-point
+    // positions, then its ends are settled by the exact ones, which differ by less than 1e-6: at most one sample at
+    // each end, unless the ray is nearly parallel to an axis and runs along the rim, where only those tell.
+    int lo, hi;
+    valid_steps(s, c, (float)(jy - m), (float)m, N, lo, hi);
+    auto valid = [&](int jx) {
+        int x, y;
+        float w0, w1, w2, w3;
+        ray.at((float)(jx - m), x, y, w0, w1, w2, w3);
+        return min(x, y) > 1 && max(x, y) < N;
+    };
+    auto inside = [&](int jx) {
+        const int x = fx_cell(xm + (jx - m) * a.c), y = fx_cell(ym + (jx - m) * a.s);
+        return (unsigned)(x - 2) < (unsigned)(N - 2) && (unsigned)(y - 2) < (unsigned)(N - 2);
+    };
+    if (some) {
+        if (fminf(fabsf(s), fabsf(c)) >= 1e-3f) {
+            const int lo0 = lo, hi0 = hi;
+            while (lo <= hi && !inside(lo)) ++lo;
+            while (lo <= hi && !inside(hi)) --hi;
+            if (lo > hi) {   // a corner: at most a sample or two, if any
+                lo = lo0;
+                hi = hi0;
+            } else {
+                lo = max(lo - 1, lo0);
+                hi = min(hi + 1, hi0);
+            }
+        }
+        while (lo <= hi && !valid(lo)) ++lo;
+        while (lo <= hi && !valid(hi)) --hi;
+        some = lo <= hi;
+        // where that puts a fixed-point sample on the rim, the ray moves in by the difference: its cells are in 1..N-1
+        const long long end = ((long long)N << 32) - 1;
+        xm -= max(0ll, max(xm + (lo - m) * a.c, xm + (hi - m) * a.c) - end);
+        ym -= max(0ll, max(ym + (lo - m) * a.s, ym + (hi - m) * a.s) - end);
+    }
+    if (!some) {
+        lo = 0x3fffffff;
+        hi = -0x3fffffff;
+    } else {
+        lo += kb;
+        hi += kb;
+    }
+    // steps of the warp: where some ray has a sample, and where all have
+    const int i0 = __reduce_min_sync(0xffffffffu, lo), i1 = __reduce_max_sync(0xffffffffu, hi);
+    const int a0 = __reduce_max_sync(0xffffffffu, lo), a1 = __reduce_min_sync(0xffffffffu, hi);
+    const long long dr = TR ? a.c : a.s, dc = TR ? a.s : a.c;
+    const long long steps = (long long)i0 - kb - m;
+    long long r = (TR ? xm : ym) + steps * dr, q = (TR ? ym : xm) + steps * dc;
+    float sum = 0.f;
+    // a step in which some rays have no sample reads a pixel of the image all the same and drops it: without a branch,
+    // the loads of several steps are in flight together
+    auto sample = [&](auto partial, int i) {
+        int cr = fx_cell(r), cq = fx_cell(q);
+        bool ok = true;
+        if constexpr (decltype(partial)::value) {
+            ok = i >= lo && i <= hi;
+            cr = min(max(cr, 1), N - 1);
+            cq = min(max(cq, 1), N - 1);
+        }
+        const float* p = base + (unsigned)((cr - 1) * N + cq - 1);
+        const float fr = fx_frac(r), fc = fx_frac(q);
+        const float v00 = __ldg(p), v01 = __ldg(p + 1), v10 = __ldg(p + N), v11 = __ldg(p + N + 1);
+        const float gr = 1.f - fr, gc = 1.f - fc;
+        const float t = fmaf(v01, fc, v00 * gc), b = fmaf(v11, fc, v10 * gc);
+        const float next = fmaf(b, fr, fmaf(t, gr, sum));
+        sum = ok ? next : sum;
+        r += dr;
+        q += dc;
+    };
+    using Some = std::true_type;
+    using All = std::false_type;
+    int i = i0;
+    const int b0 = a0 <= a1 ? a0 : i1 + 1;   // steps before all rays have samples (all steps, if there are none)
+#pragma unroll 4
+    for (; i < b0; ++i) sample(Some{}, i);
+#pragma unroll 2
+    for (; i <= a1; ++i) sample(All{}, i);
+#pragma unroll 4
+    for (; i <= i1; ++i) sample(Some{}, i);
+    return sum;
+}
+
+// Backprojection of one 32-pixel-wide tile by a block of 32 x BY threads, R rows
+// a thread (column-wise neighbours), one slice.  q: [T][N] pairs (bins y and
+// y + 1: one load per pixel), zeros in the first and the last, which are never
+// tapped.  Per angle the position of the tile's middle pixel is formed once per
+// block (split tables, common.cuh) and kept with 26 fraction bits; the pixels'
+// positions follow by additions.  |position - middle| < 32 bins: the tile is at
+// most 32 pixels high.
+constexpr int FX_CHUNK = 256;   // angles whose entries are held in shared memory
+
+template <int R>
+__device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, const float4* __restrict__ xsc, int N,
+                                               int T, float mid, int x0, int y0, int4* tab, float (&out)[R])
+{
+    const int tid = threadIdx.y * 32 + threadIdx.x, nthreads = 32 * blockDim.y, h = R * blockDim.y / 2;
+    const int lx = (int)threadIdx.x - 16, ly = (int)threadIdx.y * R - h;
+#pragma unroll
+    for (int r = 0; r < R; ++r) out[r] = 0.f;
+    for (int t0 = 0; t0 < T; t0 += FX_CHUNK) {
+        const int n = min(FX_CHUNK, T - t0);
+        __syncthreads();
+        for (int a = tid; a < n; a += nthreads) {
+            const float4 x = __ldg(xsc + t0 + a);
+            float cell, frac;
+            exact_coord(x.x, x.y, x.z, x.w, (float)(x0 + 16) - mid, (float)(y0 + h) - mid, mid, cell, frac);
+            constexpr float ONE = 67108864.f;   // 2^26
+            // cell - 1: the pair's index; 4: half of the fraction's last kept bit
+            tab[a] = make_int4((int)(frac * ONE) + 4, (int)(x.x * ONE) + __float2int_rn(x.z * ONE),
+                               (int)(x.y * ONE) + __float2int_rn(x.w * ONE), (int)cell - 1);
+        }
+        __syncthreads();
+        const float2* row = q + (size_t)t0 * N;
+        // a block's first touch of an angle's bins comes from L2: 16 loads in flight per thread
+#pragma unroll (16 / R)
+        for (int a = 0; a < n; ++a, row += N) {
+            const int4 e = tab[a];
+            int p = e.x + lx * e.y + ly * e.z;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const unsigned i = min((unsigned)((p >> 26) + e.w), (unsigned)(N - 1));
+                const float w = __uint_as_float(((unsigned)(p << 6) >> 9) | 0x3f800000u);   // fraction + 1
+                const float2 v = __ldg(row + i);
+                out[r] = fmaf(v.y, w - 1.f, fmaf(v.x, 2.f - w, out[r]));
+                p += e.z;
+            }
+        }
+    }
+}
+
+}  // namespace acu

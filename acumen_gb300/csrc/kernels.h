@@ -15,6 +15,12 @@ struct BpTable {
     float4 v[BP_TMAX];
 };
 
+// Sine and cosine of an angle times 2^32 (fixed.cuh)
+struct FxAngle {
+    long long s, c;
+};
+constexpr int FX_MAX_SIDE = 4097;
+
 // One angle of the tensor-core projector (kernels_radon_mma.cu).
 struct MmaAngle {
     float4 x;         // split sine and cosine, as xsc_fp
@@ -48,6 +54,7 @@ struct DevGeom {
     const float4* xsc_bp = nullptr;
     const float4* xsc_fp = nullptr;
     int exact = 0;
+    const FxAngle* fx_fp = nullptr;     // projector's angles in fixed point (single precision)
     const MmaAngle* mma = nullptr;      // tensor-core projector's angles (single precision), and their host copy
     const MmaAngle* h_mma = nullptr;
     const int* groups = nullptr;        // first angles of its groups, n_groups + 1 of them, and their host copy
@@ -115,13 +122,22 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
                             cudaStream_t st);
 // The staggered projector for one slice per thread (plain layout); IT is a
 // work buffer of N * N floats per slice.
+// Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
+// (sides up to FX_MAX_SIDE); launch_backproject_fx: q as pairs (bin, next bin),
+// which the filter writes or launch_pairs makes from n = slices * T * N bins.
+std::vector<FxAngle> fx_angles(const float* xsc, int T);
+void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);
+void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, float* img, cudaStream_t st);
+void launch_pairs(const float* q, float2* out, int N, size_t n, cudaStream_t st);
+void launch_transpose_v1(int N, int S, const float* img, float* IT, cudaStream_t st);
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);
 template <typename Real, int V>
 void launch_radon_adjoint(const DevGeom<Real>& g, int G, const Real* sino, Real* img, cudaStream_t st);
 template <typename Real, int V>
 void launch_filter_direct(const DevGeom<Real>& g, int G, const Real* sino, Real* out, cudaStream_t st);
 template <typename Real, int V>
-void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* out, cudaStream_t st);
+void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* out, cudaStream_t st,
+                       bool pairs = false);   // pairs (V = 1): as launch_backproject_fx reads them
 template <typename Real>
 bool fft_fits(int L);
 

@@ -102,7 +102,7 @@ template <typename Real>
 __global__ void __launch_bounds__(512) k_filter_fft(const Real* __restrict__ sino, Real* __restrict__ out,
                                                     const Real* __restrict__ H,
                                                     const typename Cplx<Real>::T* __restrict__ tw, int N, int T,
-                                                    int L, int V)
+                                                    int L, int V, bool pairs)
 {
     using C = typename Cplx<Real>::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -152,7 +152,12 @@ __global__ void __launch_bounds__(512) k_filter_fft(const Real* __restrict__ sin
     C* y = fft_stockham<C>(res, other, tw, L);
     for (int n = threadIdx.x; n < N; n += blockDim.x) {
         const C v = y[n];
-        if (V == 4) {
+        if (pairs) {   // (bin, next bin), zeros in the first and the last
+            const bool in = n > 0 && n < N - 1;
+            const C w = y[in ? n + 1 : n];
+            reinterpret_cast<C*>(out + 2 * offa)[n] = in ? C{v.x, w.x} : C{Real(0), Real(0)};
+            if (has_b) reinterpret_cast<C*>(out + 2 * offb)[n] = in ? C{-v.y, -w.y} : C{Real(0), Real(0)};
+        } else if (V == 4) {
             *reinterpret_cast<C*>(out + offa + (size_t)n * 4) = C{v.x, -v.y};
         } else {
             out[offa + (size_t)n * stride] = v.x;
@@ -245,7 +250,8 @@ __device__ void fft4096_r16(float2* b, const float2* __restrict__ tw1, const flo
 // packing, spectrum product and output as k_filter_fft, with fft4096_r16.
 __global__ void __launch_bounds__(256) k_filter_fft4096(const float* __restrict__ sino, float* __restrict__ out,
                                                         const float* __restrict__ H,
-                                                        const float2* __restrict__ tw16, int N, int T, int V)
+                                                        const float2* __restrict__ tw16, int N, int T, int V,
+                                                        bool pairs)
 {
     constexpr int L = 4096;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -290,7 +296,13 @@ __global__ void __launch_bounds__(256) k_filter_fft4096(const float* __restrict_
     fft4096_r16(b, tw1, tw2);
     for (int n = threadIdx.x; n < N; n += blockDim.x) {
         const float2 v = b[pad16(n)];
-        if (V == 4) {
+        if (pairs) {
+            const bool in = n > 0 && n < N - 1;
+            const float2 w = b[pad16(in ? n + 1 : n)];
+            reinterpret_cast<float2*>(out + 2 * offa)[n] = in ? make_float2(v.x, w.x) : make_float2(0.f, 0.f);
+            if (has_b)
+                reinterpret_cast<float2*>(out + 2 * offb)[n] = in ? make_float2(-v.y, -w.y) : make_float2(0.f, 0.f);
+        } else if (V == 4) {
             *reinterpret_cast<float2*>(out + offa + (size_t)n * 4) = make_float2(v.x, -v.y);
         } else {
             out[offa + (size_t)n * stride] = v.x;
@@ -300,7 +312,7 @@ __global__ void __launch_bounds__(256) k_filter_fft4096(const float* __restrict_
 }
 
 template <typename Real, int V>
-void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* out, cudaStream_t st)
+void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* out, cudaStream_t st, bool pairs)
 {
     using C = typename Cplx<Real>::T;
     const size_t sm = 2 * (size_t)g.fft_L * sizeof(C);
@@ -315,11 +327,11 @@ void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* ou
         if (g.fft_L == 4096 && g.fft_tw16) {   // 3.6x the radix-4 stages at this length
             const size_t sm16 = (size_t)(4096 + 256) * sizeof(float2);
             max_dynamic_smem<k_filter_fft4096>();
-            k_filter_fft4096<<<grd, 256, sm16, st>>>(sino, out, H, g.fft_tw16, g.N, g.T, V);
+            k_filter_fft4096<<<grd, 256, sm16, st>>>(sino, out, H, g.fft_tw16, g.N, g.T, V, pairs);
             return;
         }
     }
-    k_filter_fft<Real><<<grd, 512, sm, st>>>(sino, out, H, tw, g.N, g.T, g.fft_L, V);
+    k_filter_fft<Real><<<grd, 512, sm, st>>>(sino, out, H, tw, g.N, g.T, g.fft_L, V, pairs);
 }
 
 // Largest FFT length whose two shared-memory buffers fit in one block.
@@ -329,9 +341,9 @@ bool fft_fits(int L)
     return 2 * (size_t)L * 2 * sizeof(Real) <= 227 * 1024;
 }
 
-template void launch_filter_fft<float, 1>(const DevGeom<float>&, int, const float*, float*, cudaStream_t);
-template void launch_filter_fft<float, 4>(const DevGeom<float>&, int, const float*, float*, cudaStream_t);
-template void launch_filter_fft<double, 1>(const DevGeom<double>&, int, const double*, double*, cudaStream_t);
+template void launch_filter_fft<float, 1>(const DevGeom<float>&, int, const float*, float*, cudaStream_t, bool);
+template void launch_filter_fft<float, 4>(const DevGeom<float>&, int, const float*, float*, cudaStream_t, bool);
+template void launch_filter_fft<double, 1>(const DevGeom<double>&, int, const double*, double*, cudaStream_t, bool);
 template bool fft_fits<float>(int);
 template bool fft_fits<double>(int);
 

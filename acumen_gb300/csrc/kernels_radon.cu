@@ -871,10 +871,15 @@ __global__ void __launch_bounds__(256) k_transpose_lanes(const float* __restrict
     }
 }
 
+void launch_transpose_v1(int N, int S, const float* img, float* IT, cudaStream_t st)
+{
+    k_transpose_lanes<1><<<dim3((N + 31) / 32, (N + 31) / 32, S), 256, 0, st>>>(img, IT, N);
+}
+
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st)
 {
-    dim3 bp(256), gp((g.N + 31) / 32, (g.N + 31) / 32, S);
-    k_transpose_lanes<1><<<gp, bp, 0, st>>>(img, IT, g.N);
+    if (g.exact && g.N <= FX_MAX_SIDE) return launch_radon_fx(g, S, img, IT, sino, st);
+    launch_transpose_v1(g.N, S, img, IT, st);
     dim3 blk(32, 4), grd((g.N + 127) / 128, g.T, S);
     if (g.exact)
         k_radon_stag<1, true, false><<<grd, blk, 0, st>>>(img, IT, g.sc_fp, g.xsc_fp, g.fp_order, sino, g.N, g.T, g.mid);
