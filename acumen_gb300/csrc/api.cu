@@ -303,7 +303,15 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
             launch_radon<Real, V>(g, G, lin, lout, c->stream);
         }
         break;
-    case OP_RADON_ADJ: launch_radon_adjoint<Real, V>(g, G, lin, lout, c->stream); break;
+    case OP_RADON_ADJ:
+        if constexpr (sizeof(Real) == 4) {
+            if (g.exact) {
+                launch_adjoint_fx<V>(g, G, lin, nullptr, lout, c->stream);
+                break;
+            }
+        }
+        launch_radon_adjoint<Real, V>(g, G, lin, lout, c->stream);
+        break;
     case OP_FILTER: lanes_filter<Real, V>(c, g, G, lin, lout); break;
     case OP_BACKPROJECT:
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
@@ -890,7 +898,16 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     double* part = c->w_part.template as<double>();
     double* sums = part + (size_t)2 * nblk * S;
     cudaStream_t st = c->stream;
-    launch_radon_off<Real>(g, S, d_u, d_off, r, st);
+    // single precision at exact positions: the projection and its derivative from one walk
+    bool fused = false;
+    if constexpr (sizeof(Real) == 4) fused = g.exact != 0;
+    if constexpr (sizeof(Real) == 4) {
+        if (fused) {
+            CK(c, c->pairPT.ensure(sizeof(float) * nimg * S));
+            launch_ray_off(g, S, d_u, c->pairPT.template as<float>(), d_off, r, d_grad_off ? D : nullptr, st);
+        }
+    }
+    if (!fused) launch_radon_off<Real>(g, S, d_u, d_off, r, st);
     GradEw<Real>::residual(nsino, S, r, d_y, part, nblk, st);
     launch_sum_rows(part, S, nblk, sums, st);
     Real* gu = d_grad_u;
@@ -901,12 +918,19 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
         gu = c->w_q.template as<Real>();
         CK(c, cudaMemsetAsync(gu, 0, sizeof(Real) * nimg * S, st));
     } else {
-        launch_radon_adjoint_off<Real>(g, S, r, d_off, gu, st);
+        bool done = false;
+        if constexpr (sizeof(Real) == 4) {
+            if (g.exact) {
+                launch_adjoint_fx<1>(g, S, r, d_off, gu, st);
+                done = true;
+            }
+        }
+        if (!done) launch_radon_adjoint_off<Real>(g, S, r, d_off, gu, st);
     }
     GradEw<Real>::tv_grad(N, S, (Real)lambda, (Real)eps, d_u, gu, part + (size_t)nblk * S, nblk, st);
     launch_sum_rows(part + (size_t)nblk * S, S, nblk, sums + S, st);
     if (d_grad_off) {
-        launch_radon_doff<Real>(g, S, d_u, d_off, D, st);
+        if (!fused) launch_radon_doff<Real>(g, S, d_u, d_off, D, st);
         GradEw<Real>::off_grad(N, T, S, r, D, d_grad_off, st);
     }
     CKLAUNCH(c);

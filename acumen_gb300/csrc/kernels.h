@@ -123,11 +123,17 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
 // The staggered projector for one slice per thread (plain layout); IT is a
 // work buffer of N * N floats per slice.
 // Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
-// (sides up to FX_MAX_SIDE); launch_backproject_fx: q as pairs (bin, next bin),
-// which the filter writes or launch_pairs makes from n = slices * T * N bins.
+// (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
+// the derivative with respect to them or null; launch_backproject_fx: q as pairs
+// (bin, next bin), which the filter writes or launch_pairs makes from
+// n = slices * T * N bins; launch_adjoint_fx: the projector's exact transpose.
 std::vector<FxAngle> fx_angles(const float* xsc, int T);
 void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);
+void launch_ray_off(const DevGeom<float>& g, int S, const float* img, float* IT, const float* off, float* sino,
+                    float* dsino, cudaStream_t st);
 void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, float* img, cudaStream_t st);
+template <int V>
+void launch_adjoint_fx(const DevGeom<float>& g, int G, const float* sino, const float* off, float* img, cudaStream_t st);
 void launch_pairs(const float* q, float2* out, int N, size_t n, cudaStream_t st);
 void launch_transpose_v1(int N, int S, const float* img, float* IT, cudaStream_t st);
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);

@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(128) k_radon(const Real* __restrict__ img, con
     const int g = blockIdx.z;
     if (jy > N || t >= T) return;
     // bin jy is read at detector coordinate jy + off[t] (off: per-slice angle offsets, V = 1)
-    const ProjRay<Real, EX> ray(sc, xsc, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
+    const ProjRay<Real, false> ray(sc, nullptr, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
     const Real* u = img + (size_t)g * N * N * V;
     const size_t rowstride = (size_t)N * V;
     Lanes<Real, V> acc;
@@ -937,12 +937,12 @@ void launch_radon_pairs(const DevGeom<float>& g, int G, const float* img, float*
 // pixel (px,py) and angle theta the samples that use it as a bilinear tap lie
 // within sqrt(2) of its inverse-rotated position; each candidate sample is
 // re-evaluated with the projector's own arithmetic, so cells and weights are
-// identical to the forward operator's.
+// identical to the forward operator's.  The reference's positions and double
+// precision; single precision at exact positions: k_adjoint_fx (kernels_single.cu).
 // ---------------------------------------------------------------------------
-template <typename Real, int V, bool EX>
+template <typename Real, int V>
 __global__ void __launch_bounds__(256) k_radon_adjoint(const Real* __restrict__ sino,
                                                        const Real* __restrict__ sc,
-                                                       const float4* __restrict__ xsc,
                                                        Real* __restrict__ img, int N, int T, Real mid,
                                                        const Real* __restrict__ off)
 {
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(256) k_radon_adjoint(const Real* __restrict__ 
             jx0 = max(jx0, 1); jy0 = max(jy0, 1); jx1 = min(jx1, N); jy1 = min(jy1, N);
             const Real* yt = yg + (size_t)t * N * V;
             for (int jy = jy0; jy <= jy1; ++jy) {
-                const ProjRay<Real, EX> ray(sc, xsc, t, jy, mid, off_t);
+                const ProjRay<Real, false> ray(sc, nullptr, t, jy, mid, off_t);
                 Real wsum = Real(0);
                 for (int jx = jx0; jx <= jx1; ++jx) {
                     int x1, y1;
@@ -1000,13 +1000,7 @@ template <typename Real, int V>
 void launch_radon_adjoint(const DevGeom<Real>& g, int G, const Real* sino, Real* img, cudaStream_t st)
 {
     dim3 blk(32, 8), grd((g.N + 31) / 32, (g.N + 7) / 8, G);
-    if constexpr (sizeof(Real) == 4) {
-        if (g.exact) {
-            k_radon_adjoint<Real, V, true><<<grd, blk, 0, st>>>(sino, g.sc_fp, g.xsc_fp, img, g.N, g.T, g.mid, nullptr);
-            return;
-        }
-    }
-    k_radon_adjoint<Real, V, false><<<grd, blk, 0, st>>>(sino, g.sc_fp, g.xsc_fp, img, g.N, g.T, g.mid, nullptr);
+    k_radon_adjoint<Real, V><<<grd, blk, 0, st>>>(sino, g.sc_fp, img, g.N, g.T, g.mid, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1064,17 +1058,12 @@ void launch_filter_direct(const DevGeom<Real>& g, int G, const Real* sino, Real*
     k_filter_direct<Real, V, RB><<<grd, 256, sm, st>>>(sino, g.filt, out, g.N, g.T);
 }
 
-// ---- projector with per-angle detector offsets and its derivatives ------------
+// ---- projector with per-angle detector offsets and its derivatives (the
+// reference's positions and double precision; else kernels_single.cu) ----------
 template <typename Real>
 void launch_radon_off(const DevGeom<Real>& g, int S, const Real* img, const Real* off, Real* sino, cudaStream_t st)
 {
     dim3 blk(32, 4), grd((g.N + 31) / 32, (g.T + 3) / 4, S);
-    if constexpr (sizeof(Real) == 4) {
-        if (g.exact) {
-            k_radon<Real, 1, true><<<grd, blk, 0, st>>>(img, g.sc_fp, g.xsc_fp, sino, g.N, g.T, g.mid, off);
-            return;
-        }
-    }
     k_radon<Real, 1, false><<<grd, blk, 0, st>>>(img, g.sc_fp, g.xsc_fp, sino, g.N, g.T, g.mid, off);
 }
 template <typename Real>
@@ -1082,28 +1071,22 @@ void launch_radon_adjoint_off(const DevGeom<Real>& g, int S, const Real* sino, c
                               cudaStream_t st)
 {
     dim3 blk(32, 8), grd((g.N + 31) / 32, (g.N + 7) / 8, S);
-    if constexpr (sizeof(Real) == 4) {
-        if (g.exact) {
-            k_radon_adjoint<Real, 1, true><<<grd, blk, 0, st>>>(sino, g.sc_fp, g.xsc_fp, img, g.N, g.T, g.mid, off);
-            return;
-        }
-    }
-    k_radon_adjoint<Real, 1, false><<<grd, blk, 0, st>>>(sino, g.sc_fp, g.xsc_fp, img, g.N, g.T, g.mid, off);
+    k_radon_adjoint<Real, 1><<<grd, blk, 0, st>>>(sino, g.sc_fp, img, g.N, g.T, g.mid, off);
 }
 
 // D(jy,theta) = d/d(off) of the projector's value: (1/N) sum_jx of the
 // bilinear gradient along the detector direction, dB/dx * (-sin) + dB/dy * cos.
-template <typename Real, bool EX>
+template <typename Real>
 __global__ void __launch_bounds__(128) k_radon_doff(const Real* __restrict__ img, const Real* __restrict__ sc,
-                                                    const float4* __restrict__ xsc, Real* __restrict__ dsino, int N,
-                                                    int T, Real mid, const Real* __restrict__ off)
+                                                    Real* __restrict__ dsino, int N, int T, Real mid,
+                                                    const Real* __restrict__ off)
 {
     const int jy = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int t = blockIdx.y * blockDim.y + threadIdx.y;
     const int g = blockIdx.z;
     if (jy > N || t >= T) return;
     const Real s = sc[2 * t], c = sc[2 * t + 1];
-    const ProjRay<Real, EX> ray(sc, xsc, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
+    const ProjRay<Real, false> ray(sc, nullptr, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
     const Real* u = img + (size_t)g * N * N;
     Real acc = Real(0);
     for (int jx = 1; jx <= N; ++jx) {
@@ -1124,13 +1107,7 @@ template <typename Real>
 void launch_radon_doff(const DevGeom<Real>& g, int S, const Real* img, const Real* off, Real* dsino, cudaStream_t st)
 {
     dim3 blk(32, 4), grd((g.N + 31) / 32, (g.T + 3) / 4, S);
-    if constexpr (sizeof(Real) == 4) {
-        if (g.exact) {
-            k_radon_doff<Real, true><<<grd, blk, 0, st>>>(img, g.sc_fp, g.xsc_fp, dsino, g.N, g.T, g.mid, off);
-            return;
-        }
-    }
-    k_radon_doff<Real, false><<<grd, blk, 0, st>>>(img, g.sc_fp, g.xsc_fp, dsino, g.N, g.T, g.mid, off);
+    k_radon_doff<Real><<<grd, blk, 0, st>>>(img, g.sc_fp, dsino, g.N, g.T, g.mid, off);
 }
 template void launch_radon_off<float>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);
 template void launch_radon_off<double>(const DevGeom<double>&, int, const double*, const double*, double*,

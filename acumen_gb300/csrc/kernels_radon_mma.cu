@@ -37,6 +37,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "ray_weights.cuh"
 #include "umma.cuh"
 
 namespace acu {
@@ -79,50 +80,6 @@ __device__ __forceinline__ float window_lo(const MmaAngle& a, float mid, int x0,
     const float ex = (float)(a.s >= 0.f ? x0 + TP - 1 : x0) - mid;
     const float ey = (float)(a.c >= 0.f ? y0 : y0 + TP - 1) - mid;
     return __fsub_rn(__fmaf_rn(-a.s, ex, __fmaf_rn(a.c, ey, mid)), a.reach);
-}
-
-// The weights of the three rays j, j+1, j+2 nearest to pixel
-// (px, py) (ex, ey: relative to the middle).  Ray j's samples sit at the pixel's
-// distance (dx, dy) = (c e - s d, s e + c d) with d = j - w, e = k - u, where
-// (u, w) are the pixel's coordinates along and across the rays; the bilinear
-// weight of a sample is (1 - |dx|)+ (1 - |dy|)+.  Of the integers e + u only the
-// three nearest to the ray's closest approach reach the pixel.
-template <bool EDGE>
-__device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float ey, float mid, int px, int py, int N,
-                                            int& j, float (&wv)[3])
-{
-    float cu, cw, uf, wf;
-    split_floor(__fmaf_rn(a.x.y, ex, __fmaf_rn(a.x.x, ey, mid)), __fmaf_rn(a.x.w, ex, __fmul_rn(a.x.z, ey)), cu, uf);
-    split_floor(__fmaf_rn(-a.x.x, ex, __fmaf_rn(a.x.y, ey, mid)), __fmaf_rn(-a.x.z, ex, __fmul_rn(a.x.w, ey)), cw, wf);
-    const float i0 = wf > 0.5f ? 0.f : -1.f;   // |d| < |c| + |s| <= 1.42 leaves three candidates
-    j = (int)(cw + i0);
-    const float d0 = i0 - wf;
-    const float2 along = make_float2(a.c, a.s), back = make_float2(-a.c, -a.s), across = make_float2(-a.s, a.c);
-    const float2 one = make_float2(1.f, 1.f);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const float d = d0 + (float)r;
-        const float ctr = __fmaf_rn(a.t, d, uf);
-        const float kf = __fsub_rn(__fadd_rn(ctr, 12582912.f), 12582912.f);   // nearest integer
-        const float e = kf - uf;
-        const float2 p0 = fma2(along, make_float2(e, e), mul2(across, make_float2(d, d)));
-        float w = 0.f;
-#pragma unroll
-        for (int q = -1; q <= 1; ++q) {
-            const float2 p = q < 0 ? fma2(back, one, p0) : q > 0 ? fma2(along, one, p0) : p0;
-            const float hx = __saturatef(1.f - fabsf(p.x)), hy = __saturatef(1.f - fabsf(p.y));
-            if constexpr (EDGE) {
-                // the sample has to exist (step 1..N) and to lie in a valid cell
-                const float k = cu + kf + (float)q;
-                const bool ok = k >= 1.f && k <= (float)N && p.x >= (float)(2 - px) && p.x < (float)(N - px) &&
-                                p.y >= (float)(2 - py) && p.y < (float)(N - py);
-                w = ok ? fmaf(hx, hy, w) : w;
-            } else {
-                w = fmaf(hx, hy, w);
-            }
-        }
-        wv[r] = w;
-    }
 }
 
 __device__ __forceinline__ uint32_t pack(float a, float b)   // a in the low half
@@ -220,14 +177,13 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                 const bool live = t < groups[g + 1];
                 MmaAngle a;
                 int j0 = 0;
-                bool edge = false;
+                bool ends = false;
                 if (live) {
                     a = ang[t];
                     j0 = (int)ceilf(window_lo(a, mid, x0, y0));
-                    // samples of pixels at the rim of the image or at the ends of the rays need their own tests
                     const float uc = fmaf(a.c, (float)x0 + 7.5f - mid, fmaf(a.s, (float)y0 + 7.5f - mid, mid));
                     const float ur = 7.5f * a.reach + 4.f;
-                    edge = rim || uc - ur < 1.f || uc + ur > (float)N;
+                    ends = uc - ur < 1.f || uc + ur > (float)N;   // some rays may end in the tile
                 }
 #pragma unroll 1
                 for (int q0 = 0; q0 < PARTS && ok; q0 += STAGES)
@@ -242,10 +198,13 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                         const float ey = (float)py - mid;
                         float wv[3];
                         int j;
-                        if (edge)
-                            ray_weights<true>(a, ex, ey, mid, px, py, N, j, wv);
-                        else
-                            ray_weights<false>(a, ex, ey, mid, px, py, N, j, wv);
+                        if (rim) {
+                            ray_weights<RIM>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                        } else if (ends) {
+                            ray_weights<ENDS>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                        } else {
+                            ray_weights<INNER>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                        }
                         // the leading 11 bits are exact in half precision, the rest is rounded
                         float hi[3];
 #pragma unroll

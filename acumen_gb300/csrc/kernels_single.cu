@@ -1,6 +1,6 @@
 // Kernels that carry one slice per thread at exact positions: projector
-// (tomography/tv_hpc.F90:129-159) and filtered backprojection's second half
-// (:107-123).
+// (tomography/tv_hpc.F90:129-159) with its offset derivative, filtered
+// backprojection's second half (:107-123), and the projector's exact transpose.
 // Batches share a sample position among four slices or more; here the position
 // is most of the work, so it is kept in fixed point (fixed.cuh).
 #include <algorithm>
@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "fixed.cuh"
 #include "kernels.h"
+#include "ray_weights.cuh"
 
 namespace acu {
 
@@ -32,6 +33,71 @@ __global__ void __launch_bounds__(128, 12) k_ray_fx(const float* __restrict__ I,
     const float v = llabs(a.c) > llabs(a.s) ? fx_ray<true>(IT + g * N * N, N, a, ray, jy, lane)
                                             : fx_ray<false>(I + g * N * N, N, a, ray, jy, lane);
     if (jy <= N) sino[(g * T + t) * N + (jy - 1)] = v / (float)N;
+}
+
+// Projection with per-angle detector offsets and, GRAD, its derivative with
+// respect to them, from one walk along staggered rays (as fx_ray) where the
+// general kernels (k_radon, k_radon_doff) walk twice and read a column of the
+// image per step.  Positions, taps and the order of the sums are theirs: the loss
+// is a sum of squares of these values, and the derivative jumps where a sample
+// changes its cell, so neither would stand another rounding.
+// Held by the instructions of the positions.  Two slices, 1025^2 x 600: 3.31 ms the
+// projection and 3.40 ms the derivative there, 2.65 ms both here.
+template <bool TR, bool GRAD>
+__device__ __forceinline__ void ray_off(const float* __restrict__ base, int N, float s, float c,
+                                        const ProjRay<float, true>& ray, float mid, int jy, float off, int lane,
+                                        float& sum, float& der)
+{
+    const float ratio = TR ? -s / c : c / s;
+    const int kb = __float2int_rn((float)lane * ratio);
+    int lo, hi;
+    valid_steps(s, c, (float)jy - mid + off, mid, N, lo, hi);
+    if (jy > N || !(fabsf(off) < 4.f * N) || lo > hi) {   // no ray, no number, or too far out to meet a pixel
+        lo = 0x3fffffff;
+        hi = -0x3fffffff;
+    }
+    const int i0 = __reduce_min_sync(0xffffffffu, lo + kb), i1 = __reduce_max_sync(0xffffffffu, hi + kb);
+#pragma unroll 2
+    for (int i = i0; i <= i1; ++i) {
+        const int jx = i - kb;
+        int x1, y1;
+        float wxl, wxh, wyl, wyh;
+        ray.at((float)jx - mid, x1, y1, wxl, wxh, wyl, wyh);
+        if (jx >= lo && jx <= hi && min(x1, y1) > 1 && max(x1, y1) < N) {
+            const float* p = base + (TR ? (unsigned)((x1 - 1) * N + y1 - 1) : (unsigned)((y1 - 1) * N + x1 - 1));
+            const float a = __ldg(p), b = __ldg(p + (TR ? N : 1)), cc = __ldg(p + (TR ? 1 : N)), d = __ldg(p + N + 1);
+            const float w11 = wxl * wyl, w21 = wxh * wyl, w12 = wxl * wyh, w22 = wxh * wyh;
+            sum = fmaf(d, w22, fmaf(cc, w12, fmaf(b, w21, fmaf(a, w11, sum))));
+            if constexpr (GRAD) {
+                const float gx = (b - a) * wyl + (d - cc) * wyh;
+                const float gy = (cc - a) * wxl + (d - b) * wxh;
+                der += gy * c - gx * s;
+            }
+        }
+    }
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(128) k_ray_off(const float* __restrict__ I, const float* __restrict__ IT,
+                                                 const float* __restrict__ sc, const float4* __restrict__ xsc,
+                                                 const int* __restrict__ order, const float* __restrict__ off,
+                                                 float* __restrict__ sino, float* __restrict__ dsino, int N, int T,
+                                                 float mid)
+{
+    const int nb = (N + 127) / 128, lane = threadIdx.x, t = order[blockIdx.x / nb];
+    const int jy = blockIdx.x % nb * 128 + threadIdx.y * 32 + lane + 1;
+    const size_t g = blockIdx.z;
+    const float s = sc[2 * t], c = sc[2 * t + 1], o = off ? off[g * T + t] : 0.f;
+    const ProjRay<float, true> ray(sc, xsc, t, jy, mid, off ? off + g * T + t : nullptr);
+    float v = 0.f, d = 0.f;
+    if (fabsf(c) > fabsf(s))
+        ray_off<true, GRAD>(IT + g * N * N, N, s, c, ray, mid, jy, o, lane, v, d);
+    else
+        ray_off<false, GRAD>(I + g * N * N, N, s, c, ray, mid, jy, o, lane, v, d);
+    if (jy > N) return;
+    const size_t at = (g * T + t) * N + (jy - 1);
+    sino[at] = v / (float)N;
+    if constexpr (GRAD) dsino[at] = d / (float)N;
 }
 
 // Held by issue slots: an update is one 64-bit load, an addition, a shift, a
@@ -62,6 +128,90 @@ __global__ void __launch_bounds__(256) k_backproject_fx(const float2* __restrict
 #pragma unroll
     for (int r = 0; r < R; ++r)
         if (x < N && y + r < N) o[(size_t)(y + r) * N + x] = cm[r] != 0.f ? cm[r] * v[r] : 0.f;
+}
+
+template <int V>
+__device__ __forceinline__ void add_rays(Lanes<float, V>& acc, const float* __restrict__ y, const float (&w)[3], int j,
+                                         int N)
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        if ((unsigned)(j + r - 1) < (unsigned)N && w[r] != 0.f) {
+            const Lanes<float, V> v = ld_lanes<float, V>(y + (size_t)(j + r - 1) * V);
+#pragma unroll
+            for (int k = 0; k < V; ++k) acc.v[k] = fmaf(w[r], v.v[k], acc.v[k]);
+        }
+}
+
+template <int V>
+__device__ __forceinline__ void put_image(float* __restrict__ img, Lanes<float, V> acc, size_t g, int px, int py, int N)
+{
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc.v[k] = acc.v[k] / (float)N;
+    st_lanes<float, V>(img + (g * N * N + (size_t)(py - 1) * N + (px - 1)) * V, acc);
+}
+
+// Exact transpose of the projector, as a gather over the angles: the at most
+// three rays whose samples read the pixel, each with the sum of its samples'
+// weights there.  The general kernel (k_radon_adjoint) evaluates the projector at
+// 16 candidate samples per pixel and angle; this one evaluates the nine bilinear
+// weights that can differ from zero, from one position (ray_weights.cuh): held by
+// those instructions.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.65,
+// 1449^2 x 900 66.0 / 7.5, 2049^2 x 1200 170.9 / 19.2.  V slices per thread; off:
+// per-slice angle offsets or null (V = 1).
+template <int V>
+__global__ void __launch_bounds__(256) k_adjoint_fx(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
+                                                    const float* __restrict__ off, float* __restrict__ img, int N,
+                                                    int T, float mid)
+{
+    const int px = blockIdx.x * 32 + threadIdx.x + 1, py = blockIdx.y * 8 + threadIdx.y + 1;
+    const size_t g = blockIdx.z;
+    if (px > N || py > N || on_rim(px, py, N)) return;   // the rim: k_adjoint_rim
+    Lanes<float, V> acc{};
+    const float ex = (float)px - mid, ey = (float)py - mid;
+    const float* y = sino + g * T * N * V;
+#pragma unroll 1
+    for (int t = 0; t < T; ++t, y += (size_t)N * V) {
+        const MmaAngle a = ang[t];
+        const float o = off ? __ldg(off + g * T + t) : 0.f;
+        const float u = fmaf(a.c, ex, fmaf(a.s, ey, mid));
+        int j;
+        float w[3];
+        if (u < 4.f || u > (float)N - 3.f)
+            ray_weights<ENDS>(a, ex, ey, o, mid, px, py, N, j, w);
+        else
+            ray_weights<INNER>(a, ex, ey, o, mid, px, py, N, j, w);
+        add_rays<V>(acc, y, w, j, N);
+    }
+    put_image<V>(img, acc, g, px, py, N);
+}
+
+// The pixels on the rim, whose samples may lie outside and are looked at one by one: 40 times the work, so in a kernel
+// of their own (in k_adjoint_fx their warps would be the last to end).  One pixel per warp, its lanes sharing out the angles (grid.x: 6 N pixels, grid.y: slices).
+template <int V>
+__global__ void __launch_bounds__(256) k_adjoint_rim(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
+                                                     const float* __restrict__ off, float* __restrict__ img, int N,
+                                                     int T, float mid)
+{
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, side = i / N, at = i % N + 1;
+    if (side > 5) return;
+    // columns 1, 2, N and rows 1, 2, N (corners twice, with the same value)
+    const int edge = side % 3 == 2 ? N : side % 3 + 1;
+    const int px = side < 3 ? edge : at, py = side < 3 ? at : edge;
+    const size_t g = blockIdx.y;
+    Lanes<float, V> acc{};
+    if (px >= 2 && py >= 2)   // a pixel of the first column or row is never a tap (taps span 2..N)
+        for (int t = lane; t < T; t += 32) {
+            int j;
+            float w[3];
+            ray_weights<RIM>(ang[t], (float)px - mid, (float)py - mid, off ? off[g * T + t] : 0.f, mid, px, py, N, j, w);
+            add_rays<V>(acc, sino + (g * T + t) * N * V, w, j, N);
+        }
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc.v[k] += __shfl_down_sync(0xffffffffu, acc.v[k], o);
+    if (lane == 0) put_image<V>(img, acc, g, px, py, N);
 }
 
 // bins -> pairs (bin, next bin), zeros in the first and the last
@@ -97,6 +247,17 @@ void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT
                                                                      g.T, g.mid);
 }
 
+void launch_ray_off(const DevGeom<float>& g, int S, const float* img, float* IT, const float* off, float* sino,
+                    float* dsino, cudaStream_t st)
+{
+    launch_transpose_v1(g.N, S, img, IT, st);
+    const dim3 blk(32, 4), grd((g.N + 127) / 128 * g.T, 1, S);
+    if (dsino)
+        k_ray_off<true><<<grd, blk, 0, st>>>(img, IT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
+    else
+        k_ray_off<false><<<grd, blk, 0, st>>>(img, IT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
+}
+
 void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, float* img, cudaStream_t st)
 {
     const dim3 blk(32, 8);
@@ -110,6 +271,16 @@ void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, floa
     else
         k_backproject_fx<4><<<grid(4), blk, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, g.mid);
 }
+
+template <int V>
+void launch_adjoint_fx(const DevGeom<float>& g, int G, const float* sino, const float* off, float* img, cudaStream_t st)
+{
+    k_adjoint_fx<V><<<dim3((g.N + 31) / 32, (g.N + 7) / 8, G), dim3(32, 8), 0, st>>>(sino, g.mma, off, img, g.N, g.T,
+                                                                                     g.mid);
+    k_adjoint_rim<V><<<dim3((6 * g.N + 7) / 8, G), 256, 0, st>>>(sino, g.mma, off, img, g.N, g.T, g.mid);
+}
+template void launch_adjoint_fx<1>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);
+template void launch_adjoint_fx<4>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);
 
 void launch_pairs(const float* q, float2* out, int N, size_t n, cudaStream_t st)
 {

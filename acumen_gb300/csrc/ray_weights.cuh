@@ -1,0 +1,87 @@
+// The projector's weights seen from a pixel (exact positions): shared by the
+// tensor-core projector, which gathers them into a matrix, and the transpose.
+#pragma once
+#include "common.cuh"
+#include "kernels.h"
+
+namespace acu {
+
+// Whether step k of ray j lies in a valid cell, by the projector's arithmetic (ProjRay, common.cuh).
+__device__ __forceinline__ bool sample_valid(float4 x, float k, int j, float off, float mid, int N)
+{
+    const float dy = (float)j - mid, dx = k - mid;
+    float cx, cy, f;
+    split_floor(__fmaf_rn(x.y, dx, __fmaf_rn(-x.x, dy, mid)),
+                __fmaf_rn(x.w, dx, __fmaf_rn(-x.x, off, __fmaf_rn(-x.z, off, __fmul_rn(-x.z, dy)))), cx, f);
+    split_floor(__fmaf_rn(x.x, dx, __fmaf_rn(x.y, dy, mid)),
+                __fmaf_rn(x.z, dx, __fmaf_rn(x.y, off, __fmaf_rn(x.w, off, __fmul_rn(x.w, dy)))), cy, f);
+    return fminf(cx, cy) > 1.f && fmaxf(cx, cy) < (float)N;
+}
+
+// The weights of the three rays j, j+1, j+2 nearest to pixel (px, py) (ex, ey:
+// relative to the middle; off: the angle's detector offset).  Ray j's samples sit
+// at the pixel's distance (dx, dy) = (c e - s d, s e + c d) with d = j - w,
+// e = k - u, where (u, w) are the pixel's coordinates along and across the rays;
+// the bilinear weight of a sample is (1 - |dx|)+ (1 - |dy|)+.  Of the integers
+// e + u only the three nearest to the ray's closest approach reach the pixel.
+// INNER: every sample that reaches the pixel exists and is valid; ENDS: some may
+// lie beyond a ray's ends; RIM: some may lie in a cell outside 2..N-1 too.
+enum { INNER, ENDS, RIM };
+
+template <int WHERE>
+__device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float ey, float off, float mid, int px, int py,
+                                            int N, int& j, float (&wv)[3])
+{
+    float cu, cw, uf, wf;
+    split_floor(__fmaf_rn(a.x.y, ex, __fmaf_rn(a.x.x, ey, mid)), __fmaf_rn(a.x.w, ex, __fmul_rn(a.x.z, ey)), cu, uf);
+    split_floor(__fmaf_rn(-a.x.x, ex, __fmaf_rn(a.x.y, ey, mid)), __fmaf_rn(-a.x.z, ex, __fmul_rn(a.x.w, ey)) - off, cw, wf);
+    const float i0 = wf > 0.5f ? 0.f : -1.f;   // |d| < |c| + |s| <= 1.42 leaves three candidates
+    j = (int)(cw + i0);
+    const float d0 = i0 - wf;
+    const float2 along = make_float2(a.c, a.s), back = make_float2(-a.c, -a.s), across = make_float2(-a.s, a.c);
+    const float2 one = make_float2(1.f, 1.f);
+    if constexpr (WHERE == RIM) wv[0] = wv[1] = wv[2] = 0.f;
+    // rolled at the rim, which few pixels meet: its code and registers would cost all the others
+#pragma unroll (WHERE == RIM ? 1 : 3)
+    for (int r = 0; r < 3; ++r) {
+        const float d = d0 + (float)r;
+        const float ctr = __fmaf_rn(a.t, d, uf);
+        const float kf = __fsub_rn(__fadd_rn(ctr, 12582912.f), 12582912.f);   // nearest integer
+        const float e = kf - uf;
+        const float2 p0 = fma2(along, make_float2(e, e), mul2(across, make_float2(d, d)));
+        float w = 0.f;
+#pragma unroll (WHERE == RIM ? 1 : 3)
+        for (int q = -1; q <= 1; ++q) {
+            const float2 p = WHERE == RIM ? fma2(along, make_float2((float)q, (float)q), p0) : q < 0 ? fma2(back, one, p0) : q > 0 ? fma2(along, one, p0) : p0;
+            const float hx = __saturatef(1.f - fabsf(p.x)), hy = __saturatef(1.f - fabsf(p.y));
+            if constexpr (WHERE == INNER) {
+                w = fmaf(hx, hy, w);
+            } else {
+                const float k = cu + kf + (float)q;
+                bool ok = k >= 1.f && k <= (float)N;
+                if constexpr (WHERE == RIM) {
+                    // within 1e-5 of a cell edge at the rim the projector's own position decides
+                    const float xl = p.x - (float)(2 - px), xh = p.x - (float)(N - px);
+                    const float yl = p.y - (float)(2 - py), yh = p.y - (float)(N - py);
+                    if (fminf(fminf(fabsf(xl), fabsf(xh)), fminf(fabsf(yl), fabsf(yh))) < 1e-5f)
+                        ok = ok && sample_valid(a.x, k, j + r, off, mid, N);
+                    else
+                        ok = ok && xl >= 0.f && xh < 0.f && yl >= 0.f && yh < 0.f;
+                }
+                w = ok ? fmaf(hx, hy, w) : w;
+            }
+        }
+        if constexpr (WHERE == RIM) {
+            wv[0] = r == 0 ? w : wv[0];
+            wv[1] = r == 1 ? w : wv[1];
+            wv[2] = r == 2 ? w : wv[2];
+        } else {
+            wv[r] = w;
+        }
+    }
+}
+
+// pixels whose taps can belong to samples outside the valid cells
+__device__ __forceinline__ bool on_rim(int px, int py, int N) { return px < 3 || py < 3 || px >= N || py >= N; }
+
+}  // namespace acu

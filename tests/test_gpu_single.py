@@ -1,5 +1,6 @@
 """Kernels that carry one slice per thread at exact positions: positions in fixed
-point (projector, backprojection of one to three slices, ragged batches).
+point (projector, backprojection of one to three slices, ragged batches), the
+projector's transpose and the projection with detector offsets.
 
 They read the samples the four-slice gather kernels read and round in another
 order; both stay within ~1e-6 of FP64 in relative L2 (tests of the operators), so
@@ -42,6 +43,52 @@ def test_one_slice_against_the_gather_kernels(N, T, S):
         assert rel(t.backproject(q)[:1], bp) < 3e-6
         fbp = four(t.iradon, q)
         assert rel(t.iradon(q)[:1], fbp) < 3e-6
+    t.close()
+
+
+@pytest.mark.parametrize("N, T, S", [(3, 9, 1), (16, 9, 4), (33, 40, 1), (64, 37, 3), (129, 30, 5), (257, 12, 1)])
+def test_transpose_matches_the_projector(N, T, S):
+    """<A x, y> = <x, A' y> per pixel of the rim too: x is one pixel at a time there."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    t = Tomography(N, axes(T), 2)
+    y = torch.rand(S, T, N, device="cuda", generator=g)
+    at = t.radon_adjoint(y)
+    x = torch.rand(S, N, N, device="cuda", generator=g)
+    lhs, rhs = float((t.radon(x).double() * y).sum()), float((x.double() * at).sum())
+    assert abs(lhs - rhs) <= 1e-6 * abs(lhs)
+    rim = torch.zeros(N, N, device="cuda")
+    rim[:2] = rim[:, :2] = rim[-1] = rim[:, -1] = 1
+    z = torch.zeros(4, N, N, device="cuda")
+    z[0] = rim
+    z[1, N - 1, N // 2] = z[2, 1, N // 2] = z[3, N // 2, N - 1] = 1
+    r = t.radon(z)
+    for k in range(4):
+        lhs, rhs = float((r[k].double() * y[0]).sum()), float((z[k].double() * at[0]).sum())
+        assert abs(lhs - rhs) <= 2e-6 * max(abs(lhs), 1e-3)
+    t.close()
+
+
+@pytest.mark.parametrize("N, T", [(33, 20), (129, 90), (200, 61)])
+def test_offsets_loss_and_gradients(N, T):
+    """Against the double-precision kernels, offsets among them that leave the grid or are not numbers."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    t = Tomography(N, (syn.angles(T) + 0.17).astype(np.float32), 4)
+    S = 2
+    u = torch.rand(S, N, N, device="cuda", generator=g)
+    off = 2.0 * torch.randn(S, T, device="cuda", generator=g)
+    y = torch.rand(S, T, N, device="cuda", generator=g)
+    off[0, 1], off[0, 2] = 3.0 * N, 1e30
+    l32, gu, go = t.tv_loss_grad(u, off, y, 0.05, 0.05)
+    l64, gd, _ = t.tv_loss_grad(u.double(), off.double(), y.double(), 0.05, 0.05)
+    np.testing.assert_allclose(l32, l64, rtol=1e-6)
+    assert rel(gu, gd) < 2e-6
+    assert not go[0, 1:3].any()
+    off[0, 3] = float("nan")
+    l32, gu2, go2 = t.tv_loss_grad(u, off, y, 0.05, 0.05)
+    assert np.isfinite(l32).all() and torch.isfinite(gu2).all() and float(go2[0, 3]) == 0.0
+    only, none, _ = t.tv_loss_grad(u, None, y, 0.05, 0.05, want_grad=False)
+    np.testing.assert_allclose(only, t.tv_loss_grad(u, torch.zeros_like(off), y, 0.05, 0.05)[0], rtol=1e-12)
+    assert none is None
     t.close()
 
 
