@@ -242,27 +242,159 @@ __device__ __forceinline__ __int128 shfl_down_i128(__int128 v, int o)
     return ((__int128)hi << 64) | (__int128)lo;
 }
 
-__global__ void __launch_bounds__(256) k_xcorr(int ndet, int nrows, int kmax, const float* __restrict__ p0,
-                                               const float* __restrict__ p180, unsigned long long* __restrict__ w)
+// A block takes XC_LAGS lags and, one by one, its share of the frame's items (a
+// row's stretch of XC_X pixels).  In integers, a product is the 48-bit product of
+// two mantissas shifted right by what both exponents say, which is its floor at
+// 2^-32: six instructions.  (In FP64, of which an SM does two a clock, with the
+// conversion to 64 bits, 2048 x 256 pixels and 1025 lags took 5.24 ms; so: 0.24 ms,
+// with products of 2^14 and more 0.5 ms.)
+// Both operands are staged as (mantissa * 2^7, 14 - exponent), a product of two
+// is shifted right by the sum of the second parts; a thread takes 8 pixels x 8 lags from
+// 8 + 15 of them, read at a pitch of 9 per 8, so that neither 8-element stride meets a
+// bank twice.  An item's largest magnitudes say how: below 2^14 its floors add up in 64
+// bits; below 2^31 the shift may go left by up to two, and high and low words add
+// up apart; else, or with a value that is not finite, product by product in FP64.
+constexpr int XC_X = 1024, XC_LAGS = 64, XC_ITEMS = 256;   // XC_ITEMS: items a block sums up in 64 bits at most
+constexpr int XC_Q = XC_X + XC_LAGS;
+
+__device__ __forceinline__ int xc_slot(int i) { return i + (i >> 3); }
+__device__ __forceinline__ int2 xc_split(float v, unsigned& top)
 {
-    const int k = (int)blockIdx.y - kmax;
-    const long n = (long)ndet * nrows;
-    __int128 acc = 0;
-    bool bad = false;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % ndet), y = (int)(i / ndet);
-        const int xm = ndet - 1 - x + k;
-        if (xm >= 0 && xm < ndet) {
-            const double p = (double)p0[i] * (double)p180[(size_t)y * ndet + xm];   // exact
-            if (fabs(p) < kFixLimit) acc += (__int128)__double2ll_rd(p * kFixScale);
-            else bad = true;                                                          // also NaN
+    const unsigned b = __float_as_uint(v);
+    const int e = (int)(b >> 23 & 255u);
+    top = max(top, b & 0x7fffffffu);
+    const int m = (int)((b & 0x7fffffu) << 7 | (e ? 0x40000000u : 0u));
+    return make_int2((int)b < 0 ? -m : m, 14 + 127 - max(e, 1));
+}
+// v >> n, n = 0..; 63 and more leave the sign
+__device__ __forceinline__ long long shr_floor(long long v, int n)
+{
+    long long r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+}
+
+// what(j, product of the mantissas, shift) for a thread's pixels and its lags lg * 8 + j (n: pixels in the stretch)
+template <class F>
+__device__ __forceinline__ void xc_products(const int2* s_a, const int2* s_q, int xg, int lg, int n, F&& what)
+{
+#pragma unroll 1
+    for (int x8 = xg; x8 < XC_X / 8 && x8 * 8 < n; x8 += 32) {
+        const int2* pa = s_a + x8 * 9;
+        const int2* pq = s_q + (x8 - lg + XC_LAGS / 8) * 9;   // q of the first pixel at the first lag
+        int2 b[15];
+#pragma unroll
+        for (int j = 0; j < 15; ++j) b[j] = pq[j < 7 ? j - 8 : j - 7];   // pixel - lag = j - 7
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            const int2 v = pa[x];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int2 u = b[x - j + 7];
+                what(j, (long long)v.x * u.x, v.y + u.y);
+            }
         }
     }
+}
+
+// adds the sums of the four lanes with the same lags to the warp's
+__device__ __forceinline__ void xc_gather(__int128 v, __int128* sum, int lag)
+{
+    v += shfl_down_i128(v, 16);
+    v += shfl_down_i128(v, 8);
+    if ((threadIdx.x & 31) < 8) sum[lag] += v;
+}
+
+__global__ void __launch_bounds__(256, 2) k_xcorr(int ndet, int nrows, int kmax, const float* __restrict__ p0,
+                                               const float* __restrict__ p180, unsigned long long* __restrict__ w)
+{
+    __shared__ int2 s_a[XC_X * 9 / 8], s_q[XC_Q * 9 / 8];
+    __shared__ unsigned s_top[2][2];
+    __shared__ __int128 s_sum[8][XC_LAGS];
+    const int tid = threadIdx.x, lg = tid & 7, xg = tid >> 3;
+    const int nk = 2 * kmax + 1, i0 = blockIdx.y * XC_LAGS;
+    const int nxt = (ndet + XC_X - 1) / XC_X, items = nxt * nrows;
+    long long acc[8];
+    bool bad = false;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += shfl_down_i128(acc, o);
-    if ((threadIdx.x & 31) == 0 && acc != 0) atomic_add_i128(&w[2 * blockIdx.y], acc);
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) {
-        unsigned int* flag = reinterpret_cast<unsigned int*>(w + 2 * (2 * kmax + 1)) + 1;
+    for (int j = 0; j < 8; ++j) acc[j] = 0;
+    if (tid < 4) s_top[tid >> 1][tid & 1] = 0u;
+    for (int i = tid; i < 8 * XC_LAGS; i += 256) s_sum[i / XC_LAGS][i % XC_LAGS] = 0;
+    __syncthreads();
+    int buf = 0;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int y = it / nxt, xt = it % nxt * XC_X;
+        // C(k) = sum_x p0(x) q(x - k), q(z) = p180(ndet - 1 - z); place of q(z): z - z0
+        const int z0 = xt - i0 - XC_LAGS + kmax;
+        if (z0 >= ndet || z0 + XC_Q <= 0) continue;   // no partner for any of its pixels
+        const float* a = p0 + (size_t)y * ndet;
+        const float* q = p180 + (size_t)y * ndet;
+        unsigned ta = 0u, tq = 0u;
+        for (int i = tid; i < XC_X; i += 256)
+            s_a[xc_slot(i)] = xc_split(xt + i < ndet ? __ldg(a + xt + i) : 0.f, ta);
+        for (int i = tid; i < XC_Q; i += 256) {
+            const int z = z0 + i;
+            s_q[xc_slot(i)] = xc_split(z >= 0 && z < ndet ? __ldg(q + ndet - 1 - z) : 0.f, tq);
+        }
+        ta = __reduce_max_sync(0xffffffffu, ta);
+        tq = __reduce_max_sync(0xffffffffu, tq);
+        if ((tid & 31) == 0) {
+            atomicMax(&s_top[buf][0], ta);
+            atomicMax(&s_top[buf][1], tq);
+        }
+        __syncthreads();
+        const double top = (double)__uint_as_float(s_top[buf][0]) * (double)__uint_as_float(s_top[buf][1]);
+        const bool finite = max(s_top[buf][0], s_top[buf][1]) < 0x7f800000u;
+        if (tid < 2) s_top[buf ^ 1][tid] = 0u;
+        buf ^= 1;
+        if (finite && top < 16384.) {
+            xc_products(s_a, s_q, xg, lg, ndet - xt, [&](int j, long long m, int n) { acc[j] += shr_floor(m, n); });
+        } else if (finite && top < kFixLimit) {
+            long long hi[8];
+            unsigned long long lo[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                hi[j] = 0;
+                lo[j] = 0;
+            }
+            xc_products(s_a, s_q, xg, lg, ndet - xt, [&](int j, long long m, int n) {
+                const long long t = shr_floor(m, max(n, 0)) << max(-n, 0);
+                hi[j] += t >> 32;
+                lo[j] += (unsigned)t;
+            });
+#pragma unroll
+            for (int j = 0; j < 8; ++j) xc_gather(((__int128)hi[j] << 32) + lo[j], s_sum[tid >> 5], lg * 8 + j);
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+                const int i = i0 + lg * 8 + j;
+                __int128 v = 0;
+                if (i < nk)
+#pragma unroll 1
+                    for (int x = xt + xg; x < min(xt + XC_X, ndet); x += 32) {
+                        const int z = x - (i - kmax);
+                        if (z < 0 || z >= ndet) continue;
+                        const double p = (double)a[x] * (double)q[ndet - 1 - z];   // exact
+                        if (fabs(p) < kFixLimit) v += (__int128)__double2ll_rd(p * kFixScale);
+                        else bad = true;                                            // also NaN
+                    }
+                __syncwarp();
+                xc_gather(v, s_sum[tid >> 5], lg * 8 + j);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) xc_gather(acc[j], s_sum[tid >> 5], lg * 8 + j);
+    __syncthreads();
+    if (tid < XC_LAGS && i0 + tid < nk) {
+        __int128 v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += s_sum[k][tid];
+        if (v != 0) atomic_add_i128(&w[2 * (i0 + tid)], v);
+    }
+    if (__any_sync(0xffffffffu, bad) && (tid & 31) == 0) {
+        unsigned int* flag = reinterpret_cast<unsigned int*>(w + 2 * nk) + 1;
         atomicOr(flag, 1u);
     }
 }
@@ -275,13 +407,13 @@ __device__ __forceinline__ bool i128_better(long long ah, unsigned long long al,
     return ai < bi;
 }
 
-// Warp-shuffle argmax over the nk 128-bit correlation values (ties: lowest index).
+// Argmax over the nk 128-bit correlation values (ties: lowest index), one block of 256.
 __global__ void k_argmax(int nk, unsigned long long* __restrict__ w)
 {
     long long bh = LLONG_MIN;
     unsigned long long bl = 0;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < nk; i += 32) {
+    for (int i = threadIdx.x; i < nk; i += 256) {
         const long long h = (long long)w[2 * i + 1];
         const unsigned long long l = w[2 * i];
         if (i128_better(h, l, i, bh, bl, bi)) { bh = h; bl = l; bi = i; }
@@ -293,7 +425,20 @@ __global__ void k_argmax(int nk, unsigned long long* __restrict__ w)
         const int oi = __shfl_down_sync(0xffffffffu, bi, o);
         if (i128_better(oh, ol, oi, bh, bl, bi)) { bh = oh; bl = ol; bi = oi; }
     }
-    if (threadIdx.x == 0) reinterpret_cast<int*>(w + 2 * nk)[0] = bi;
+    __shared__ long long s_h[8];
+    __shared__ unsigned long long s_l[8];
+    __shared__ int s_i[8];
+    if ((threadIdx.x & 31) == 0) {
+        s_h[threadIdx.x >> 5] = bh;
+        s_l[threadIdx.x >> 5] = bl;
+        s_i[threadIdx.x >> 5] = bi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k)
+            if (i128_better(s_h[k], s_l[k], s_i[k], bh, bl, bi)) { bh = s_h[k]; bl = s_l[k]; bi = s_i[k]; }
+        reinterpret_cast<int*>(w + 2 * nk)[0] = bi;
+    }
 }
 
 // ---- 27-point median (:426-452): the reference's descending exchange sort,
@@ -492,10 +637,13 @@ cudaError_t launch_xcorr(int ndet, int nrows, int kmax, const float* p0, const f
     const int nk = 2 * kmax + 1;
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long) * xcorr_scratch_words(kmax), st);
     if (e != cudaSuccess) return e;
-    dim3 grd(nblocks((long)ndet * nrows, 256, 64), nk);
+    // a few blocks for every SM, each with a whole number of items, and no more items than its sums hold
+    const int items = (ndet + XC_X - 1) / XC_X * nrows, tiles = (nk + XC_LAGS - 1) / XC_LAGS;
+    const int want = std::max(1, std::min(items, 152 * 8 / tiles)), per = std::min((items + want - 1) / want, XC_ITEMS);
+    dim3 grd((items + per - 1) / per, tiles);
     e = launch_k(k_xcorr, grd, dim3(256), st, ndet, nrows, kmax, p0, p180, scratch);
     if (e != cudaSuccess) return e;
-    return launch_k(k_argmax, dim3(1), dim3(32), st, nk, scratch);
+    return launch_k(k_argmax, dim3(1), dim3(256), st, nk, scratch);
 }
 
 int xcorr_finish(int kmax, const unsigned long long* h, int64_t* corr_out, int* k_best, double* k_sub,

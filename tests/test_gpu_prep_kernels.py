@@ -1,0 +1,40 @@
+"""Preprocessing kernels at the sizes where they can go wrong: the cross-correlation
+at the edges of its stretches (1024 pixels) and lag tiles (64) and on both sides
+of its magnitude rules.  Everything is bit-exact against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from acumen_gb300.preprocess import Preprocessor
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def pp(built_lib):
+    return Preprocessor()
+
+
+def cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("ndet,nrows,kmax", [(2, 1, 1), (7, 3, 31), (64, 2, 32), (65, 3, 33), (1023, 2, 63), (1024, 3, 64),
+                                             (1025, 2, 256), (2049, 5, 512), (130, 700, 8)])
+@pytest.mark.parametrize("kind", ["logs", "wide", "large"])
+def test_xcorr_tiles(pp, oracle, ndet, nrows, kmax, kind):
+    rng = np.random.default_rng(ndet + nrows)
+    p0 = rng.normal(0.5, 1.0, (nrows, ndet)).astype(np.float32)
+    p180 = (p0[:, ::-1] + rng.normal(0, 0.1, p0.shape)).astype(np.float32)
+    if kind == "wide":      # zeros, denormals, products far below and just below the left shift
+        p0 *= np.exp2(rng.integers(-140, 7, p0.shape)).astype(np.float32)
+        p180 *= np.exp2(rng.integers(-20, 4, p0.shape)).astype(np.float32)
+        p0[rng.random(p0.shape) < 0.1] = 0.0
+        p180[rng.random(p0.shape) < 0.1] = -0.0
+    if kind == "large":     # some stretches take the other route
+        p0[rng.random(p0.shape) < 0.5 / (nrows * ndet) ** 0.5] *= np.float32(3e4)
+        p180[0, ndet // 2] = 5e3
+    kb, ks, corr = pp.xcorr_register(cu(p0), cu(p180), kmax)
+    ko, kso, corr_o = oracle.xcorr_register(p0, p180, kmax)
+    np.testing.assert_array_equal(corr, corr_o)
+    assert kb == ko and ks == pytest.approx(kso, abs=1e-12)
