@@ -1,6 +1,7 @@
 """Preprocessing kernels at the sizes where they can go wrong: the cross-correlation
 at the edges of its stretches (1024 pixels) and lag tiles (64) and on both sides
-of its magnitude rules.  Everything is bit-exact against the oracle."""
+of its magnitude rules, the median at the edges of its tiles (32 x 16 pixels) and
+walks (several projections and two pixels per thread at 400 x 250).  Everything is bit-exact against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -38,3 +39,23 @@ def test_xcorr_tiles(pp, oracle, ndet, nrows, kmax, kind):
     ko, kso, corr_o = oracle.xcorr_register(p0, p180, kmax)
     np.testing.assert_array_equal(corr, corr_o)
     assert kb == ko and ks == pytest.approx(kso, abs=1e-12)
+
+
+@pytest.mark.parametrize("ndet,nrows,nproj", [(2, 1, 1), (31, 15, 2), (32, 16, 3), (33, 17, 16), (65, 33, 17), (5, 2, 33), (400, 250, 34)])
+@pytest.mark.parametrize("special", [False, True])
+def test_median_tiles(pp, oracle, ndet, nrows, nproj, special):
+    rng = np.random.default_rng(ndet * nproj)
+    proj = rng.normal(0, 1, (nproj, nrows, ndet)).astype(np.float32)
+    if special:             # ties, both zeros, infinities, a NaN
+        proj = np.round(proj * 2).astype(np.float32)
+        proj[rng.random(proj.shape) < 0.2] = -0.0
+        proj[rng.random(proj.shape) < 0.02] = np.inf
+        proj[rng.random(proj.shape) < 0.02] = -np.inf
+        proj[nproj // 2, nrows // 2, ndet // 2] = np.nan
+    for p in range(nproj if ndet < 100 else 0):
+        l, r = proj[max(p - 1, 0)], proj[min(p + 1, nproj - 1)]
+        got = pp.median27(cu(l), cu(proj[p]), cu(r)).cpu().numpy()
+        np.testing.assert_array_equal(got.view(np.uint32), oracle.median27(l, proj[p], r).view(np.uint32))
+    with np.errstate(invalid="ignore"):
+        got = pp.proj_to_sino(cu(proj), 0.003, 0.01).cpu().numpy()
+        np.testing.assert_array_equal(got, oracle.proj_to_sino(proj, 0.003, 0.01))
