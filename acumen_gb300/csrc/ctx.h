@@ -111,9 +111,14 @@ struct acu_ctx {
     acu::DevBuf mmaT, mmaP, mmaF; // tiles, partial sums and flags of the tensor-core projector
     acu::DevBuf bpQ, bpS;         // bins in operand layout and per-slice scalars of the tensor-core backprojection
     acu::DevBuf w_part;          // FP64 / int64 partial sums of the preprocessing reductions
+    double* pinned = nullptr;    // their results in host memory (MIRROR_MAX of them)
     acu::TvState<float> tv32;
     acu::TvState<double> tv64;
     std::vector<double> last_delta;
+    ~acu_ctx()
+    {
+        if (pinned) cudaFreeHost(pinned);
+    }
 };
 
 namespace acu {

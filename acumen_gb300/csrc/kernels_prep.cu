@@ -174,23 +174,53 @@ __global__ void k_resample(ResampleGeom g, const float* __restrict__ src, float*
 }
 
 // ---- registration objective (:279-284 / :308-313 / :346-351) ----------------
-// sum |V0(jx,jy) - V180(nx-jx+1,jy)| over the padded grid: one FP64 partial
-// per block, summed afterwards in block order (deterministic).
-__global__ void __launch_bounds__(256) k_mirror_error(ResampleGeom g, const float* __restrict__ p0,
-                                                      const float* __restrict__ p180, double* __restrict__ part)
+// sum |V0(jx,jy) - V180(nx-jx+1,jy)| over the padded grid for up to MIRROR_MAX
+// candidates (grid.y): one FP64 partial per block, summed in block order
+// (deterministic) by the candidate's last block, into host memory.  An evaluation is
+// bound by its latency: one launch and a synchronisation per candidate sweep in place of two
+// launches, a copy and a synchronisation per candidate, and no 64-bit division per
+// pixel, take a search at 1025 x 64 from 27 to 5 us per candidate.
+__global__ void __launch_bounds__(256) k_mirror_errors(int ndet, int nrows, MirrorCandidates cand,
+                                                       const float* __restrict__ p0, const float* __restrict__ p180,
+                                                       double* __restrict__ part, unsigned* __restrict__ done,
+                                                       double* __restrict__ out)
 {
     __shared__ double sh[32];
+    __shared__ bool last;
+    const int k = blockIdx.y, nblk = gridDim.x;
+    const ResampleGeom g{ndet, nrows, ndet % 2 == 0 ? 1 : 0, cand.cth[k], cand.sth[k], cand.shift[k]};
     const int nx = g.ndet + g.add;
-    const long n = (long)nx * g.nrows;
+    const long n = (long)nx * g.nrows, first = blockIdx.x * 256l + threadIdx.x;
+    const int stride = nblk * 256, dx = stride % nx, dy = stride / nx;
+    int jx = (int)(first % nx) + 1, jy = (int)(first / nx) + 1;
     double acc = 0.0;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const int jx = (int)(i % nx) + 1, jy = (int)(i / nx) + 1;
+    for (long i = first; i < n; i += stride) {
         const float a = resample_at(g, p0, jx, jy);
         const float b = resample_at(g, p180, nx - jx + 1, jy);
         acc += (double)fabsf(__fsub_rn(a, b));
+        jx += dx;
+        jy += dy;
+        if (jx > nx) {
+            jx -= nx;
+            ++jy;
+        }
     }
-    const double r = block_sum(acc, sh);
-    if (threadIdx.x == 0 && threadIdx.y == 0) part[blockIdx.x] = r;
+    double r = block_sum(acc, sh);
+    if (threadIdx.x == 0) {
+        part[k * nblk + blockIdx.x] = r;
+        __threadfence();
+        last = atomicAdd(done + k, 1u) == nblk - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    acc = 0.0;
+    for (int i = threadIdx.x; i < nblk; i += 256) acc += __ldcg(part + k * nblk + i);
+    r = block_sum(acc, sh);
+    if (threadIdx.x == 0) {
+        done[k] = 0;
+        out[k] = r;
+    }
 }
 
 // centre-of-mass sums (:234-243): tm, cmx_0, cmx_180 as FP64 partials
@@ -220,14 +250,14 @@ __global__ void __launch_bounds__(256) k_com(int ndet, int nrows, int add, const
     if (threadIdx.x == 0) part[3 * blockIdx.x + 2] = r;
 }
 
-// fixed-order sum of `n` partials with stride `stride` (offset `off`) into out[0]
-__global__ void k_sum_partials(const double* __restrict__ part, int n, int stride, int off, double* __restrict__ out)
+// fixed-order sums of n interleaved partials, one per block, into out[block]
+__global__ void k_sum_partials(const double* __restrict__ part, int n, double* __restrict__ out)
 {
     __shared__ double sh[32];
     double v = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) v += part[(size_t)i * stride + off];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v += part[(size_t)i * gridDim.x + blockIdx.x];
     const double r = block_sum(v, sh);
-    if (threadIdx.x == 0) out[0] = r;
+    if (threadIdx.x == 0) out[blockIdx.x] = r;
 }
 
 // ---- cross-correlation registration (new) --------------------------------------
@@ -705,18 +735,16 @@ int mirror_error_blocks(int ndet, int nrows)
 {
     return (int)nblocks((long)(ndet + 1) * nrows, 256, 1024);
 }
-void launch_mirror_error(int ndet, int nrows, const float* p0, const float* p180, float cth, float sth, float shift,
-                         double* part, int nblk, double* out, cudaStream_t st)
+void launch_mirror_errors(int ndet, int nrows, const float* p0, const float* p180, const MirrorCandidates& cand, int n,
+                          double* part, int nblk, unsigned* done, double* out, cudaStream_t st)
 {
-    ResampleGeom g{ndet, nrows, ndet % 2 == 0 ? 1 : 0, cth, sth, shift};
-    k_mirror_error<<<nblk, 256, 0, st>>>(g, p0, p180, part);
-    k_sum_partials<<<1, 256, 0, st>>>(part, nblk, 1, 0, out);
+    k_mirror_errors<<<dim3(nblk, n), 256, 0, st>>>(ndet, nrows, cand, p0, p180, part, done, out);
 }
 void launch_com(int ndet, int nrows, const float* p0, const float* p180, double* part, int nblk, double* out3,
                 cudaStream_t st)
 {
     k_com<<<nblk, 256, 0, st>>>(ndet, nrows, ndet % 2 == 0 ? 1 : 0, p0, p180, part);
-    for (int j = 0; j < 3; ++j) k_sum_partials<<<1, 256, 0, st>>>(part, nblk, 3, j, out3 + j);
+    k_sum_partials<<<3, 256, 0, st>>>(part, nblk, out3);
 }
 size_t xcorr_scratch_words(int kmax) { return 2 * (size_t)(2 * kmax + 1) + 1; }
 

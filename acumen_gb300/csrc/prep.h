@@ -16,9 +16,15 @@ void launch_lerp(long n, const float* a, const float* b, float ta, float tb, flo
 void launch_resample(int ndet, int nrows, const float* src, float cth, float sth, float shift, float* out,
                      cudaStream_t st);
 int mirror_error_blocks(int ndet, int nrows);
-// writes the FP64 mismatch to out[0]; part holds nblk partials (scratch)
-void launch_mirror_error(int ndet, int nrows, const float* p0, const float* p180, float cth, float sth, float shift,
-                         double* part, int nblk, double* out, cudaStream_t st);
+// Candidates of the registration's pattern search: rotation (its cosine and sine) and shift.
+constexpr int MIRROR_MAX = 6;
+struct MirrorCandidates {
+    float cth[MIRROR_MAX], sth[MIRROR_MAX], shift[MIRROR_MAX];
+};
+// writes the FP64 mismatches of n candidates to out[0..n-1]; part holds n * nblk
+// partials (scratch), done n counters that are and stay 0
+void launch_mirror_errors(int ndet, int nrows, const float* p0, const float* p180, const MirrorCandidates& cand, int n,
+                          double* part, int nblk, unsigned* done, double* out, cudaStream_t st);
 // writes tm, cmx_0, cmx_180 to out3[0..2]; part holds 3 * nblk partials
 void launch_com(int ndet, int nrows, const float* p0, const float* p180, double* part, int nblk, double* out3,
                 cudaStream_t st);

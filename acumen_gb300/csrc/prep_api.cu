@@ -40,32 +40,30 @@ int minloc_abs(int n, const float* theta, float target)
     return best;
 }
 
-double read_scalar(acu_ctx* c, const double* d, int* rc)
-{
-    double h = 0.0;
-    cudaError_t e = cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    *rc = e == cudaSuccess ? ACU_OK : set_err(c, ACU_ERR_CUDA, "scalar read failed: %s", cudaGetErrorString(e));
-    return h;
-}
+// Objective of the pattern search, as the reference's single-precision
+// `error_diff` (accumulated in FP64, rounded once), for n candidates at once.
+struct MirrorSearch {
+    acu_ctx* c;
+    int ndet, nrows, nblk;
+    const float *p0, *p180;
+    double* part;
 
-// Objective of the pattern search for one candidate, as the reference's
-// single-precision `error_diff` (accumulated in FP64, rounded once).
-int mirror_error(acu_ctx* c, int ndet, int nrows, const float* p0, const float* p180, float th, float shift,
-                 float* out)
-{
-    const int nblk = mirror_error_blocks(ndet, nrows);
-    CK(c, c->w_part.ensure(sizeof(double) * (nblk + 8)));
-    double* part = c->w_part.as<double>();
-    launch_mirror_error(ndet, nrows, p0, p180, std::cos(th), std::sin(th), shift, part, nblk, part + nblk,
-                        c->stream);
-    CKLAUNCH(c);
-    int rc;
-    const double e = read_scalar(c, part + nblk, &rc);
-    if (rc != ACU_OK) return rc;
-    *out = (float)e;
-    return ACU_OK;
-}
+    int evaluate(const float* th, const float* shift, int n, float* err) const
+    {
+        MirrorCandidates cand{};
+        for (int k = 0; k < n; ++k) {
+            cand.cth[k] = std::cos(th[k]);
+            cand.sth[k] = std::sin(th[k]);
+            cand.shift[k] = shift[k];
+        }
+        unsigned* done = reinterpret_cast<unsigned*>(part + MIRROR_MAX * nblk);
+        launch_mirror_errors(ndet, nrows, p0, p180, cand, n, part, nblk, done, c->pinned, c->stream);
+        CKLAUNCH(c);
+        CK(c, cudaStreamSynchronize(c->stream));
+        for (int k = 0; k < n; ++k) err[k] = (float)c->pinned[k];
+        return ACU_OK;
+    }
+};
 
 }  // namespace
 
@@ -151,52 +149,63 @@ int acu_register_dev(acu_ctx* c, int ndet, int nrows, const float* d_p0, const f
 {
     CKRET(check_proj(c, ndet, nrows));
     if (!d_p0 || !d_p180 || !theta_out || !shift_out) return set_err(c, ACU_ERR_INVALID, "null argument");
-    const int add = (ndet % 2 == 0) ? 1 : 0;
     // centre of mass (:231-248)
     const int nblk = mirror_error_blocks(ndet, nrows);
-    CK(c, c->w_part.ensure(sizeof(double) * (3 * nblk + 8)));
+    CK(c, c->w_part.ensure(sizeof(double) * (MIRROR_MAX * nblk + 8)));
+    if (!c->pinned) CK(c, cudaHostAlloc((void**)&c->pinned, sizeof(double) * MIRROR_MAX, cudaHostAllocMapped));
     double* part = c->w_part.as<double>();
-    launch_com(ndet, nrows, d_p0, d_p180, part, nblk, part + 3 * nblk, c->stream);
+    launch_com(ndet, nrows, d_p0, d_p180, part, nblk, c->pinned, c->stream);
     CKLAUNCH(c);
-    double sums[3];
-    CK(c, cudaMemcpyAsync(sums, part + 3 * nblk, sizeof sums, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemsetAsync(part + MIRROR_MAX * nblk, 0, sizeof(unsigned) * MIRROR_MAX, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    (void)add;
-    const float tm = (float)sums[0], cmx0 = (float)sums[1], cmx180 = (float)sums[2];
+    const float tm = (float)c->pinned[0], cmx0 = (float)c->pinned[1], cmx180 = (float)c->pinned[2];
     const float shift_scale = (float)ndet;
     float best_shift = -((cmx0 / tm + cmx180 / tm) / (2.0f * shift_scale));
     float best_theta = 0.0f;
     float dshift = 1e-4f, dtheta = 1e-4f;
     const int n_sp = 6;
     const float n_mag = 1.05f, n_min = 2.0f / (float)n_sp;
+    const MirrorSearch search{c, ndet, nrows, nblk, d_p0, d_p180, part};
     int ne = 1;
     float best_error;
-    CKRET(mirror_error(c, ndet, nrows, d_p0, d_p180, best_theta, best_shift, &best_error));
+    CKRET(search.evaluate(&best_theta, &best_shift, 1, &best_error));
+    // Candidates 1..n_sp around the best, which a better one replaces at once.  All
+    // that are left are evaluated together, and again from the next one on after
+    // each improvement.  Candidate n_sp / 2 is the best itself: its error is known.
+    auto sweep = [&](float& best, float step) -> int {
+        for (int jsp = 1; jsp <= n_sp;) {
+            float th[MIRROR_MAX], sh[MIRROR_MAX], cand[MIRROR_MAX], err[MIRROR_MAX];
+            int n = 0;
+            for (int j = jsp; j <= n_sp; ++j) {
+                if (j == n_sp / 2) continue;
+                th[n] = best_theta;
+                sh[n] = best_shift;
+                cand[n] = best + step * (float)(j - n_sp / 2);
+                (&best == &best_theta ? th : sh)[n] = cand[n];
+                ++n;
+            }
+            CKRET(search.evaluate(th, sh, n, err));
+            bool better = false;
+            for (int k = 0; jsp <= n_sp && !better; ++jsp) {
+                ++ne;
+                if (jsp == n_sp / 2) continue;
+                better = err[k] < best_error;
+                if (better) {
+                    best = cand[k];
+                    best_error = err[k];
+                }
+                ++k;
+            }
+        }
+        return ACU_OK;
+    };
     // multiplicative pattern search (:287-364)
     while (std::fmax(dtheta, dshift) > 1e-8f) {
         float perr = best_error;
-        for (int jsp = 1; jsp <= n_sp; ++jsp) {
-            const float th = best_theta + dtheta * (float)(jsp - n_sp / 2);
-            float e;
-            CKRET(mirror_error(c, ndet, nrows, d_p0, d_p180, th, best_shift, &e));
-            ++ne;
-            if (e < best_error) {
-                best_theta = th;
-                best_error = e;
-            }
-        }
+        CKRET(sweep(best_theta, dtheta));
         dtheta = (best_error < perr) ? n_mag * dtheta : n_min * dtheta;
         perr = best_error;
-        for (int jsp = 1; jsp <= n_sp; ++jsp) {
-            const float sh = best_shift + dshift * (float)(jsp - n_sp / 2);
-            float e;
-            CKRET(mirror_error(c, ndet, nrows, d_p0, d_p180, best_theta, sh, &e));
-            ++ne;
-            if (e < best_error) {
-                best_shift = sh;
-                best_error = e;
-            }
-        }
+        CKRET(sweep(best_shift, dshift));
         dshift = (best_error < perr) ? n_mag * dshift : n_min * dshift;
         if (ne > 200000) return set_err(c, ACU_ERR_TIMEOUT, "registration did not converge in 200000 evaluations");
     }

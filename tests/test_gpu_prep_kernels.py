@@ -59,3 +59,19 @@ def test_median_tiles(pp, oracle, ndet, nrows, nproj, special):
     with np.errstate(invalid="ignore"):
         got = pp.proj_to_sino(cu(proj), 0.003, 0.01).cpu().numpy()
         np.testing.assert_array_equal(got, oracle.proj_to_sino(proj, 0.003, 0.01))
+
+
+@pytest.mark.parametrize("ndet,nrows,shift", [(65, 3, 2), (66, 9, -1), (1025, 4, 5), (300, 120, -3)])
+def test_registration_sizes(pp, oracle, ndet, nrows, shift):
+    """The search ends where the oracle's does.  Its errors differ by the order of
+    FP64 sums, rounded to single precision: steps of 1e-4 times 1.05 and 1/3 end
+    within 1e-4 of each other, as in the registration tests."""
+    rng = np.random.default_rng(ndet)
+    x = np.linspace(0, 1, ndet)[None, :] + 0.02 * np.arange(nrows)[:, None]
+    p0 = (np.exp(-((x - 0.45) / 0.2) ** 2) + 0.3 * np.sin(9 * x) ** 2 + 0.01 * rng.normal(size=x.shape)).astype(np.float32)
+    p180 = np.ascontiguousarray(np.roll(p0, shift, axis=1)[:, ::-1])
+    th_g, sh_g, ne_g = pp.register(cu(p0), cu(p180))
+    th_o, sh_o, ne_o = oracle.register(p0, p180, red_mode=1)
+    assert abs(th_g - th_o) < 1e-4 and abs(sh_g - sh_o) < 1e-4
+    again = pp.register(cu(p0), cu(p180))
+    assert again == (th_g, sh_g, ne_g)
