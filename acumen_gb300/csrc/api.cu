@@ -101,13 +101,25 @@ int ensure_geom(acu_ctx* c)
     ord = lines_angle_order(s32.data(), c->T);
     put(gs.d.lines_order, ord.data(), sizeof(int) * ord.size());
     if constexpr (sizeof(Real) == 4) {
-        gs.h_mma = mma_angles(h.xsc_fp.data(), c->T);
+        int dev = 0;
+        CK(c, cudaGetDevice(&dev));
+        CK(c, cudaDeviceGetAttribute(&gs.d.sms, cudaDevAttrMultiProcessorCount, dev));
+        gs.d.stretches = mma_stretches(c->N, gs.d.sms);
+        gs.h_mma = mma_angles(h.xsc_fp.data(), c->T, c->N, gs.d.stretches);
         put(gs.d.mma, gs.h_mma.data(), sizeof(MmaAngle) * gs.h_mma.size());
+        std::vector<MmaAngle> in_order(gs.h_mma.size());
+        for (const MmaAngle& a : gs.h_mma) in_order[a.at] = a;
+        put(gs.d.angles, in_order.data(), sizeof(MmaAngle) * in_order.size());
         gs.d.h_mma = gs.h_mma.data();
         gs.h_groups = mma_groups(gs.h_mma);
         put(gs.d.groups, gs.h_groups.data(), sizeof(int) * gs.h_groups.size());
         gs.d.h_groups = gs.h_groups.data();
         gs.d.n_groups = (int)gs.h_groups.size() - 1;
+        while (gs.d.n_groups_x < gs.d.n_groups) {
+            const MmaAngle& a = gs.h_mma[gs.h_groups[gs.d.n_groups_x]];
+            if (std::fabs(a.c) < std::fabs(a.s)) break;
+            ++gs.d.n_groups_x;
+        }
         const std::vector<FxAngle> fx = fx_angles(h.xsc_fp.data(), c->T);
         put(gs.d.fx_fp, fx.data(), sizeof(FxAngle) * fx.size());
         std::vector<int> tiles;
@@ -240,7 +252,7 @@ int ensure_projector_buffers(acu_ctx* c, int G)
         const MmaPlan p = mma_plan(c->g32.d, G);
         CK(c, c->mmaT.ensure(p.tile_bytes));
         CK(c, c->mmaP.ensure(p.part_bytes));
-        CK(c, c->mmaF.ensure(2 * sizeof(int)));
+        CK(c, c->mmaF.ensure(sizeof(int) * mma_flag_words(G)));
     } else if (v == 6) {
         CK(c, c->lineL.ensure(sizeof(float) * lines_image_floats(c->N, G)));
         CK(c, c->lineA.ensure(sizeof(float) * lines_sums_floats(c->N, c->T, G)));

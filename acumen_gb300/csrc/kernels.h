@@ -21,13 +21,15 @@ struct FxAngle {
 };
 constexpr int FX_MAX_SIDE = 4097;
 
-// One angle of the tensor-core projector (kernels_radon_mma.cu).
+// One angle of the tensor-core projector (kernels_radon_mma.cu), for which angles whose
+// rays run along x (|c| >= |s|) come before the others, and of the transpose.
 struct MmaAngle {
     float4 x;         // split sine and cosine, as xsc_fp
     float c, s, t;    // cosine, sine, slope of a ray's closest approach
     float reach;      // |c| + |s| and a margin: how far a pixel's taps reach across the rays
-    int nr, roff;     // rows (rays) of the angle's window in a tile, and the rows of the angles before it
-    int pad[2];
+    int nr;           // rows (rays) of the angle's window in a tile
+    int span, roff;   // rows of its window in a stretch of tiles, and those of the angles before it
+    int at;           // the angle's number
 };
 
 // Geometry of one reconstruction grid on the device, for one precision.
@@ -55,11 +57,14 @@ struct DevGeom {
     const float4* xsc_fp = nullptr;
     int exact = 0;
     const FxAngle* fx_fp = nullptr;     // projector's angles in fixed point (single precision)
-    const MmaAngle* mma = nullptr;      // tensor-core projector's angles (single precision), and their host copy
+    const MmaAngle* angles = nullptr;   // single precision: the angles in order
+    const MmaAngle* mma = nullptr;      // those along x first, and their host copy
     const MmaAngle* h_mma = nullptr;
     const int* groups = nullptr;        // first angles of its groups, n_groups + 1 of them, and their host copy
     const int* h_groups = nullptr;
-    int n_groups = 0;
+    int n_groups = 0, n_groups_x = 0;   // those along x come first
+    int stretches = 1;                  // of tiles, per line of them
+    int sms = 152;
     const int* tiles_in = nullptr;      // 16 x 16 pixel tiles that meet the mask (n_tiles_in), then the others
     int n_tiles_in = 0;
     const float4* h_xsc_bp = nullptr;   // host copy of xsc_bp (for the parameter table)
@@ -102,13 +107,15 @@ struct MmaPlan {
     int nt = 0;        // tiles per side
     int nblk = 0;      // 64-slice blocks of the batch
     int nb = 0;        // of them at once
-    int ng = 0;        // groups of angles at once
+    int ng = 0;        // groups of angles at once, at most
     size_t tile_bytes = 0, part_bytes = 0;
 };
 constexpr size_t MMA_PART_CAP = (size_t)4 << 30;   // bytes of partial sums at once
-std::vector<MmaAngle> mma_angles(const float* xsc, int T);
+int mma_stretches(int N, int sms);
+std::vector<MmaAngle> mma_angles(const float* xsc, int T, int N, int stretches);
 bool mma_fits(int N);
 std::vector<int> mma_groups(const std::vector<MmaAngle>& ang);
+size_t mma_flag_words(int G);
 MmaPlan mma_plan(const DevGeom<float>& g, int G);
 void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned char* tiles, float* P, int* flags,
                       const MmaPlan& p, float* sino, cudaStream_t st);

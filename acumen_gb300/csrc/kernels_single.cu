@@ -275,9 +275,9 @@ void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, floa
 template <int V>
 void launch_adjoint_fx(const DevGeom<float>& g, int G, const float* sino, const float* off, float* img, cudaStream_t st)
 {
-    k_adjoint_fx<V><<<dim3((g.N + 31) / 32, (g.N + 7) / 8, G), dim3(32, 8), 0, st>>>(sino, g.mma, off, img, g.N, g.T,
+    k_adjoint_fx<V><<<dim3((g.N + 31) / 32, (g.N + 7) / 8, G), dim3(32, 8), 0, st>>>(sino, g.angles, off, img, g.N, g.T,
                                                                                      g.mid);
-    k_adjoint_rim<V><<<dim3((6 * g.N + 7) / 8, G), 256, 0, st>>>(sino, g.mma, off, img, g.N, g.T, g.mid);
+    k_adjoint_rim<V><<<dim3((6 * g.N + 7) / 8, G), 256, 0, st>>>(sino, g.angles, off, img, g.N, g.T, g.mid);
 }
 template void launch_adjoint_fx<1>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);
 template void launch_adjoint_fx<4>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);

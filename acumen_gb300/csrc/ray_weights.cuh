@@ -40,9 +40,7 @@ __device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float e
     const float d0 = i0 - wf;
     const float2 along = make_float2(a.c, a.s), back = make_float2(-a.c, -a.s), across = make_float2(-a.s, a.c);
     const float2 one = make_float2(1.f, 1.f);
-    if constexpr (WHERE == RIM) wv[0] = wv[1] = wv[2] = 0.f;
-    // rolled at the rim, which few pixels meet: its code and registers would cost all the others
-#pragma unroll (WHERE == RIM ? 1 : 3)
+#pragma unroll
     for (int r = 0; r < 3; ++r) {
         const float d = d0 + (float)r;
         const float ctr = __fmaf_rn(a.t, d, uf);
@@ -50,9 +48,9 @@ __device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float e
         const float e = kf - uf;
         const float2 p0 = fma2(along, make_float2(e, e), mul2(across, make_float2(d, d)));
         float w = 0.f;
-#pragma unroll (WHERE == RIM ? 1 : 3)
+#pragma unroll
         for (int q = -1; q <= 1; ++q) {
-            const float2 p = WHERE == RIM ? fma2(along, make_float2((float)q, (float)q), p0) : q < 0 ? fma2(back, one, p0) : q > 0 ? fma2(along, one, p0) : p0;
+            const float2 p = q < 0 ? fma2(back, one, p0) : q > 0 ? fma2(along, one, p0) : p0;
             const float hx = __saturatef(1.f - fabsf(p.x)), hy = __saturatef(1.f - fabsf(p.y));
             if constexpr (WHERE == INNER) {
                 w = fmaf(hx, hy, w);
@@ -71,13 +69,7 @@ __device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float e
                 w = ok ? fmaf(hx, hy, w) : w;
             }
         }
-        if constexpr (WHERE == RIM) {
-            wv[0] = r == 0 ? w : wv[0];
-            wv[1] = r == 1 ? w : wv[1];
-            wv[2] = r == 2 ? w : wv[2];
-        } else {
-            wv[r] = w;
-        }
+        wv[r] = w;
     }
 }
 

@@ -88,6 +88,29 @@ __device__ __forceinline__ void tmem_ld_wait(float2 (&v)[4])
                    "+f"(v[3].y)::"memory");
 }
 
+// the same, 16 columns at a time
+__device__ __forceinline__ void tmem_ld16(uint32_t t, float2 (&v)[8])
+{
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(t)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+__device__ __forceinline__ void tmem_ld_wait(float2 (&v)[8], float2 (&x)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[3].x),
+                   "+f"(v[3].y), "+f"(v[4].x), "+f"(v[4].y), "+f"(v[5].x), "+f"(v[5].y), "+f"(v[6].x), "+f"(v[6].y),
+                   "+f"(v[7].x), "+f"(v[7].y), "+f"(x[0].x), "+f"(x[0].y), "+f"(x[1].x), "+f"(x[1].y), "+f"(x[2].x),
+                   "+f"(x[2].y), "+f"(x[3].x), "+f"(x[3].y), "+f"(x[4].x), "+f"(x[4].y), "+f"(x[5].x), "+f"(x[5].y),
+                   "+f"(x[6].x), "+f"(x[6].y), "+f"(x[7].x), "+f"(x[7].y)::"memory");
+}
+
 // registers a thread of this warpgroup may use from here on
 template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -163,6 +186,14 @@ __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t 
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// the same, added to what is there (FP32, rounded to nearest; subnormals count as zero)
+__device__ __forceinline__ void bulk_add(void* dst, const void* src, uint32_t bytes)
+{
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+                 "r"(smem_addr(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 // box of a 3-d tensor map at (c0, c1, c2); c0 times the element size is a multiple of 16 bytes
 __device__ __forceinline__ void tensor_load_3d(void* dst, const void* map, int c0, int c1, int c2, uint64_t* bar)
 {
@@ -180,7 +211,12 @@ __device__ __forceinline__ void bulk_store_wait_read()
 {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
 }
-__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// all but the last PENDING groups are done
+template <int PENDING = 0>
+__device__ __forceinline__ void bulk_store_wait()
+{
+    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(PENDING) : "memory");
+}
 // generic-proxy shared-memory writes become visible to MMAs and bulk copies
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

@@ -63,27 +63,46 @@ def tensor_projector(option, positions, S, N):
     return option == 7 and positions == 1 and (S + 3) // 4 >= 7 and 200 <= N <= 4096
 
 
-def tensor_radon_launches(N, theta, S):
+def tensor_radon_launches(N, theta, S, sms=152):
     """Kernels of one projection on the tensor cores (csrc/kernels_radon_mma.cu
     mma_plan): per pass over slice blocks one layout kernel, per chunk of angle
     groups a product and a reduction, and the flagged fallback."""
     import numpy as np
-    c = np.pi * (np.asarray(theta, np.float64) - 90.0) / 180.0
-    nr = np.minimum(25, np.floor(17.0 * (np.abs(np.cos(c)) + np.abs(np.sin(c))) + 0.002).astype(int) + 1)
-    groups, t = [], 0
-    while t < len(nr):
-        n = min(5, len(nr) - t)
-        n = 4 if n == 5 and nr[t + 4] > 24 else n
-        groups.append(int(nr[t:t + n].sum()))
-        t += n
-    row, cap, nblk = ((N + 15) // 16) ** 2 * 256, 4 << 30, (S + 63) // 64
-    nb, ng, total = min(nblk, 2), len(groups), row * sum(groups)
-    if total * nb <= cap:
-        nb = min(nblk, cap // total)
-        nb = nb & ~1 if nb > 2 else nb
-    else:
-        ng = max(1, cap // (row * 125 * nb))
-    return 1 + -(-nblk // nb) * (1 + 2 * -(-len(groups) // ng))
+    nt, nblk = (N + 15) // 16, (S + 63) // 64
+    cost = [-(-nt * q // sms) * -(-nt // q) * (1 + 0.5 * ((6.0 * (-(-nt // q) - 1) + 22) / -(-nt // q)) / 22)
+            for q in range(1, nt + 1)]
+    stretches = 1 + int(np.argmin(cost))
+    a = np.pi * (np.asarray(theta, np.float64) - 90.0) / 180.0
+    c, s = np.abs(np.cos(a).astype(np.float32)), np.abs(np.sin(a).astype(np.float32))
+    nr = np.minimum(25, np.floor(np.float32(17) * (c + s) + np.float32(0.002)).astype(int) + 1)
+    length = -(-nt // stretches)
+    span = np.floor(16 * (length - 1) * np.minimum(c, s) + 0.01).astype(int) + 1 + nr
+    sides = []   # rows of the groups: angles along x, then the others
+    for side in (c >= s, c < s):
+        n, rows, groups, t = nr[side], span[side], [], 0
+        while t < len(n):
+            k = min(5, len(n) - t)
+            k = 4 if k == 5 and n[t + 4] > 24 else k
+            groups.append(int(rows[t:t + k].sum()))
+            t += k
+        sides.append(groups)
+
+    def chunks(ng):
+        out = []
+        for g in sides:
+            k = -(-len(g) // ng)
+            out += [sum(g[i * len(g) // k:(i + 1) * len(g) // k]) for i in range(k)]
+        return out
+
+    units = nt * stretches
+    nb = min(nblk, 2)
+    if nb == 2 and units < 4 * sms:
+        nb = min(nblk, 2 * -(-4 * sms // units))
+    nb = nb & ~1 if nb > 2 else nb
+    ng = min(sum(map(len, sides)), max(1, (144 << 20) // (256 * 110 * min(sms, units) * min(nb, 2))))
+    while 256 * max(chunks(ng)) * units * nb > 4 << 30 and not (nb <= 2 and ng == 1):
+        nb, ng = (nb - 2, ng) if nb > 2 else (nb, ng - 1)
+    return 1 + -(-nblk // nb) * (1 + 2 * len(chunks(ng)))
 
 
 def iradon_launches(positions, S, N):
