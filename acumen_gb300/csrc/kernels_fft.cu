@@ -5,9 +5,9 @@
 // complex signal z = a + i b, zero-pads it to L >= 2N-2 (a power of two),
 // and computes y = IFFT(H . FFT(z)) with H the real spectrum of the wrapped,
 // symmetric tap sequence (computed in double on the host, 1/L folded in).
-// Because H is real, Re(y) and Im(y) are the two filtered columns.  At
-// L = 4096 in single precision (grids 1449 to 2049) the transforms are three
-// radix-16 passes held in registers (k_filter_fft4096); otherwise radix-4
+// Because H is real, Re(y) and Im(y) are the two filtered columns.  In single
+// precision at L = 512 to 4096 (grids 130 to 2049) the transforms are passes of
+// radix 16, L / 256 and 16 held in registers (k_filter_fft_r16); otherwise radix-4
 // Stockham stages (a radix-2 stage last when log2 L is odd) in shared memory.
 // All twiddles come from double-precision-built tables.
 #include "common.cuh"
@@ -166,15 +166,21 @@ __global__ void __launch_bounds__(512) k_filter_fft(const Real* __restrict__ sin
     }
 }
 
-// ---- L = 4096 in single precision: three radix-16 passes in registers ------
-// Each of 256 threads holds 16 values of a pass: it reads them from the shared
-// buffer (element j + 256 m), multiplies by the pass's twiddles, forms a
-// 16-point DFT as 4 x 4 (4-point DFTs, the internal twiddles w16^(m1 q2), 4-point
-// DFTs) and writes the outputs to their Stockham places.  Against the radix-4
-// stages this halves the shared-memory traffic and reads the twiddles from
-// tables laid out per pass, which the filter's L1 data pipe (93 % busy with
-// the radix-4 stages) needs.  One buffer per transform, padded by one slot per
-// 16 so that the strided writes of the first pass spread over the banks.
+// ---- L = 256 M, M = 2, 4, 8, 16, in single precision: passes of radix 16, M, 16 ------
+// Each of 16 M threads holds 16 values of a pass: those j + 16 M m of the first
+// and the last, read from the shared buffer, multiplied by the pass's twiddles,
+// transformed (16 points as 4 x 4: 4-point DFTs, the internal twiddles w16^(m1 q2),
+// 4-point DFTs) and written to their Stockham places.  The first pass reads the
+// sinogram itself; the last pass's values are those that the inverse
+// transform's first pass needs, so the spectrum never leaves the registers; the
+// last pass writes the result.  That leaves four exchanges through shared memory
+// per filtered pair, of eight with separate transforms (its data pipe was 93 % busy
+// with radix-4 stages).  One buffer per transform, padded by one slot per 16 so that the
+// strided writes of the first pass spread over the banks.
+// Measured (us, before / now; before: radix-4 stages, three separate radix-16
+// passes at L = 4096): 257 x 180 angles, 64 slices 63 / 15; 513 x 360, 64 slices 213 / 49;
+// 725 x 720 22.5 / 8.4; 1025 x 600, 64 slices 788 / 183; 1449 x 900 18.0 / 13.0;
+// 2049 x 300, 64 slices 294 / 186.  Fewer registers for more warps (128 now) gained nothing.
 __device__ __forceinline__ int pad16(int i) { return i + (i >> 4); }
 
 // (a0..a3) -> their 4-point DFT, e^(-2 pi i / 4) = -i
@@ -188,25 +194,39 @@ __device__ __forceinline__ void dft4(float2& a0, float2& a1, float2& a2, float2&
     a3 = csub(t1, t3);
 }
 
+// a times the constant (rh + rl) + i (ih + il): constants in two parts, as their
+// rounding would otherwise be in every value (a filtered row's error 1.5e-7
+// instead of 1.8e-7 at L = 4096, 1.7e-7 with radix-4 stages)
+__device__ __forceinline__ float2 cmul_const(float2 a, float rh, float rl, float ih, float il)
+{
+    return make_float2(fmaf(a.x, rh, -fmaf(a.y, ih, fmaf(a.y, il, -(a.x * rl)))),
+                       fmaf(a.x, ih, fmaf(a.y, rh, fmaf(a.y, rl, a.x * il))));
+}
+
+// cos(pi/8), sin(pi/8), sqrt(1/2)
+constexpr double C8 = 0.92387953251128675613, S8 = 0.38268343236508977173, R2 = 0.70710678118654752440;
+
+__device__ __forceinline__ float2 mul_w(float2 a, double re, double im)   // re, im: compile-time constants
+{
+    return cmul_const(a, (float)re, (float)(re - (double)(float)re), (float)im, (float)(im - (double)(float)im));
+}
+
 // x -> its 16-point DFT y, y[q2 + 4 q1] = sum_m x[m] w16^(m (q2 + 4 q1)),
 // m = m1 + 4 m2; the result is returned in x in natural order
 __device__ __forceinline__ void dft16(float2 (&x)[16])
 {
-    constexpr float C8 = 0.92387953251128675613f;   // cos(pi/8)
-    constexpr float S8 = 0.38268343236508977173f;   // sin(pi/8)
-    constexpr float R2 = 0.70710678118654752440f;   // sqrt(1/2)
 #pragma unroll
     for (int m1 = 0; m1 < 4; ++m1) dft4(x[m1], x[m1 + 4], x[m1 + 8], x[m1 + 12]);   // over m2 -> q2 = 0..3
     // x[m1 + 4 q2] *= w16^(m1 q2)
-    x[5] = cmul(x[5], make_float2(C8, -S8));     // 1
-    x[9] = cmul(x[9], make_float2(R2, -R2));     // 2
-    x[13] = cmul(x[13], make_float2(S8, -C8));   // 3
-    x[6] = cmul(x[6], make_float2(R2, -R2));     // 2
-    x[10] = make_float2(x[10].y, -x[10].x);      // 4: -i
-    x[14] = cmul(x[14], make_float2(-R2, -R2));  // 6
-    x[7] = cmul(x[7], make_float2(S8, -C8));     // 3
-    x[11] = cmul(x[11], make_float2(-R2, -R2));  // 6
-    x[15] = cmul(x[15], make_float2(-C8, S8));   // 9
+    x[5] = mul_w(x[5], C8, -S8);     // 1
+    x[9] = mul_w(x[9], R2, -R2);     // 2
+    x[13] = mul_w(x[13], S8, -C8);   // 3
+    x[6] = mul_w(x[6], R2, -R2);     // 2
+    x[10] = make_float2(x[10].y, -x[10].x);   // 4: -i
+    x[14] = mul_w(x[14], -R2, -R2);  // 6
+    x[7] = mul_w(x[7], S8, -C8);     // 3
+    x[11] = mul_w(x[11], -R2, -R2);  // 6
+    x[15] = mul_w(x[15], -C8, S8);   // 9
 #pragma unroll
     for (int q2 = 0; q2 < 4; ++q2) dft4(x[4 * q2], x[4 * q2 + 1], x[4 * q2 + 2], x[4 * q2 + 3]);   // over m1 -> q1
     // now x[4 q2 + q1] holds y[q2 + 4 q1]: transpose the 4 x 4 index
@@ -219,83 +239,127 @@ __device__ __forceinline__ void dft16(float2 (&x)[16])
     for (int r = 0; r < 16; ++r) x[r] = y[r];
 }
 
-// Forward DFT of 4096 points held in the padded buffer b (blockDim.x = 256);
-// tw1: [15][16] = w^(m k 16), tw2: [15][256] = w^(m k), w = e^(-2 pi i / 4096)
-__device__ void fft4096_r16(float2* b, const float2* __restrict__ tw1, const float2* __restrict__ tw2)
+// x[0..R-1] -> their R-point DFT in natural order
+template <int R>
+__device__ __forceinline__ void dft(float2* x)
 {
-    const int j = threadIdx.x;
-#pragma unroll 1
-    for (int p = 0; p < 3; ++p) {
-        const int lgNs = 4 * p, k = j & ((1 << lgNs) - 1);
-        float2 x[16];
+    if constexpr (R == 2) {
+        const float2 a = cadd(x[0], x[1]), b = csub(x[0], x[1]);
+        x[0] = a;
+        x[1] = b;
+    } else if constexpr (R == 4) {
+        dft4(x[0], x[1], x[2], x[3]);
+    } else if constexpr (R == 8) {
+        float2 e[4] = {x[0], x[2], x[4], x[6]}, o[4] = {x[1], x[3], x[5], x[7]};
+        dft4(e[0], e[1], e[2], e[3]);
+        dft4(o[0], o[1], o[2], o[3]);
+        o[1] = mul_w(o[1], R2, -R2);
+        o[2] = make_float2(o[2].y, -o[2].x);
+        o[3] = mul_w(o[3], -R2, -R2);
 #pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] = b[pad16(j + 256 * m)];
-        __syncthreads();
-        if (p == 1) {
-#pragma unroll
-            for (int m = 1; m < 16; ++m) x[m] = cmul(x[m], __ldg(tw1 + (m - 1) * 16 + k));
-        } else if (p == 2) {
-#pragma unroll
-            for (int m = 1; m < 16; ++m) x[m] = cmul(x[m], __ldg(tw2 + (m - 1) * 256 + k));
+        for (int q = 0; q < 4; ++q) {
+            x[q] = cadd(e[q], o[q]);
+            x[q + 4] = csub(e[q], o[q]);
         }
-        dft16(x);
-        const int idxD = ((j >> lgNs) << (lgNs + 4)) + k;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) b[pad16(idxD + (r << lgNs))] = x[r];
-        __syncthreads();
+    } else {
+        dft16(*reinterpret_cast<float2(*)[16]>(x));
     }
 }
 
-// k_filter_fft for L = 4096 in single precision (256 threads): the same
-// packing, spectrum product and output as k_filter_fft, with fft4096_r16.
-__global__ void __launch_bounds__(256) k_filter_fft4096(const float* __restrict__ sino, float* __restrict__ out,
-                                                        const float* __restrict__ H,
-                                                        const float2* __restrict__ tw16, int N, int T, int V,
-                                                        bool pairs)
+// The passes after the first of a DFT of 256 M points: the first pass's outputs
+// x (thread j: places 16 j + r) -> the thread's values j + 16 M r.
+// tw1: [M - 1][16] = w^(m k 16), tw2: [15][16 M] = w^(m k), w = e^(-2 pi i / L)
+template <int M>
+__device__ __forceinline__ void fft_passes(float2 (&x)[16], float2* b, int j, const float2* __restrict__ tw1,
+                                           const float2* __restrict__ tw2)
 {
-    constexpr int L = 4096;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* b = reinterpret_cast<float2*>(smem_raw);
-    const float2* tw1 = tw16;
-    const float2* tw2 = tw16 + 15 * 16;
-    const int g = blockIdx.y;
+    constexpr int TH = 16 * M;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) b[pad16(16 * j + r)] = x[r];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16 / M; ++q)
+#pragma unroll
+        for (int m = 0; m < M; ++m) x[q * M + m] = b[pad16(j + q * TH + 256 * m)];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16 / M; ++q) {
+        const int jj = j + q * TH, k = jj & 15;
+#pragma unroll
+        for (int m = 1; m < M; ++m) x[q * M + m] = cmul(x[q * M + m], __ldg(tw1 + (m - 1) * 16 + k));
+        dft<M>(x + q * M);
+#pragma unroll
+        for (int r = 0; r < M; ++r) b[pad16((jj >> 4) * TH + k + 16 * r)] = x[q * M + r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; ++m) x[m] = b[pad16(j + TH * m)];
+    __syncthreads();
+#pragma unroll
+    for (int m = 1; m < 16; ++m) x[m] = cmul(x[m], __ldg(tw2 + (m - 1) * TH + j));
+    dft16(x);
+}
+
+// k_filter_fft for these lengths: RB column pairs per block of 16 M RB threads.
+template <int M, int RB>
+__global__ void __launch_bounds__(16 * M * RB) k_filter_fft_r16(const float* __restrict__ sino, float* __restrict__ out,
+                                                                const float* __restrict__ H,
+                                                                const float2* __restrict__ tw16, int N, int T, int V,
+                                                                bool pairs)
+{
+    constexpr int L = 256 * M, TH = 16 * M;
+    __shared__ float2 s_b[RB][L + L / 16];
+    const int j = threadIdx.x % TH, col = blockIdx.x * RB + threadIdx.x / TH, g = blockIdx.y;
+    float2* const b = s_b[threadIdx.x / TH];
+    const float2* const tw2 = tw16 + (M - 1) * 16;
     size_t offa, offb;
-    int stride;
-    bool has_b = true;
+    bool live, has_b = true;
     if (V == 4) {
-        const int t = blockIdx.x >> 1, h = blockIdx.x & 1;
-        offa = (((size_t)g * T + t) * N) * 4 + 2 * h;
+        offa = (((size_t)g * T + (col >> 1)) * N) * 4 + 2 * (col & 1);
         offb = offa + 1;
-        stride = 4;
+        live = col < 2 * T;
     } else {
-        const int t0 = 2 * blockIdx.x;
+        const int t0 = 2 * col;
         offa = ((size_t)g * T + t0) * N;
         offb = offa + N;
-        stride = 1;
-        has_b = (t0 + 1) < T;
+        live = t0 < T;
+        has_b = t0 + 1 < T;
     }
-    for (int n = threadIdx.x; n < L; n += blockDim.x) {
-        float2 z;
-        if (V == 4) {
-            z = n < N ? __ldg(reinterpret_cast<const float2*>(sino + offa + (size_t)n * 4)) : make_float2(0.f, 0.f);
-        } else {
-            z.x = n < N ? sino[offa + (size_t)n * stride] : 0.f;
-            z.y = (n < N && has_b) ? sino[offb + (size_t)n * stride] : 0.f;
+    float2 x[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+        const int n = j + TH * m;
+        x[m] = make_float2(0.f, 0.f);
+        if (live && n < N) {
+            if (V == 4) {
+                x[m] = __ldg(reinterpret_cast<const float2*>(sino + offa + (size_t)n * 4));
+            } else {
+                x[m].x = sino[offa + n];
+                if (has_b) x[m].y = sino[offb + n];
+            }
         }
-        b[pad16(n)] = z;
     }
-    __syncthreads();
-    fft4096_r16(b, tw1, tw2);
+    dft16(x);
+    fft_passes<M>(x, b, j, tw16, tw2);
     // W = H/L * conj(Z); y = conj(FFT(W))
-    for (int m = threadIdx.x; m < L; m += blockDim.x) {
-        const float2 z = b[pad16(m)];
-        const float h = H[m];
-        b[pad16(m)] = make_float2(h * z.x, -h * z.y);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const float h = __ldg(H + j + TH * r);
+        x[r] = make_float2(h * x[r].x, -h * x[r].y);
     }
-    __syncthreads();
-    fft4096_r16(b, tw1, tw2);
-    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-        const float2 v = b[pad16(n)];
+    dft16(x);
+    fft_passes<M>(x, b, j, tw16, tw2);
+    if (pairs) {   // (bin, next bin), zeros in the first and the last
+#pragma unroll
+        for (int r = 0; r < 16; ++r) b[pad16(j + TH * r)] = x[r];
+        __syncthreads();
+    }
+    if (!live) return;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const int n = j + TH * r;
+        if (n >= N) continue;
+        const float2 v = x[r];
         if (pairs) {
             const bool in = n > 0 && n < N - 1;
             const float2 w = b[pad16(in ? n + 1 : n)];
@@ -305,10 +369,19 @@ __global__ void __launch_bounds__(256) k_filter_fft4096(const float* __restrict_
         } else if (V == 4) {
             *reinterpret_cast<float2*>(out + offa + (size_t)n * 4) = make_float2(v.x, -v.y);
         } else {
-            out[offa + (size_t)n * stride] = v.x;
-            if (has_b) out[offb + (size_t)n * stride] = -v.y;
+            out[offa + n] = v.x;
+            if (has_b) out[offb + n] = -v.y;
         }
     }
+}
+
+template <int M, int RB>
+void filter_fft_r16(const DevGeom<float>& g, int G, int V, const float* sino, float* out, const float* H, bool pairs,
+                    cudaStream_t st)
+{
+    const int cols = V == 4 ? 2 * g.T : (g.T + 1) / 2;
+    k_filter_fft_r16<M, RB><<<dim3((cols + RB - 1) / RB, G), 16 * M * RB, 0, st>>>(sino, out, H, g.fft_tw16, g.N, g.T, V,
+                                                                                   pairs);
 }
 
 template <typename Real, int V>
@@ -324,11 +397,16 @@ void launch_filter_fft(const DevGeom<Real>& g, int G, const Real* sino, Real* ou
     // exact positions filter with the spectrum of the FP64 taps
     const Real* H = (g.exact && g.fft_h_x) ? g.fft_h_x : g.fft_h;
     if constexpr (sizeof(Real) == 4) {
-        if (g.fft_L == 4096 && g.fft_tw16) {   // 3.6x the radix-4 stages at this length
-            const size_t sm16 = (size_t)(4096 + 256) * sizeof(float2);
-            max_dynamic_smem<k_filter_fft4096>();
-            k_filter_fft4096<<<grd, 256, sm16, st>>>(sino, out, H, g.fft_tw16, g.N, g.T, V, pairs);
-            return;
+        // column pairs per block: the two of a 4-slice lane together, and 128 threads or more
+        if (g.fft_tw16) {
+            if (g.fft_L == 4096)
+                return filter_fft_r16<16, 1>(g, G, V, sino, out, H, pairs, st);
+            if (g.fft_L == 2048)
+                return filter_fft_r16<8, 2>(g, G, V, sino, out, H, pairs, st);
+            if (g.fft_L == 1024)
+                return filter_fft_r16<4, 2>(g, G, V, sino, out, H, pairs, st);
+            if (g.fft_L == 512)
+                return filter_fft_r16<2, 4>(g, G, V, sino, out, H, pairs, st);
         }
     }
     k_filter_fft<Real><<<grd, 512, sm, st>>>(sino, out, H, tw, g.N, g.T, g.fft_L, V, pairs);

@@ -154,16 +154,15 @@ void make_tables(int N, int T, const float* theta, int wpu, HostTables<Real>& ou
         out.fft_tw[2 * k + 1] = std::sin(a);
     }
     out.fft_tw16.clear();
-    if (L == 4096) {
+    if (L >= 512 && L <= 4096) {
         auto put = [&](long e) {
-            const double a = -2.0 * pid * (double)(e % L) / (double)L;
-            out.fft_tw16.push_back(std::cos(a));
-            out.fft_tw16.push_back(std::sin(a));
+            out.fft_tw16.push_back(out.fft_tw[2 * (e % L)]);
+            out.fft_tw16.push_back(out.fft_tw[2 * (e % L) + 1]);
         };
-        for (int m = 1; m < 16; ++m)
+        for (int m = 1; m < L / 256; ++m)
             for (int k = 0; k < 16; ++k) put((long)m * k * 16);
         for (int m = 1; m < 16; ++m)
-            for (int k = 0; k < 256; ++k) put((long)m * k);
+            for (int k = 0; k < L / 16; ++k) put((long)m * k);
     }
 }
 
