@@ -179,7 +179,7 @@ void lanes_filter(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* in, Rea
 constexpr int BP_MMA_MIN_GROUPS = 10, BP_MMA_MIN_SIDE = 200;
 bool bp_mma(const acu_ctx* c, int G)
 {
-    return c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma && G >= BP_MMA_MIN_GROUPS &&
+    return c->bp_room && c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma && G >= BP_MMA_MIN_GROUPS &&
            c->N >= BP_MMA_MIN_SIDE;
 }
 
@@ -187,7 +187,13 @@ bool bp_mma(const acu_ctx* c, int G)
 int ensure_backproject_buffers(acu_ctx* c, int G)
 {
     if (!bp_mma(c, G)) return ACU_OK;
-    CK(c, c->bpQ.ensure(bp_mma_bins_bytes(c->N, c->T, G)));
+    const cudaError_t e = c->bpQ.ensure(bp_mma_bins_bytes(c->N, c->T, G));
+    if (e == cudaErrorMemoryAllocation) {   // the gathers need no buffer
+        cudaGetLastError();
+        c->bp_room = false;
+        return ACU_OK;
+    }
+    CK(c, e);
     CK(c, c->bpS.ensure(sizeof(unsigned) * bp_mma_scalars(G)));
     return ACU_OK;
 }
@@ -235,7 +241,7 @@ int projector_variant(const acu_ctx* c, int G)
     // the tensor-core projector works on blocks of 64 slices, whatever part of one is filled.  Measured (ms, it / the
     // better gather variant): 1025^2 x 600, 16 slices 9.6 / 6.6, 24 slices 9.6 / 10.0, 64 slices 9.6 / 23.4; 257^2 x
     // 180, 20 slices 0.29 / 0.26, 32 slices 0.30 / 0.31; at 129^2 it gains nothing at any batch that fits a block
-    if (c->opt_positions == 1 && G >= MMA_MIN_GROUPS && c->N >= MMA_MIN_SIDE && mma_fits(c->N)) return PROJ_MMA;
+    if (c->mma_cap > 0 && c->opt_positions == 1 && G >= MMA_MIN_GROUPS && c->N >= MMA_MIN_SIDE && mma_fits(c->N)) return PROJ_MMA;
     return 8 * ((G + 7) / 8) <= G + G / 8 ? 6 : 5;
 }
 
@@ -249,9 +255,16 @@ int ensure_projector_buffers(acu_ctx* c, int G)
         CK(c, c->pairP.ensure(sizeof(float) * 2 * nimg));
         CK(c, c->pairPT.ensure(sizeof(float) * 2 * nimg));
     } else if (v == PROJ_MMA) {
-        const MmaPlan p = mma_plan(c->g32.d, G);
-        CK(c, c->mmaT.ensure(p.tile_bytes));
-        CK(c, c->mmaP.ensure(p.part_bytes));
+        const MmaPlan p = mma_plan(c->g32.d, G, c->mma_cap);
+        cudaError_t e = c->mmaT.ensure(p.tile_bytes);
+        if (e == cudaSuccess) e = c->mmaP.ensure(p.part_bytes);
+        if (e == cudaErrorMemoryAllocation) {   // smaller chunks, then the gathers
+            cudaGetLastError();
+            c->mmaT.release();
+            c->mma_cap = c->mma_cap > ((size_t)1 << 30) ? c->mma_cap / 2 : 0;
+            return ensure_projector_buffers(c, G);
+        }
+        CK(c, e);
         CK(c, c->mmaF.ensure(sizeof(int) * mma_flag_words(G)));
     } else if (v == 6) {
         CK(c, c->lineL.ensure(sizeof(float) * lines_image_floats(c->N, G)));
@@ -269,7 +282,7 @@ void radon_quads(acu_ctx* c, const DevGeom<float>& g, int G, const float* img, f
     const int v = projector_variant(c, G);
     if (v == PROJ_MMA)
         launch_radon_mma(g, G, img, c->mmaT.as<unsigned char>(), c->mmaP.as<float>(), c->mmaF.as<int>(),
-                         mma_plan(g, G), sino, c->stream);
+                         mma_plan(g, G, c->mma_cap), sino, c->stream);
     else if (v == 6)
         launch_radon_lines(g, G, img, c->lineL.as<float>(), c->lineA.as<float>(), sino, c->stream);
     else if (v >= 1)
@@ -596,8 +609,8 @@ int tv_iterate_v(acu_ctx* c, int nouter)
                  c->opt_residual, c->g32.d.bp_tma * 100 + c->g32.d.bp_groups * 10 + c->g32.d.bp_param, s.uk.p, s.part.p, c->pairP.p,
                  c->pairPT.p, c->lineL.p, c->lineA.p, c->mmaT.p, c->mmaP.p, c->mmaF.p, c->bpQ.p,
                  c->bpS.p);
-        char key2[600];
-        snprintf(key2, sizeof key2, "%s/%d", key, c->opt_refresh);
+        char key2[640];
+        snprintf(key2, sizeof key2, "%s/%d/%zu/%d", key, c->opt_refresh, c->mma_cap, (int)c->bp_room);
         if (!s.graph || s.graph_key != key2) {
             for (cudaGraphExec_t* gx : {&s.graph, &s.graph_inc})
                 if (*gx) {

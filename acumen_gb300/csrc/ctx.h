@@ -109,6 +109,8 @@ struct acu_ctx {
     acu::DevBuf pairP, pairPT;   // pair images of the single-precision projector
     acu::DevBuf lineL, lineA;    // line image and ray sums of projector variant 6
     acu::DevBuf mmaT, mmaP, mmaF; // tiles, partial sums and flags of the tensor-core projector
+    size_t mma_cap = acu::MMA_PART_CAP;   // bytes of mmaP at most; smaller once memory ran out, 0: no room for it
+    bool bp_room = true;          // memory did not run out for bpQ
     acu::DevBuf bpQ, bpS;         // bins in operand layout and per-slice scalars of the tensor-core backprojection
     acu::DevBuf w_part;          // FP64 / int64 partial sums of the preprocessing reductions
     double* pinned = nullptr;    // their results in host memory (MIRROR_MAX of them)

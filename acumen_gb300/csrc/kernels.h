@@ -116,7 +116,7 @@ std::vector<MmaAngle> mma_angles(const float* xsc, int T, int N, int stretches);
 bool mma_fits(int N);
 std::vector<int> mma_groups(const std::vector<MmaAngle>& ang);
 size_t mma_flag_words(int G);
-MmaPlan mma_plan(const DevGeom<float>& g, int G);
+MmaPlan mma_plan(const DevGeom<float>& g, int G, size_t cap);
 void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned char* tiles, float* P, int* flags,
                       const MmaPlan& p, float* sino, cudaStream_t st);
 // Backprojection on the tensor cores (kernels_bp_mma.cu; exact positions): work

@@ -724,7 +724,7 @@ static int chunk_end(int first, int last, int ng, int ga)
 // Groups of angles at once: as many as keep the rows that the SMs are adding to
 // in the L2 cache (bulk reductions there ran at 6.3 TB/s, at 3.3 where the rows
 // were 150 MB).  More would read the tiles less often (64 KB per tile and chunk).
-MmaPlan mma_plan(const DevGeom<float>& g, int G)
+MmaPlan mma_plan(const DevGeom<float>& g, int G, size_t cap)
 {
     MmaPlan p;
     p.nt = (g.N + TP - 1) / TP;
@@ -746,7 +746,7 @@ MmaPlan mma_plan(const DevGeom<float>& g, int G)
                 rows = std::max(rows, part_rows(g, a, b));
             }
         }
-        if (row * rows * units * p.nb <= MMA_PART_CAP || (p.nb <= 2 && p.ng == 1)) break;
+        if (row * rows * units * p.nb <= cap || (p.nb <= 2 && p.ng == 1)) break;
         if (p.nb > 2) p.nb -= 2;
         else --p.ng;
     }

@@ -115,3 +115,23 @@ def test_in_the_solver():
     mask = t.backproject(torch.ones(1, T, N, device="cuda"))[0] != 0
     assert rel(tv[:, mask], ref[:, mask]) < 2e-5
     t.close()
+
+
+def test_little_memory():
+    """Where the work buffers do not fit, smaller chunks and then the gathers take over."""
+    N, T, S = 513, 180, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.rand(S, N, N, device="cuda", generator=g)
+    t = Tomography(N, syn.angles(T), 25)
+    p, img = t.radon(x), t.iradon(t.radon(x))
+    t.close()
+    torch.cuda.empty_cache()
+    for room in (1500, 550):      # MB: three images of the batch are 200
+        t = Tomography(N, syn.angles(T), 25)
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (room << 20), dtype=torch.uint8, device="cuda")
+        got = t.radon(x)
+        back = t.iradon(p)
+        del hold
+        torch.cuda.empty_cache()
+        assert rel(got, p) < 3e-6 and rel(back, img) < 3e-6
+        t.close()
