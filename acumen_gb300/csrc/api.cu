@@ -322,7 +322,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
             CKRET(ensure_projector_buffers(c, G));
             radon_quads(c, g, G, lin, lout);
         } else if constexpr (V == 1 && sizeof(Real) == 4) {
-            CK(c, c->pairPT.ensure(sizeof(float) * nimg * G));
+            CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg * G));
             launch_radon_v1_fast(g, G, lin, c->pairPT.template as<float>(), lout, c->stream);
         } else {
             launch_radon<Real, V>(g, G, lin, lout, c->stream);
@@ -538,7 +538,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
         CKRET(ensure_projector_buffers(c, G));
         CKRET(ensure_backproject_buffers(c, G));
     } else if constexpr (sizeof(Real) == 4) {
-        CK(c, c->pairPT.ensure(sizeof(float) * nimg));
+        CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg));
     }
     const int Sp = G * V;
     s.nblk = (int)std::min<size_t>(((size_t)N * N + 255) / 256, 512);

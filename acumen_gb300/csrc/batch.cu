@@ -26,7 +26,8 @@ namespace acu {
 
 // One staggered ray of the single-slice projector at the reference's positions
 // (as radon_stag_ray<1> in kernels_radon.cu), through the image (TR = false) or its
-// transpose, over the warp's steps i0..i1.  Exact positions: fx_ray (fixed.cuh).
+// transpose, over the warp's steps i0..i1.  Exact positions: fx_ray (fixed.cuh)
+// through pairs.
 template <bool TR>
 __device__ __forceinline__ void radon_stag_ray_v1(const float* __restrict__ base, int N, int kb, int i0, int i1,
                                                   const ProjRay<float, false>& ray, float mid, int jy,
@@ -90,8 +91,9 @@ __global__ void __launch_bounds__(512) k_batch_radon(const ProbDesc* __restrict_
         const ProjRay<float, EX> ray(sc + d.sc, xsc + d.sc / 2, t, jy, d.mid, nullptr);
         if constexpr (EX) {
             const FxAngle a = fx[d.sc / 2 + t];
-            const float v = llabs(a.c) > llabs(a.s) ? fx_ray<true>(IT + d.img, N, a, ray, jy, lane)
-                                                    : fx_ray<false>(img + d.img, N, a, ray, jy, lane);
+            const bool tr = llabs(a.c) > llabs(a.s);
+            const float2* const P = reinterpret_cast<const float2*>(tr ? IT : img) + d.img;   // pairs
+            const float v = tr ? fx_ray<true>(P, N, a, ray, jy, lane) : fx_ray<false>(P, N, a, ray, jy, lane);
             if (jy <= N) sino[d.sino + (size_t)t * N + (jy - 1)] = v / (float)N;
         } else {
         const bool transposed = fabsf(c) > fabsf(s);
@@ -139,6 +141,17 @@ __global__ void __launch_bounds__(256) k_batch_transpose(const ProbDesc* __restr
         const int ty = i / 32, tx = i % 32;
         if (x0 + ty < N && y0 + tx < N) dst[(size_t)(x0 + ty) * N + y0 + tx] = tile[tx][ty];
     }
+}
+
+// the same as pairs (fixed.cuh): of the images, then of their transposes
+__global__ void __launch_bounds__(256) k_batch_pairs(const ProbDesc* __restrict__ pd, int nprob,
+                                                     const float* __restrict__ img, float2* __restrict__ P,
+                                                     float2* __restrict__ PT)
+{
+    const long long it = blockIdx.x;
+    const ProbDesc d = pd[find_prob<&ProbDesc::it_tr>(pd, nprob, it)];
+    const int nt = (d.N + 31) / 32, local = (int)(it - d.it_tr);
+    pair_tile(img + d.img, P + d.img, PT + d.img, d.N, local % nt * 32, local / nt * 32);
 }
 
 // ---- backprojection: one block item = a 32-pixel-wide tile of one problem; here at the reference's positions ----
@@ -511,12 +524,17 @@ static int sm_count()
 
 void batch_radon(const BatchDev& b, const float* img, float* sino, int slot, cudaStream_t st)
 {
-    k_batch_transpose<<<(unsigned)b.n_tr, 256, 0, st>>>(b.pd, b.nprob, img, b.IT);
+    float* const PT = b.IT + 2 * b.img_total;   // exact positions: the transposes' pairs after the images'
+    if (b.exact)
+        k_batch_pairs<<<(unsigned)b.n_tr, 256, 0, st>>>(b.pd, b.nprob, img, reinterpret_cast<float2*>(b.IT),
+                                                        reinterpret_cast<float2*>(PT));
+    else
+        k_batch_transpose<<<(unsigned)b.n_tr, 256, 0, st>>>(b.pd, b.nprob, img, b.IT);
     cudaMemsetAsync(b.counter + slot, 0, sizeof(int), st);
     const int threads = 32 * b.radon_warps;
     const int blocks = sm_count() * (2048 / threads);
     if (b.exact)
-        k_batch_radon<true><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.fx_fp,
+        k_batch_radon<true><<<blocks, threads, 0, st>>>(b.pd, b.nprob, b.IT, PT, sino, b.sc_fp, b.xsc_fp, b.fx_fp,
                                                         b.n_radon, b.counter + slot);
     else
         k_batch_radon<false><<<blocks, threads, 0, st>>>(b.pd, b.nprob, img, b.IT, sino, b.sc_fp, b.xsc_fp, b.fx_fp,
@@ -893,8 +911,9 @@ int ensure_state(acu_batch* b)
     const size_t ni = sizeof(float) * (size_t)b->dev.img_total, ns = sizeof(float) * (size_t)b->dev.sino_total;
     for (DevBuf* x : {&b->f, &b->fk, &b->ruk, &b->rp}) CK(c, x->ensure(ns));
     CK(c, b->q.ensure(2 * ns));   // exact positions: pairs of bins
-    for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->rhs, &b->r, &b->p, &b->Ap, &b->tmp, &b->it_img})
+    for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->rhs, &b->r, &b->p, &b->Ap, &b->tmp})
         CK(c, x->ensure(ni));
+    CK(c, b->it_img.ensure(4 * ni));   // exact positions: pairs of the images and of their transposes
     b->dev.IT = b->it_img.as<float>();
     CK(c, b->part.ensure(sizeof(double) * (size_t)b->dev.n_ew));
     for (DevBuf* x : {&b->rsold, &b->alpha, &b->beta}) CK(c, x->ensure(sizeof(double) * b->nprob));

@@ -20,16 +20,35 @@ namespace acu {
 __device__ __forceinline__ int fx_cell(long long v) { return (int)(v >> 32); }
 __device__ __forceinline__ float fx_frac(long long v)
 {
-    return __uint_as_float(((unsigned)v >> 9) | 0x3f800000u) - 1.f;
+    return __uint_as_float(__funnelshift_r((unsigned)v, 0x3f800000u >> 23, 9)) - 1.f;   // 1.fraction, less 1
 }
 constexpr long long FX_HALF = 1ll << 8;   // half of the fraction's last kept bit: fractions are rounded, not cut
+
+// One 32 x 32 tile (at x0, y0, 0-based) of an image as pairs (pixel, next pixel of
+// the row) and of its transpose likewise, by a block of 256: a tap row of the
+// projector is one load.
+__device__ __forceinline__ void pair_tile(const float* __restrict__ img, float2* __restrict__ P, float2* __restrict__ PT,
+                                          int N, int x0, int y0)
+{
+    __shared__ float tile[33][34];
+    for (int i = threadIdx.x; i < 33 * 33; i += 256) {
+        const int ty = i / 33, tx = i % 33;
+        tile[ty][tx] = x0 + tx < N && y0 + ty < N ? img[(size_t)(y0 + ty) * N + x0 + tx] : 0.f;
+    }
+    __syncthreads();
+    const int a = threadIdx.x & 31;
+    for (int b = threadIdx.x >> 5; b < 32; b += 8) {
+        if (x0 + a < N && y0 + b < N) P[(size_t)(y0 + b) * N + x0 + a] = make_float2(tile[b][a], tile[b][a + 1]);
+        if (y0 + a < N && x0 + b < N) PT[(size_t)(x0 + b) * N + y0 + a] = make_float2(tile[a][b], tile[a + 1][b]);
+    }
+}
 
 // One ray (bin jy) of the single-slice projector: the sum of its samples.  The
 // rays of a warp are staggered so that the 32 samples of a step lie in one or two
 // rows of the copy read.  TR: through the transpose (rows follow x), else the
 // image (rows follow y).
 template <bool TR>
-__device__ __forceinline__ float fx_ray(const float* __restrict__ base, int N, FxAngle a,
+__device__ __forceinline__ float fx_ray(const float2* __restrict__ base, int N, FxAngle a,
                                         const ProjRay<float, true>& ray, int jy, int lane)
 {
     const int m = (N + 1) / 2;
@@ -88,6 +107,7 @@ __device__ __forceinline__ float fx_ray(const float* __restrict__ base, int N, F
     const long long dr = TR ? a.c : a.s, dc = TR ? a.s : a.c;
     const long long steps = (long long)i0 - kb - m;
     long long r = (TR ? xm : ym) + steps * dr, q = (TR ? ym : xm) + steps * dc;
+    const float2* const base0 = base - (N + 1);   // of cell (0, 0)
     float sum = 0.f;
     // a step in which some rays have no sample reads a pixel of the image all the same and drops it: without a branch,
     // the loads of several steps are in flight together
@@ -99,11 +119,11 @@ __device__ __forceinline__ float fx_ray(const float* __restrict__ base, int N, F
             cr = min(max(cr, 1), N - 1);
             cq = min(max(cq, 1), N - 1);
         }
-        const float* p = base + (unsigned)((cr - 1) * N + cq - 1);
+        const float2* p = base0 + (unsigned)(cr * N + cq);
         const float fr = fx_frac(r), fc = fx_frac(q);
-        const float v00 = __ldg(p), v01 = __ldg(p + 1), v10 = __ldg(p + N), v11 = __ldg(p + N + 1);
+        const float2 v0 = __ldg(p), v1 = __ldg(p + N);
         const float gr = 1.f - fr, gc = 1.f - fc;
-        const float t = fmaf(v01, fc, v00 * gc), b = fmaf(v11, fc, v10 * gc);
+        const float t = fmaf(v0.y, fc, v0.x * gc), b = fmaf(v1.y, fc, v1.x * gc);
         const float next = fmaf(b, fr, fmaf(t, gr, sum));
         sum = ok ? next : sum;
         r += dr;

@@ -128,7 +128,7 @@ size_t bp_mma_scalars(int G);
 bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
                             cudaStream_t st);
 // The staggered projector for one slice per thread (plain layout); IT is a
-// work buffer of N * N floats per slice.
+// work buffer of 4 N * N floats per slice (pairs of the image and its transpose).
 // Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
 // (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
 // the derivative with respect to them or null; launch_backproject_fx: q as pairs

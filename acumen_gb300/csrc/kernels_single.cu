@@ -15,12 +15,19 @@ namespace acu {
 
 namespace {
 
+__global__ void __launch_bounds__(256) k_pair_images(const float* __restrict__ img, float2* __restrict__ P,
+                                                     float2* __restrict__ PT, int N)
+{
+    const size_t g = blockIdx.z, at = g * N * N;
+    pair_tile(img + at, P + at, PT + at, N, blockIdx.x * 32, blockIdx.y * 32);
+}
+
 // grid (128 rays, angle in copy order, slice).  Held by the instructions of a
-// sample (31 issue slots, 4 of them loads) and the latency of its four loads: 12 blocks an SM
-// rather than 9 gain 6 %, deeper unrolling nothing.  Against positions from split
-// tables (us, before / now): 363^2 x 360 159 / 99, 725^2 x 720 882 / 453,
-// 1449^2 x 900 3896 / 1955, 2049^2 x 1200 9979 / 4969.
-__global__ void __launch_bounds__(128, 12) k_ray_fx(const float* __restrict__ I, const float* __restrict__ IT,
+// sample and by its two loads (the taps of a row as pairs: four single loads took 4 to 15 %
+// longer); deeper unrolling and more blocks an SM gain nothing.  Against positions
+// from split tables (us, before / now): 363^2 x 360 159 / 84, 725^2 x 720 882 / 408,
+// 1449^2 x 900 3896 / 1802, 2049^2 x 1200 9979 / 4761.
+__global__ void __launch_bounds__(128, 8) k_ray_fx(const float2* __restrict__ I, const float2* __restrict__ IT,
                                                     const FxAngle* __restrict__ fx, const float4* __restrict__ xsc,
                                                     const int* __restrict__ order, float* __restrict__ sino, int N,
                                                     int T, float mid)
@@ -242,8 +249,9 @@ std::vector<FxAngle> fx_angles(const float* xsc, int T)
 
 void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st)
 {
-    launch_transpose_v1(g.N, S, img, IT, st);
-    k_ray_fx<<<dim3((g.N + 127) / 128, g.T, S), dim3(32, 4), 0, st>>>(img, IT, g.fx_fp, g.xsc_fp, g.fp_order, sino, g.N,
+    float2 *P = reinterpret_cast<float2*>(IT), *PT = P + (size_t)g.N * g.N * S;
+    k_pair_images<<<dim3((g.N + 31) / 32, (g.N + 31) / 32, S), 256, 0, st>>>(img, P, PT, g.N);
+    k_ray_fx<<<dim3((g.N + 127) / 128, g.T, S), dim3(32, 4), 0, st>>>(P, PT, g.fx_fp, g.xsc_fp, g.fp_order, sino, g.N,
                                                                      g.T, g.mid);
 }
 
