@@ -928,7 +928,7 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     if constexpr (sizeof(Real) == 4) fused = g.exact != 0;
     if constexpr (sizeof(Real) == 4) {
         if (fused) {
-            CK(c, c->pairPT.ensure(sizeof(float) * nimg * S));
+            CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg * S));
             launch_ray_off(g, S, d_u, c->pairPT.template as<float>(), d_off, r, d_grad_off ? D : nullptr, st);
         }
     }

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(128, 8) k_ray_fx(const float2* __restrict__ I,
 // Held by the instructions of the positions.  Two slices, 1025^2 x 600: 3.31 ms the
 // projection and 3.40 ms the derivative there, 2.65 ms both here.
 template <bool TR, bool GRAD>
-__device__ __forceinline__ void ray_off(const float* __restrict__ base, int N, float s, float c,
+__device__ __forceinline__ void ray_off(const float2* __restrict__ base, int N, float s, float c,
                                         const ProjRay<float, true>& ray, float mid, int jy, float off, int lane,
                                         float& sum, float& der)
 {
@@ -71,8 +71,9 @@ __device__ __forceinline__ void ray_off(const float* __restrict__ base, int N, f
         float wxl, wxh, wyl, wyh;
         ray.at((float)jx - mid, x1, y1, wxl, wxh, wyl, wyh);
         if (jx >= lo && jx <= hi && min(x1, y1) > 1 && max(x1, y1) < N) {
-            const float* p = base + (TR ? (unsigned)((x1 - 1) * N + y1 - 1) : (unsigned)((y1 - 1) * N + x1 - 1));
-            const float a = __ldg(p), b = __ldg(p + (TR ? N : 1)), cc = __ldg(p + (TR ? 1 : N)), d = __ldg(p + N + 1);
+            const float2* p = base + (TR ? (unsigned)((x1 - 1) * N + y1 - 1) : (unsigned)((y1 - 1) * N + x1 - 1));
+            const float2 v0 = __ldg(p), v1 = __ldg(p + N);
+            const float a = v0.x, b = TR ? v1.x : v0.y, cc = TR ? v0.y : v1.x, d = v1.y;
             const float w11 = wxl * wyl, w21 = wxh * wyl, w12 = wxl * wyh, w22 = wxh * wyh;
             sum = fmaf(d, w22, fmaf(cc, w12, fmaf(b, w21, fmaf(a, w11, sum))));
             if constexpr (GRAD) {
@@ -85,7 +86,7 @@ __device__ __forceinline__ void ray_off(const float* __restrict__ base, int N, f
 }
 
 template <bool GRAD>
-__global__ void __launch_bounds__(128) k_ray_off(const float* __restrict__ I, const float* __restrict__ IT,
+__global__ void __launch_bounds__(128) k_ray_off(const float2* __restrict__ I, const float2* __restrict__ IT,
                                                  const float* __restrict__ sc, const float4* __restrict__ xsc,
                                                  const int* __restrict__ order, const float* __restrict__ off,
                                                  float* __restrict__ sino, float* __restrict__ dsino, int N, int T,
@@ -258,12 +259,13 @@ void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT
 void launch_ray_off(const DevGeom<float>& g, int S, const float* img, float* IT, const float* off, float* sino,
                     float* dsino, cudaStream_t st)
 {
-    launch_transpose_v1(g.N, S, img, IT, st);
+    float2 *P = reinterpret_cast<float2*>(IT), *PT = P + (size_t)g.N * g.N * S;
+    k_pair_images<<<dim3((g.N + 31) / 32, (g.N + 31) / 32, S), 256, 0, st>>>(img, P, PT, g.N);
     const dim3 blk(32, 4), grd((g.N + 127) / 128 * g.T, 1, S);
     if (dsino)
-        k_ray_off<true><<<grd, blk, 0, st>>>(img, IT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
+        k_ray_off<true><<<grd, blk, 0, st>>>(P, PT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
     else
-        k_ray_off<false><<<grd, blk, 0, st>>>(img, IT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
+        k_ray_off<false><<<grd, blk, 0, st>>>(P, PT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
 }
 
 void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, float* img, cudaStream_t st)
