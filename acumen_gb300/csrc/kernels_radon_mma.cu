@@ -235,15 +235,15 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                     uint32_t h0 = 0, h1 = 0, l0 = 0, l1 = 0;
                     int pair = -100;
                     if (live && __any_sync(0xffffffffu, px <= N && py <= N)) {
-                        const float ey = (float)py - mid;
+                        const RayPos at = ray_pos(a.x, ex, (float)py - mid, 0.f, mid);
                         float wv[3];
                         int j;
                         if (rim && __any_sync(0xffffffffu, on_rim(px, py, N))) {
-                            ray_weights<RIM>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                            ray_weights<RIM>(a, at, 0.f, mid, px, py, N, j, wv);
                         } else if (ends) {
-                            ray_weights<ENDS>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                            ray_weights<ENDS>(a, at, 0.f, mid, px, py, N, j, wv);
                         } else {
-                            ray_weights<INNER>(a, ex, ey, 0.f, mid, px, py, N, j, wv);
+                            ray_weights<INNER>(a, at, 0.f, mid, px, py, N, j, wv);
                         }
                         // the leading 11 bits are exact in half precision, the rest is rounded
                         float hi[3];

@@ -164,34 +164,52 @@ __device__ __forceinline__ void put_image(float* __restrict__ img, Lanes<float, 
 // weights there.  The general kernel (k_radon_adjoint) evaluates the projector at
 // 16 candidate samples per pixel and angle; this one evaluates the nine bilinear
 // weights that can differ from zero, from one position (ray_weights.cuh): held by
-// those instructions.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.65,
-// 1449^2 x 900 66.0 / 7.5, 2049^2 x 1200 170.9 / 19.2.  V slices per thread; off:
+// those instructions; a block forms an angle's position once and its pixels step
+// from there.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.46,
+// 1449^2 x 900 66.0 / 6.6, 2049^2 x 1200 170.9 / 16.8.  V slices per thread; off:
 // per-slice angle offsets or null (V = 1).
 template <int V>
 __global__ void __launch_bounds__(256) k_adjoint_fx(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
                                                     const float* __restrict__ off, float* __restrict__ img, int N,
                                                     int T, float mid)
 {
-    const int px = blockIdx.x * 32 + threadIdx.x + 1, py = blockIdx.y * 8 + threadIdx.y + 1;
+    __shared__ RayFrame frames[FX_CHUNK];
+    __shared__ float4 slopes[FX_CHUNK];
+    const int tid = threadIdx.y * 32 + threadIdx.x, x0 = blockIdx.x * 32 + 1, y0 = blockIdx.y * 8 + 1;
+    const int px = x0 + threadIdx.x, py = y0 + threadIdx.y;
     const size_t g = blockIdx.z;
-    if (px > N || py > N || on_rim(px, py, N)) return;   // the rim: k_adjoint_rim
+    const bool inside = px <= N && py <= N && !on_rim(px, py, N);   // the rim: k_adjoint_rim
     Lanes<float, V> acc{};
-    const float ex = (float)px - mid, ey = (float)py - mid;
     const float* y = sino + g * T * N * V;
+    for (int t0 = 0; t0 < T; t0 += FX_CHUNK) {
+        const int n = min(FX_CHUNK, T - t0);
+        __syncthreads();
+        if (tid < n) {
+            const MmaAngle a = ang[t0 + tid];
+            frames[tid] = RayFrame(a.x, (float)(x0 + 16) - mid, (float)(y0 + 4) - mid, off ? off[g * T + t0 + tid] : 0.f, mid);
+            slopes[tid] = make_float4(a.c, a.s, a.t, 0.f);
+        }
+        __syncthreads();
+        if (!inside) continue;
 #pragma unroll 1
-    for (int t = 0; t < T; ++t, y += (size_t)N * V) {
-        const MmaAngle a = ang[t];
-        const float o = off ? __ldg(off + g * T + t) : 0.f;
-        const float u = fmaf(a.c, ex, fmaf(a.s, ey, mid));
-        int j;
-        float w[3];
-        if (u < 4.f || u > (float)N - 3.f)
-            ray_weights<ENDS>(a, ex, ey, o, mid, px, py, N, j, w);
-        else
-            ray_weights<INNER>(a, ex, ey, o, mid, px, py, N, j, w);
-        add_rays<V>(acc, y, w, j, N);
+        for (int i = 0; i < n; ++i, y += (size_t)N * V) {
+            RayFrame f = frames[i];
+            f.move((int)threadIdx.x - 16, (int)threadIdx.y - 4);
+            MmaAngle a;
+            a.c = slopes[i].x;
+            a.s = slopes[i].y;
+            a.t = slopes[i].z;
+            const RayPos p = f.pos();
+            int j;
+            float w[3];
+            if (p.cu < 4 || p.cu > N - 4)
+                ray_weights<ENDS>(a, p, 0.f, mid, px, py, N, j, w);
+            else
+                ray_weights<INNER>(a, p, 0.f, mid, px, py, N, j, w);
+            add_rays<V>(acc, y, w, j, N);
+        }
     }
-    put_image<V>(img, acc, g, px, py, N);
+    if (inside) put_image<V>(img, acc, g, px, py, N);
 }
 
 // The pixels on the rim, whose samples may lie outside and are looked at one by one: 40 times the work, so in a kernel
@@ -212,7 +230,9 @@ __global__ void __launch_bounds__(256) k_adjoint_rim(const float* __restrict__ s
         for (int t = lane; t < T; t += 32) {
             int j;
             float w[3];
-            ray_weights<RIM>(ang[t], (float)px - mid, (float)py - mid, off ? off[g * T + t] : 0.f, mid, px, py, N, j, w);
+            const MmaAngle a = ang[t];
+            const float o = off ? off[g * T + t] : 0.f;
+            ray_weights<RIM>(a, ray_pos(a.x, (float)px - mid, (float)py - mid, o, mid), o, mid, px, py, N, j, w);
             add_rays<V>(acc, sino + (g * T + t) * N * V, w, j, N);
         }
 #pragma unroll

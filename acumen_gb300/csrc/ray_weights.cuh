@@ -2,6 +2,7 @@
 // tensor-core projector, which gathers them into a matrix, and the transpose.
 #pragma once
 #include "common.cuh"
+#include "fixed.cuh"
 #include "kernels.h"
 
 namespace acu {
@@ -18,9 +19,56 @@ __device__ __forceinline__ bool sample_valid(float4 x, float k, int j, float off
     return fminf(cx, cy) > 1.f && fmaxf(cx, cy) < (float)N;
 }
 
-// The weights of the three rays j, j+1, j+2 nearest to pixel (px, py) (ex, ey:
-// relative to the middle; off: the angle's detector offset).  Ray j's samples sit
-// at the pixel's distance (dx, dy) = (c e - s d, s e + c d) with d = j - w,
+// A pixel's coordinates along (u) and across (w) the rays: cells and fractions.
+struct RayPos {
+    int cu, cw;
+    float uf, wf;
+};
+
+// Exact positions (split tables); ex, ey: the pixel's place relative to the middle, off: the angle's detector offset.
+__device__ __forceinline__ RayPos ray_pos(float4 x, float ex, float ey, float off, float mid)
+{
+    RayPos p;
+    float cell;
+    split_floor(__fmaf_rn(x.y, ex, __fmaf_rn(x.x, ey, mid)), __fmaf_rn(x.w, ex, __fmul_rn(x.z, ey)), cell, p.uf);
+    p.cu = (int)cell;
+    split_floor(__fmaf_rn(-x.x, ex, __fmaf_rn(x.y, ey, mid)), __fmaf_rn(-x.z, ex, __fmul_rn(x.w, ey)) - off, cell, p.wf);
+    p.cw = fabsf(off) < 1e6f ? (int)cell : -(1 << 30);   // no number, or too far out: meets no ray
+    return p;
+}
+
+// The pixels around one pixel: its exact coordinates, and the
+// steps from one to the next, with 26 fraction bits.  Within 31 cells a fraction is off by
+// 5e-7 at most (half a bit of either step per pixel); 6 instructions a
+// coordinate in place of 14.  It pays where a frame serves many pixels (the transpose);
+// in the tensor-core projector, where it serves two, it took 3 % longer.
+struct RayFrame {
+    int u, w, c, s, cu, cw;
+    RayFrame() = default;
+    __device__ __forceinline__ RayFrame(float4 x, float ex, float ey, float off, float mid)
+    {
+        constexpr float ONE = 67108864.f;   // 2^26
+        const RayPos p = ray_pos(x, ex, ey, off, mid);
+        cu = p.cu;
+        cw = p.cw;
+        u = (int)(p.uf * ONE) + 4;   // 4: half of the fraction's last kept bit
+        w = (int)(p.wf * ONE) + 4;
+        s = (int)(x.x * ONE) + __float2int_rn(x.z * ONE);
+        c = (int)(x.y * ONE) + __float2int_rn(x.w * ONE);
+    }
+    __device__ __forceinline__ void move(int dx, int dy)
+    {
+        u += dx * c + dy * s;
+        w += dy * c - dx * s;
+    }
+    __device__ __forceinline__ RayPos pos() const
+    {
+        return {cu + (u >> 26), cw + (w >> 26), fx_frac((long long)(unsigned)(u << 6)), fx_frac((long long)(unsigned)(w << 6))};
+    }
+};
+
+// The weights of the three rays j, j+1, j+2 nearest to pixel (px, py) at p (off:
+// the angle's detector offset).  Ray j's samples sit at the pixel's distance (dx, dy) = (c e - s d, s e + c d) with d = j - w,
 // e = k - u, where (u, w) are the pixel's coordinates along and across the rays;
 // the bilinear weight of a sample is (1 - |dx|)+ (1 - |dy|)+.  Of the integers
 // e + u only the three nearest to the ray's closest approach reach the pixel.
@@ -29,15 +77,13 @@ __device__ __forceinline__ bool sample_valid(float4 x, float k, int j, float off
 enum { INNER, ENDS, RIM };
 
 template <int WHERE>
-__device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float ey, float off, float mid, int px, int py,
-                                            int N, int& j, float (&wv)[3])
+__device__ __forceinline__ void ray_weights(const MmaAngle& a, RayPos at, float off, float mid, int px, int py, int N,
+                                            int& j, float (&wv)[3])
 {
-    float cu, cw, uf, wf;
-    split_floor(__fmaf_rn(a.x.y, ex, __fmaf_rn(a.x.x, ey, mid)), __fmaf_rn(a.x.w, ex, __fmul_rn(a.x.z, ey)), cu, uf);
-    split_floor(__fmaf_rn(-a.x.x, ex, __fmaf_rn(a.x.y, ey, mid)), __fmaf_rn(-a.x.z, ex, __fmul_rn(a.x.w, ey)) - off, cw, wf);
-    const float i0 = wf > 0.5f ? 0.f : -1.f;   // |d| < |c| + |s| <= 1.42 leaves three candidates
-    j = (int)(cw + i0);
-    const float d0 = i0 - wf;
+    const float uf = at.uf;
+    const bool up = at.wf > 0.5f;   // |d| < |c| + |s| <= 1.42 leaves three candidates
+    j = at.cw - (up ? 0 : 1);
+    const float d0 = (up ? 0.f : -1.f) - at.wf;
     const float2 along = make_float2(a.c, a.s), back = make_float2(-a.c, -a.s), across = make_float2(-a.s, a.c);
     const float2 one = make_float2(1.f, 1.f);
 #pragma unroll
@@ -55,7 +101,7 @@ __device__ __forceinline__ void ray_weights(const MmaAngle& a, float ex, float e
             if constexpr (WHERE == INNER) {
                 w = fmaf(hx, hy, w);
             } else {
-                const float k = cu + kf + (float)q;
+                const float k = (float)at.cu + kf + (float)q;
                 bool ok = k >= 1.f && k <= (float)N;
                 if constexpr (WHERE == RIM) {
                     // within 1e-5 of a cell edge at the rim the projector's own position decides
