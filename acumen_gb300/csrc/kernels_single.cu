@@ -165,51 +165,63 @@ __device__ __forceinline__ void put_image(float* __restrict__ img, Lanes<float, 
 // 16 candidate samples per pixel and angle; this one evaluates the nine bilinear
 // weights that can differ from zero, from one position (ray_weights.cuh): held by
 // those instructions; a block forms an angle's position once and its pixels step
-// from there.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.46,
-// 1449^2 x 900 66.0 / 6.6, 2049^2 x 1200 170.9 / 16.8.  V slices per thread; off:
+// from there.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.44,
+// 1449^2 x 900 66.0 / 6.4, 2049^2 x 1200 170.9 / 15.8.  V slices per thread; off:
 // per-slice angle offsets or null (V = 1).
-template <int V>
+template <int V, int R>   // R: pixel rows a thread
 __global__ void __launch_bounds__(256) k_adjoint_fx(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
                                                     const float* __restrict__ off, float* __restrict__ img, int N,
                                                     int T, float mid)
 {
     __shared__ RayFrame frames[FX_CHUNK];
     __shared__ float4 slopes[FX_CHUNK];
-    const int tid = threadIdx.y * 32 + threadIdx.x, x0 = blockIdx.x * 32 + 1, y0 = blockIdx.y * 8 + 1;
-    const int px = x0 + threadIdx.x, py = y0 + threadIdx.y;
+    const int tid = threadIdx.y * 32 + threadIdx.x, x0 = blockIdx.x * 32 + 1, y0 = blockIdx.y * (8 * R) + 1;
+    const int px = x0 + threadIdx.x, py = y0 + threadIdx.y * R;
     const size_t g = blockIdx.z;
-    const bool inside = px <= N && py <= N && !on_rim(px, py, N);   // the rim: k_adjoint_rim
-    Lanes<float, V> acc{};
+    bool inside[R], any = false;   // the rim: k_adjoint_rim
+    Lanes<float, V> acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        inside[r] = px <= N && py + r <= N && !on_rim(px, py + r, N);
+        any |= inside[r];
+        acc[r] = Lanes<float, V>{};
+    }
     const float* y = sino + g * T * N * V;
     for (int t0 = 0; t0 < T; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, T - t0);
         __syncthreads();
         if (tid < n) {
             const MmaAngle a = ang[t0 + tid];
-            frames[tid] = RayFrame(a.x, (float)(x0 + 16) - mid, (float)(y0 + 4) - mid, off ? off[g * T + t0 + tid] : 0.f, mid);
+            frames[tid] = RayFrame(a.x, (float)(x0 + 16) - mid, (float)(y0 + 4 * R) - mid, off ? off[g * T + t0 + tid] : 0.f, mid);
             slopes[tid] = make_float4(a.c, a.s, a.t, 0.f);
         }
         __syncthreads();
-        if (!inside) continue;
+        if (!any) continue;
 #pragma unroll 1
         for (int i = 0; i < n; ++i, y += (size_t)N * V) {
             RayFrame f = frames[i];
-            f.move((int)threadIdx.x - 16, (int)threadIdx.y - 4);
+            f.move((int)threadIdx.x - 16, (int)threadIdx.y * R - 4 * R);
             MmaAngle a;
             a.c = slopes[i].x;
             a.s = slopes[i].y;
             a.t = slopes[i].z;
-            const RayPos p = f.pos();
-            int j;
-            float w[3];
-            if (p.cu < 4 || p.cu > N - 4)
-                ray_weights<ENDS>(a, p, 0.f, mid, px, py, N, j, w);
-            else
-                ray_weights<INNER>(a, p, 0.f, mid, px, py, N, j, w);
-            add_rays<V>(acc, y, w, j, N);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const RayPos p = f.pos();
+                int j;
+                float w[3];
+                if (p.cu < 4 || p.cu > N - 4)
+                    ray_weights<ENDS>(a, p, 0.f, mid, px, py + r, N, j, w);
+                else
+                    ray_weights<INNER>(a, p, 0.f, mid, px, py + r, N, j, w);
+                add_rays<V>(acc[r], y, w, j, N);
+                f.move(0, 1);
+            }
         }
     }
-    if (inside) put_image<V>(img, acc, g, px, py, N);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (inside[r]) put_image<V>(img, acc[r], g, px, py + r, N);
 }
 
 // The pixels on the rim, whose samples may lie outside and are looked at one by one: 40 times the work, so in a kernel
@@ -305,8 +317,18 @@ void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, floa
 template <int V>
 void launch_adjoint_fx(const DevGeom<float>& g, int G, const float* sino, const float* off, float* img, cudaStream_t st)
 {
-    k_adjoint_fx<V><<<dim3((g.N + 31) / 32, (g.N + 7) / 8, G), dim3(32, 8), 0, st>>>(sino, g.angles, off, img, g.N, g.T,
-                                                                                     g.mid);
+    // rows per thread: more share an angle's entry, fewer keep the chip busy.  Measured with 1 / 2 / 4 rows (ms): 725^2 x
+    // 720 1.47 / 1.44 / 1.77, two of 1025^2 x 600 4.36 / 4.23 / 4.30, 1449^2 x 900 6.58 / 6.43 / 6.35
+    auto run = [&](auto kernel, int rows) {
+        kernel<<<dim3((g.N + 31) / 32, (g.N + 8 * rows - 1) / (8 * rows), G), dim3(32, 8), 0, st>>>(sino, g.angles, off, img,
+                                                                                                 g.N, g.T, g.mid);
+    };
+    if (g.N < 500)
+        run(k_adjoint_fx<V, 1>, 1);
+    else if (g.N < 1400 || V > 1)
+        run(k_adjoint_fx<V, 2>, 2);
+    else
+        run(k_adjoint_fx<V, 4>, 4);
     k_adjoint_rim<V><<<dim3((6 * g.N + 7) / 8, G), 256, 0, st>>>(sino, g.angles, off, img, g.N, g.T, g.mid);
 }
 template void launch_adjoint_fx<1>(const DevGeom<float>&, int, const float*, const float*, float*, cudaStream_t);
