@@ -173,8 +173,8 @@ __device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, con
         }
         __syncthreads();
         const float2* row = q + (size_t)t0 * N;
-        // a block's first touch of an angle's bins comes from L2: 16 loads in flight per thread
-#pragma unroll (16 / R)
+        // a block's first touch of an angle's bins comes from L2: 32 loads in flight per thread
+#pragma unroll (32 / R)
         for (int a = 0; a < n; ++a, row += N) {
             const int4 e = tab[a];
             int p = e.x + lx * e.y + ly * e.z;

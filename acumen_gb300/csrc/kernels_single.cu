@@ -110,10 +110,11 @@ __global__ void __launch_bounds__(128) k_ray_off(const float2* __restrict__ I, c
 
 // Held by issue slots: an update is one 64-bit load, an addition, a shift, a
 // subtraction and two multiply-adds.  Against the gather with both bins loaded and
-// positions from split tables (us, before / now): 725^2 x 720 328 / 195,
-// 1449^2 x 900 1261 / 734, 2049^2 x 1200 3215 / 1712.
+// positions from split tables (us, before / now): 725^2 x 720 328 / 180,
+// 1449^2 x 900 1261 / 713, 2049^2 x 1200 3215 / 1652.  Registers for the loads in flight
+// count more than blocks: with five blocks an SM instead of four 725^2 took 50 % longer.
 template <int R>
-__global__ void __launch_bounds__(256) k_backproject_fx(const float2* __restrict__ q, const float* __restrict__ cmask,
+__global__ void __launch_bounds__(256, R == 1 ? 3 : 4) k_backproject_fx(const float2* __restrict__ q, const float* __restrict__ cmask,
                                                         const float4* __restrict__ xsc, float* __restrict__ img, int N,
                                                         int T, float mid)
 {
@@ -305,7 +306,7 @@ void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, floa
     const dim3 blk(32, 8);
     auto grid = [&](int r) { return dim3((g.N + 31) / 32, (g.N + 8 * r - 1) / (8 * r), S); };
     // rows per thread: more share an angle's entry, fewer keep the chip busy.  Measured with 1 / 2 / 4 rows (us): 363^2 x
-    // 360 55 / 90 / -, 725^2 x 720 200 / 196 / 242, 1449^2 x 900 795 / 768 / 735
+    // 360 50 / 54 / 94, 725^2 x 720 193 / 190 / 252, 1449^2 x 900 813 / 748 / 738
     if (g.N < 500)
         k_backproject_fx<1><<<grid(1), blk, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, g.mid);
     else if (g.N < 1000)
