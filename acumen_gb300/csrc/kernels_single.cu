@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128, 8) k_ray_fx(const float2* __restrict__ I,
 // is a sum of squares of these values, and the derivative jumps where a sample
 // changes its cell, so neither would stand another rounding.
 // Held by the instructions of the positions.  Two slices, 1025^2 x 600: 3.31 ms the
-// projection and 3.40 ms the derivative there, 2.65 ms both here.
+// projection and 3.40 ms the derivative there, 2.4 ms both here.
 template <bool TR, bool GRAD>
 __device__ __forceinline__ void ray_off(const float2* __restrict__ base, int N, float s, float c,
                                         const ProjRay<float, true>& ray, float mid, int jy, float off, int lane,
@@ -64,7 +64,7 @@ __device__ __forceinline__ void ray_off(const float2* __restrict__ base, int N, 
         hi = -0x3fffffff;
     }
     const int i0 = __reduce_min_sync(0xffffffffu, lo + kb), i1 = __reduce_max_sync(0xffffffffu, hi + kb);
-#pragma unroll 2
+#pragma unroll 4
     for (int i = i0; i <= i1; ++i) {
         const int jx = i - kb;
         int x1, y1;
@@ -166,11 +166,11 @@ __device__ __forceinline__ void put_image(float* __restrict__ img, Lanes<float, 
 // 16 candidate samples per pixel and angle; this one evaluates the nine bilinear
 // weights that can differ from zero, from one position (ray_weights.cuh): held by
 // those instructions; a block forms an angle's position once and its pixels step
-// from there.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.44,
-// 1449^2 x 900 66.0 / 6.4, 2049^2 x 1200 170.9 / 15.8.  V slices per thread; off:
+// from there.  One slice (ms, before / now): 725^2 x 720 14.7 / 1.4,
+// 1449^2 x 900 66.0 / 6.2, 2049^2 x 1200 170.9 / 15.5.  V slices per thread; off:
 // per-slice angle offsets or null (V = 1).
 template <int V, int R>   // R: pixel rows a thread
-__global__ void __launch_bounds__(256) k_adjoint_fx(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
+__global__ void __launch_bounds__(256, V == 1 ? 6 : 1) k_adjoint_fx(const float* __restrict__ sino, const MmaAngle* __restrict__ ang,
                                                     const float* __restrict__ off, float* __restrict__ img, int N,
                                                     int T, float mid)
 {
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) k_adjoint_fx(const float* __restrict__ si
         }
         __syncthreads();
         if (!any) continue;
-#pragma unroll 1
+#pragma unroll (V == 1 ? 2 : 1)
         for (int i = 0; i < n; ++i, y += (size_t)N * V) {
             RayFrame f = frames[i];
             f.move((int)threadIdx.x - 16, (int)threadIdx.y * R - 4 * R);
