@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(128) k_radon(const Real* __restrict__ img, con
     const int g = blockIdx.z;
     if (jy > N || t >= T) return;
     // bin jy is read at detector coordinate jy + off[t] (off: per-slice angle offsets, V = 1)
-    const ProjRay<Real, false> ray(sc, nullptr, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
+    const ProjRay<Real, EX> ray(sc, xsc, t, jy, mid, off ? off + (size_t)g * T + t : nullptr);
     const Real* u = img + (size_t)g * N * N * V;
     const size_t rowstride = (size_t)N * V;
     Lanes<Real, V> acc;
