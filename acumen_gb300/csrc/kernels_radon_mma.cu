@@ -70,8 +70,8 @@ constexpr int HALF = NS / 2;                            // partial sums are stor
 // Warps by role.  Two crews take turns at the stages of W; four warps store a block.
 template <int BLK>
 struct Roles {
-    static constexpr int CREWS = 2, OUTS = BLK;
-    static constexpr int MMA = CREWS * CREW, LOAD = MMA + 1, OUT = MMA + 2, ROWS = OUT + 4 * OUTS, WARPS = ROWS + 1;
+    static constexpr int OUTS = BLK;
+    static constexpr int MMA = STAGES * CREW, LOAD = MMA + 1, OUT = MMA + 2, ROWS = OUT + 4 * OUTS, WARPS = ROWS + 1;
 };
 template <int BLK>
 struct Smem {   // tiles of BLK blocks, stages of W, staged output rows, scales, barriers
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                 *reinterpret_cast<uint32_t*>(sm + at + STAGE_HALF) = lo;
             }
         };
-        uint32_t last0[STAGES] = {0, 0}, last1[STAGES] = {0, 0};   // the two words written last time, per stage
-        unsigned n = 0;                                            // groups
+        uint32_t last0 = 0, last1 = 0;   // the two words written last time
+        unsigned n = 0;                  // groups
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x)
         for (Stretch w(u, nt, stretches); w.k0 < w.k1 && ok; ++w.k0) {
             const int x0 = (xm ? w.k0 : w.line) * TP + 1, y0 = (xm ? w.line : w.k0) * TP + 1;
@@ -226,10 +226,8 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                     ends = uc - ur < 1.f || uc + ur > (float)N;   // some rays may end in the tile
                 }
 #pragma unroll 1
-                for (int q0 = 0; q0 < PARTS && ok; q0 += STAGES)
-#pragma unroll
-                for (int own = 0; own < STAGES / R::CREWS; ++own) {
-                    const int st = R::CREWS == 1 ? own : crew, q = q0 + st;
+                for (int q = crew; q < PARTS && ok; q += STAGES) {
+                    const int st = crew;   // a crew has a stage of its own
                     const unsigned fills = (n * PARTS + q) / STAGES;   // of this stage, before
                     const int py = y0 + PART_ROWS * q + trow;
                     uint32_t h0 = 0, h1 = 0, l0 = 0, l1 = 0;
@@ -262,12 +260,12 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                     }
                     ok = umma::bar_wait_warp(&sh.w_empty[st], (fills & 1) ^ 1);
                     if (!ok) break;
-                    put(last0[own], 0, 0);
-                    put(last1[own], 0, 0);
-                    last0[own] = place(pair, st);
-                    last1[own] = place(pair + 1, st);
-                    put(last0[own], h0, l0);
-                    put(last1[own], h1, l1);
+                    put(last0, 0, 0);
+                    put(last1, 0, 0);
+                    last0 = place(pair, st);
+                    last1 = place(pair + 1, st);
+                    put(last0, h0, l0);
+                    put(last1, h1, l1);
                     umma::fence_async_smem();
                     __syncwarp();
                     if (lane == 0) umma::bar_arrive(&sh.w_full[st]);

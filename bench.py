@@ -892,8 +892,8 @@ def main():
                             "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                             "peak_kind": kind, "traffic": traffic,
                             "algorithmic_bytes": alg_bytes, "launch_ms": 1000 * t_radon,
-                            "note": "tensor cores: ~1.76 KB of partial sums written and read per tile, angle and 20 "
-                                    "rays of 64 slices; gather variants: runs from L2 and L1, traffic (from one "
+                            "note": "tensor cores: partial sums are added up in L2 along stretches of tiles, a third of "
+                                    "the rows is written and read; gather variants: runs from L2 and L1, traffic (from one "
                                     "32-slice ncu capture, scaled by 32-slice line groups) is mostly the ray sums "
                                     "carried between the band launches",
                             "l1_level": l1_level(16.0 * N * N * T * S / t_radon / 1e9, clocks, probe,
