@@ -207,18 +207,27 @@ void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q,
     launch_backproject<Real, V>(g, G, q, img, c->stream);
 }
 
-// Floats per bin of the filtered sinogram's buffer: single slices are
-// backprojected from pairs (bin, next bin).
+// Elements of the filtered sinogram's buffer (nsino each, G groups).  Single
+// slices are backprojected from pairs (bin, next bin), some slices at a time.
 template <typename Real, int V>
-constexpr size_t q_width() { return V == 1 && sizeof(Real) == 4 ? 2 : 1; }
+size_t q_size(size_t nsino, int G)
+{
+    const size_t all = nsino * G * V;
+    return V == 1 && sizeof(Real) == 4 ? std::max(all, 2 * nsino * pair_slices(8 * nsino, G)) : all;
+}
 
 template <typename Real, int V>
 void lanes_iradon(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* sino, Real* q, Real* img)
 {
     if constexpr (V == 1 && sizeof(Real) == 4) {
         if (g.exact && c->opt_filter == 0 && g.fft_L > 0 && fft_fits<Real>(g.fft_L)) {
-            launch_filter_fft<Real, V>(g, G, sino, q, c->stream, true);
-            launch_backproject_fx(g, G, reinterpret_cast<const float2*>(q), img, c->stream);
+            const size_t nsino = (size_t)g.T * g.N, nimg = (size_t)g.N * g.N;
+            const int at_once = pair_slices(8 * nsino, G);
+            for (int s = 0; s < G; s += at_once) {
+                const int n = std::min(at_once, G - s);
+                launch_filter_fft<Real, V>(g, n, sino + s * nsino, q, c->stream, true);
+                launch_backproject_fx(g, n, reinterpret_cast<const float2*>(q), img + s * nimg, c->stream);
+            }
             return;
         }
     }
@@ -314,7 +323,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     switch (op) {
     case OP_IRADON:
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
-        CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * V * q_width<Real, V>()));
+        CK(c, c->w_q.ensure(sizeof(Real) * q_size<Real, V>(nsino, G)));
         lanes_iradon<Real, V>(c, g, G, lin, c->w_q.template as<Real>(), lout);
         break;
     case OP_RADON:
@@ -322,7 +331,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
             CKRET(ensure_projector_buffers(c, G));
             radon_quads(c, g, G, lin, lout);
         } else if constexpr (V == 1 && sizeof(Real) == 4) {
-            CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg * G));
+            CK(c, c->pairPT.ensure(sizeof(float) * std::max(nimg * G, pair_image_floats(N, G))));
             launch_radon_v1_fast(g, G, lin, c->pairPT.template as<float>(), lout, c->stream);
         } else {
             launch_radon<Real, V>(g, G, lin, lout, c->stream);
@@ -342,9 +351,14 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
         if constexpr (V == 1 && sizeof(Real) == 4) {
             if (g.exact) {
-                CK(c, c->w_q.ensure(sizeof(Real) * nsino * G * 2));
-                launch_pairs(lin, c->w_q.template as<float2>(), N, nsino * G, c->stream);
-                launch_backproject_fx(g, G, c->w_q.template as<float2>(), lout, c->stream);
+                const int at_once = pair_slices(8 * nsino, G);
+                CK(c, c->w_q.ensure(sizeof(float2) * nsino * at_once));
+                float2* const q = c->w_q.template as<float2>();
+                for (int s = 0; s < G; s += at_once) {
+                    const int n = std::min(at_once, G - s);
+                    launch_pairs(lin + s * nsino, q, N, nsino * n, c->stream);
+                    launch_backproject_fx(g, n, q, lout + s * nimg, c->stream);
+                }
                 break;
             }
         }
@@ -530,7 +544,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     const int N = c->N, T = c->T, G = (S + V - 1) / V;
     const size_t nimg = (size_t)N * N * G * V, nsino = (size_t)T * N * G * V;
     for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CK(c, b->ensure(sizeof(Real) * nsino));
-    CK(c, s.q.ensure(sizeof(Real) * nsino * q_width<Real, V>()));
+    CK(c, s.q.ensure(sizeof(Real) * q_size<Real, V>((size_t)T * N, G)));
     for (DevBuf* b : {&s.uk, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap, &s.tmp})
         CK(c, b->ensure(sizeof(Real) * nimg));
     if (c->opt_verbose) CK(c, s.ukp.ensure(sizeof(Real) * nimg));
@@ -538,7 +552,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
         CKRET(ensure_projector_buffers(c, G));
         CKRET(ensure_backproject_buffers(c, G));
     } else if constexpr (sizeof(Real) == 4) {
-        CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg));
+        CK(c, c->pairPT.ensure(sizeof(float) * std::max(nimg, pair_image_floats(N, G))));
     }
     const int Sp = G * V;
     s.nblk = (int)std::min<size_t>(((size_t)N * N + 255) / 256, 512);
@@ -928,7 +942,7 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     if constexpr (sizeof(Real) == 4) fused = g.exact != 0;
     if constexpr (sizeof(Real) == 4) {
         if (fused) {
-            CK(c, c->pairPT.ensure(sizeof(float) * 4 * nimg * S));
+            CK(c, c->pairPT.ensure(sizeof(float) * pair_image_floats(N, S)));
             launch_ray_off(g, S, d_u, c->pairPT.template as<float>(), d_off, r, d_grad_off ? D : nullptr, st);
         }
     }

@@ -627,7 +627,7 @@ struct acu_batch {
     std::vector<int> order;           // execution order (largest work first) -> caller index
     BatchDev dev;
     DevBuf d_pd, d_sc_bp, d_sc_fp, d_xsc_bp, d_xsc_fp, d_fx_fp, d_cm, d_fh, d_fhx, d_tw, d_counter;
-    DevBuf f, fk, ruk, rp, q, uk, dx, dy, bx, by, rhs, r, p, Ap, tmp, part, rsold, alpha, beta, it_img;
+    DevBuf f, fk, ruk, rp, q, uk, dx, dy, bx, by, rhs, r, p, Ap, tmp, part, rsold, alpha, beta;
     DevBuf io_in, io_out;
     cudaGraphExec_t graph = nullptr, graph_inc = nullptr;
     std::string graph_key;
@@ -910,11 +910,11 @@ int ensure_state(acu_batch* b)
     acu_ctx* c = b->ctx;
     const size_t ni = sizeof(float) * (size_t)b->dev.img_total, ns = sizeof(float) * (size_t)b->dev.sino_total;
     for (DevBuf* x : {&b->f, &b->fk, &b->ruk, &b->rp}) CK(c, x->ensure(ns));
-    CK(c, b->q.ensure(2 * ns));   // exact positions: pairs of bins
     for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->rhs, &b->r, &b->p, &b->Ap, &b->tmp})
         CK(c, x->ensure(ni));
-    CK(c, b->it_img.ensure(4 * ni));   // exact positions: pairs of the images and of their transposes
-    b->dev.IT = b->it_img.as<float>();
+    // one buffer, at exact positions for pairs: the projector's of the images and their transposes, or the filtered bins'
+    CK(c, b->q.ensure(std::max(4 * ni, 2 * ns)));
+    b->dev.IT = b->q.as<float>();
     CK(c, b->part.ensure(sizeof(double) * (size_t)b->dev.n_ew));
     for (DevBuf* x : {&b->rsold, &b->alpha, &b->beta}) CK(c, x->ensure(sizeof(double) * b->nprob));
     return ACU_OK;

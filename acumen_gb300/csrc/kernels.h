@@ -1,5 +1,6 @@
 // Internal launcher declarations shared by the .cu translation units.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -128,12 +129,19 @@ size_t bp_mma_scalars(int G);
 bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
                             cudaStream_t st);
 // The staggered projector for one slice per thread (plain layout); IT is a
-// work buffer of 4 N * N floats per slice (pairs of the image and its transpose).
+// work buffer of N * N floats per slice and no less than pair_image_floats.
 // Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
 // (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
 // the derivative with respect to them or null; launch_backproject_fx: q as pairs
 // (bin, next bin), which the filter writes or launch_pairs makes from
 // n = slices * T * N bins; launch_adjoint_fx: the projector's exact transpose.
+// Their buffers of pairs hold 1 GB at most, as many slices as that takes: slices
+// at once of so many bytes each, and the floats of a projector's buffer.
+inline int pair_slices(size_t bytes, int S)
+{
+    return (int)std::max<size_t>(1, std::min<size_t>(S, ((size_t)1 << 30) / bytes));
+}
+inline size_t pair_image_floats(int N, int S) { return (size_t)4 * N * N * pair_slices((size_t)16 * N * N, S); }
 std::vector<FxAngle> fx_angles(const float* xsc, int T);
 void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);
 void launch_ray_off(const DevGeom<float>& g, int S, const float* img, float* IT, const float* off, float* sino,

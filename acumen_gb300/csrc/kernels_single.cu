@@ -281,24 +281,38 @@ std::vector<FxAngle> fx_angles(const float* xsc, int T)
     return out;
 }
 
+// f(first slice, slices, pairs of their images, pairs of the transposes), the slices' pairs made before
+template <class F>
+static void for_pairs(int N, int S, const float* img, float* buf, cudaStream_t st, F&& f)
+{
+    const size_t NN = (size_t)N * N;
+    const int at_once = pair_slices(16 * NN, S);
+    float2 *const P = reinterpret_cast<float2*>(buf), *const PT = P + NN * at_once;
+    for (int s0 = 0; s0 < S; s0 += at_once) {
+        const int n = std::min(at_once, S - s0);
+        k_pair_images<<<dim3((N + 31) / 32, (N + 31) / 32, n), 256, 0, st>>>(img + s0 * NN, P, PT, N);
+        f(s0, n, P, PT);
+    }
+}
+
 void launch_radon_fx(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st)
 {
-    float2 *P = reinterpret_cast<float2*>(IT), *PT = P + (size_t)g.N * g.N * S;
-    k_pair_images<<<dim3((g.N + 31) / 32, (g.N + 31) / 32, S), 256, 0, st>>>(img, P, PT, g.N);
-    k_ray_fx<<<dim3((g.N + 127) / 128, g.T, S), dim3(32, 4), 0, st>>>(P, PT, g.fx_fp, g.xsc_fp, g.fp_order, sino, g.N,
-                                                                     g.T, g.mid);
+    for_pairs(g.N, S, img, IT, st, [&](int s0, int n, const float2* P, const float2* PT) {
+        k_ray_fx<<<dim3((g.N + 127) / 128, g.T, n), dim3(32, 4), 0, st>>>(
+            P, PT, g.fx_fp, g.xsc_fp, g.fp_order, sino + (size_t)s0 * g.T * g.N, g.N, g.T, g.mid);
+    });
 }
 
 void launch_ray_off(const DevGeom<float>& g, int S, const float* img, float* IT, const float* off, float* sino,
                     float* dsino, cudaStream_t st)
 {
-    float2 *P = reinterpret_cast<float2*>(IT), *PT = P + (size_t)g.N * g.N * S;
-    k_pair_images<<<dim3((g.N + 31) / 32, (g.N + 31) / 32, S), 256, 0, st>>>(img, P, PT, g.N);
-    const dim3 blk(32, 4), grd((g.N + 127) / 128 * g.T, 1, S);
-    if (dsino)
-        k_ray_off<true><<<grd, blk, 0, st>>>(P, PT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
-    else
-        k_ray_off<false><<<grd, blk, 0, st>>>(P, PT, g.sc_fp, g.xsc_fp, g.fp_order, off, sino, dsino, g.N, g.T, g.mid);
+    for_pairs(g.N, S, img, IT, st, [&](int s0, int n, const float2* P, const float2* PT) {
+        const dim3 blk(32, 4), grd((g.N + 127) / 128 * g.T, 1, n);
+        const size_t at = (size_t)s0 * g.T;
+        (dsino ? k_ray_off<true> : k_ray_off<false>)<<<grd, blk, 0, st>>>(
+            P, PT, g.sc_fp, g.xsc_fp, g.fp_order, off ? off + at : nullptr, sino + at * g.N,
+            dsino ? dsino + at * g.N : nullptr, g.N, g.T, g.mid);
+    });
 }
 
 void launch_backproject_fx(const DevGeom<float>& g, int S, const float2* q, float* img, cudaStream_t st)

@@ -111,3 +111,24 @@ def test_ragged_batch_against_single_problems():
             assert np.linalg.norm(i[k] - ref) <= 3e-6 * max(np.linalg.norm(ref), 1e-30)
             t.close()
     b.close()
+
+
+def test_more_slices_than_a_buffer_of_pairs():
+    """One slice per thread by option, more slices than the 1 GB of pairs hold at once (64 of 1025^2): those of the
+    first and the last share are what they are alone."""
+    N, T, S = 1025, 24, 130
+    g = torch.Generator(device="cuda").manual_seed(4)
+    u = torch.rand(S, N, N, device="cuda", generator=g)
+    off = torch.rand(S, T, device="cuda", generator=g) - 0.5
+    t = Tomography(N, syn.angles(T), 50)
+    y = t.radon(u[:2])
+    one = [(t.radon(u[s:s + 1]), t.iradon(y[:1] * (s + 1)), t.backproject(y[:1] * (s + 1)),
+            t.tv_loss_grad(u[s:s + 1], off[s:s + 1], y[:1], 0.1, 1e-3)) for s in (0, 63, 64, S - 1)]
+    yy = y[:1] * torch.arange(1, S + 1, device="cuda")[:, None, None]
+    loss, gu, go = t.tv_loss_grad(u, off, y[:1].expand(S, T, N).contiguous(), 0.1, 1e-3)
+    t.set_option(2, 1)
+    p, r, b = t.radon(u), t.iradon(yy), t.backproject(yy)
+    for k, s in enumerate((0, 63, 64, S - 1)):
+        assert torch.equal(p[s], one[k][0][0]) and torch.equal(r[s], one[k][1][0]) and torch.equal(b[s], one[k][2][0])
+        assert loss[s] == one[k][3][0][0] and torch.equal(gu[s], one[k][3][1][0]) and torch.equal(go[s], one[k][3][2][0])
+    t.close()
