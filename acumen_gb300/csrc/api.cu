@@ -172,15 +172,17 @@ void lanes_filter(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* in, Rea
 }
 
 // Whether G groups are backprojected on the tensor cores (blocks of 64 slices,
-// whatever part of one is filled).  Measured (ms, there / gathers): 725^2 x 360,
-// 32 slices 1.36 / 1.28, 40 slices 1.38 / 1.63; 1025^2 x 600, 36 slices 3.99 /
-// 4.64, 64 slices 4.09 / 8.18; 257^2 x 180, 48 slices 0.18 / 0.19; 129^2 x 90,
-// 128 slices 0.12 / 0.09.
-constexpr int BP_MMA_MIN_GROUPS = 10, BP_MMA_MIN_SIDE = 200;
+// whatever part of one is filled; small sides and few angles leave its launches
+// short).  Measured (ms, there / gathers): 725^2 x 360, 32 slices 1.36 / 1.28, 40
+// slices 1.38 / 1.63; 1025^2 x 600, 36 slices 3.99 / 4.64, 64 slices 4.09 / 8.18; 257^2 x
+// 180, 40 slices 0.16 / 0.13, 48 slices 0.16 / 0.17; 209^2 x 180, 48 slices 0.10 / 0.13;
+// 513^2 x 20, 45 slices 0.096 / 0.084; 129^2 x 90, 128 slices 0.12 / 0.09.
+constexpr int BP_MMA_MIN_SIDE = 200;
+int bp_mma_min_groups(int N, int T) { return N < 800 && T < 60 ? 16 : N < 300 ? 12 : 10; }
 bool bp_mma(const acu_ctx* c, int G)
 {
-    return c->bp_room && c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma && G >= BP_MMA_MIN_GROUPS &&
-           c->N >= BP_MMA_MIN_SIDE;
+    return c->bp_room && c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma &&
+           G >= bp_mma_min_groups(c->N, c->T) && c->N >= BP_MMA_MIN_SIDE;
 }
 
 // Work buffers of the single-precision backprojection of G 4-slice groups (grow-only).
@@ -243,14 +245,19 @@ enum OpKind { OP_IRADON, OP_RADON, OP_RADON_ADJ, OP_FILTER, OP_BACKPROJECT };
 // large batches at exact positions, else the pixel-line projector (6) when the
 // groups fill their 8-group lines to 8/9 or more (its cost follows the lines,
 // the others' the groups), else variant 5.
-constexpr int PROJ_MMA = 8, MMA_MIN_GROUPS = 7, MMA_MIN_SIDE = 200;
+constexpr int PROJ_MMA = 8, MMA_MIN_SIDE = 200;
+// It works on blocks of 64 slices, whatever part of one is filled, and a small
+// side leaves its launches short.  Measured (ms, it / the better gather
+// variant): 1025^2 x 600, 16 slices 9.6 / 6.6, 25 slices 9.6 / 10.2; 513^2 x 360, 25
+// slices 1.81 / 1.85; 450^2 x 360, 25 slices 1.53 / 1.44; 363^2 x 360, 25 slices 1.03 / 0.96, 33 slices 1.03 / 1.1; 257^2 x
+// 180, 32 slices 0.36 / 0.29, 48 slices 0.36 / 0.48; 209^2 x 180, 32 slices 0.31 / 0.24,
+// 48 slices 0.32 / 0.35; at 129^2 it gains nothing at any batch that fits a block.
+int mma_min_groups(int N) { return N >= 500 ? 7 : N >= 250 ? 9 : 12; }
 int projector_variant(const acu_ctx* c, int G)
 {
     if (c->opt_projector != 7) return c->opt_projector;
-    // the tensor-core projector works on blocks of 64 slices, whatever part of one is filled.  Measured (ms, it / the
-    // better gather variant): 1025^2 x 600, 16 slices 9.6 / 6.6, 24 slices 9.6 / 10.0, 64 slices 9.6 / 23.4; 257^2 x
-    // 180, 20 slices 0.29 / 0.26, 32 slices 0.30 / 0.31; at 129^2 it gains nothing at any batch that fits a block
-    if (c->mma_cap > 0 && c->opt_positions == 1 && G >= MMA_MIN_GROUPS && c->N >= MMA_MIN_SIDE && mma_fits(c->N)) return PROJ_MMA;
+    if (c->mma_cap > 0 && c->opt_positions == 1 && G >= mma_min_groups(c->N) && c->N >= MMA_MIN_SIDE && mma_fits(c->N))
+        return PROJ_MMA;
     return 8 * ((G + 7) / 8) <= G + G / 8 ? 6 : 5;
 }
 

@@ -60,7 +60,8 @@ def projector_variant(option, S):
 
 def tensor_projector(option, positions, S, N):
     """Whether the library projects on the tensor cores (csrc/api.cu projector_variant)."""
-    return option == 7 and positions == 1 and (S + 3) // 4 >= 7 and 200 <= N <= 4096
+    groups = 7 if N >= 500 else 9 if N >= 250 else 12
+    return option == 7 and positions == 1 and (S + 3) // 4 >= groups and 200 <= N <= 4096
 
 
 def tensor_radon_launches(N, theta, S, sms=152):
@@ -105,12 +106,13 @@ def tensor_radon_launches(N, theta, S, sms=152):
     return 1 + -(-nblk // nb) * (1 + 2 * len(chunks(ng)))
 
 
-def iradon_launches(positions, S, N):
+def iradon_launches(positions, S, N, T=T_ANG):
     """Kernels of one filtered backprojection: the filter, then the gather
     kernel, or on the tensor cores (csrc/kernels_bp_mma.cu) the largest
     magnitudes, layout and product per pass of up to 128 slices, the tiles
     outside the mask and the flagged fallback."""
-    if positions != 1 or (S + 3) // 4 < 10 or N < 200:
+    groups = 16 if N < 800 and T < 60 else 12 if N < 300 else 10
+    if positions != 1 or (S + 3) // 4 < groups or N < 200:
         return 2
     return 1 + 1 + 2 * -(-S // 128) + 2
 
@@ -832,7 +834,7 @@ def main():
     variant = projector_variant(t.get_option(7), S)
     tensor = tensor_projector(t.get_option(7), t.get_option(8), S, N)
     per_radon = tensor_radon_launches(N, t.theta, S) if tensor else radon_launches(variant, N)
-    per_iradon = iradon_launches(t.get_option(8), S, N)
+    per_iradon = iradon_launches(t.get_option(8), S, N, T)
     kernel_launches = (per_radon * n_radon + per_iradon * n_iradon + n_ew) * args.steps + per_radon * n_full
     if carried_res:   # each refresh: two differences and two backprojections instead of the sum
         kernel_launches += n_full * (2 * per_iradon + 2 - 1)
@@ -943,7 +945,7 @@ def main():
         # the other hot kernel: the backprojection (8 bytes per update at L1 level)
         t_bp = cuda_time(lambda: t.backproject(f), 2)
         line["roofline_backprojection"] = {
-            "kernel": ("k_bp_mma (tensor cores" if iradon_launches(t.get_option(8), S, N) > 2 else
+            "kernel": ("k_bp_mma (tensor cores" if iradon_launches(t.get_option(8), S, N, T) > 2 else
                        "k_backproject_exact_ct<4, 1> (gathers") + "; tv_hpc.F90:107-123)", "launch_ms": 1000 * t_bp,
             "updates_per_s": N * N * T * S / t_bp,
             "l1_level": l1_level(8.0 * N * N * T * S / t_bp / 1e9, clocks, probe, bytes_per_update=8),

@@ -69,8 +69,8 @@ int acu_set_stream(acu_ctx *ctx, void *cuda_stream);
                                  of the previous sample reused, 4 reuse with each warp's steps limited
                                  to those that can meet a valid cell, 5 the same with paired FP32 FMAs
                                  (fma.rn.f32x2), 6 pixel lines of 32 slices walked in bands of rows,
-                                 7 automatic (default): with exact positions, 25 slices or more and a
-                                 side of 200 or more a projector on the tensor cores (the same sums to
+                                 7 automatic (default): with exact positions, 25 slices or more at a
+                                 side from 500 (33 from 250, 45 from 200) a projector on the tensor cores (the same sums to
                                  single-precision rounding; same results on every call), else 6 when
                                  the batch fills its 32-slice lines to 8/9 or more, else 5; 1 and 3 to
                                  6 give identical results */

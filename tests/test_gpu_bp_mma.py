@@ -1,5 +1,5 @@
-"""The backprojection on the tensor cores (automatic from 37 slices and a side of
-200 on, exact positions) against the gather kernel (ACU_OPT_BP_GROUPS = 1) and
+"""The backprojection on the tensor cores (automatic from 37 slices on, more on small
+grids, exact positions) against the gather kernel (ACU_OPT_BP_GROUPS = 1) and
 the FP64 oracle.
 
 Each sums up to 2 T products in single precision in another order and stays
@@ -31,7 +31,7 @@ def both(N, th, q, wpu=None):
 
 # sides around multiples of the 16-pixel tile, one and two blocks of 64 slices and more, angle counts around the four
 # angles of two stages, angles on and near the axes and the diagonals (the widest windows)
-@pytest.mark.parametrize("N, T, S", [(200, 1, 37), (208, 2, 64), (209, 3, 65), (223, 4, 128), (224, 5, 130), (257, 41, 200)])
+@pytest.mark.parametrize("N, T, S", [(200, 1, 61), (800, 3, 37), (208, 2, 64), (209, 3, 65), (223, 4, 128), (224, 5, 130), (257, 41, 200)])
 def test_matches_the_gather_kernel(N, T, S):
     near = [45.0, 0.0, 90.0, 135.0, 180.0, 44.0, 46.5, 89.9999, 90.0001, 1e-5]
     th = np.concatenate([near, syn.angles(T)]).astype(np.float32)[:T]
@@ -56,7 +56,7 @@ def test_against_fp64_and_same_result_twice(oracle, built_lib):
 
 
 def test_scales_of_slices():
-    N, T, S = 209, 30, 40
+    N, T, S = 209, 30, 64
     q = torch.randn(S, T, N, device="cuda")
     q[0] *= 1e30
     q[1] *= 1e-30
@@ -69,7 +69,7 @@ def test_scales_of_slices():
 
 
 def test_values_that_are_not_finite_stay_on_their_pixels():
-    N, T, S = 209, 30, 40
+    N, T, S = 209, 30, 64
     q = torch.randn(S, T, N, device="cuda")
     q[1, 3, 60] = float("nan")
     q[2, 7, 150] = float("inf")
@@ -81,6 +81,6 @@ def test_values_that_are_not_finite_stay_on_their_pixels():
 
 def test_no_tile_meets_the_mask():
     """A margin wider than the grid leaves a mask of zeros."""
-    q = torch.randn(40, 9, 209, device="cuda")
+    q = torch.randn(64, 9, 209, device="cuda")
     got, ref = both(209, syn.angles(9), q, wpu=300)
     assert not got.any() and torch.equal(got, ref)

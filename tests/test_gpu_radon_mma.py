@@ -1,6 +1,6 @@
-"""The projector on the tensor cores (automatic from 25 slices and a side of 200
-on, exact positions) against the gather projector (variant 5) and the FP64
-oracle.
+"""The projector on the tensor cores (exact positions; automatic from 25 slices on
+at sides from 500, from 33 or 45 at smaller ones from 200) against the gather
+projector (variant 5) and the FP64 oracle.
 
 Both round each sum to single precision in another order; a sum of up to 3 N
 terms of one sign stays within ~1e-6 of FP64 either way (the bar of
@@ -37,7 +37,7 @@ def both(N, th, x):
 
 # sides at and around multiples of the 16-pixel tile; slices at the rule's lower end and around blocks of 64 and pairs
 # of them; angle counts that leave a group of five partly filled
-@pytest.mark.parametrize("N, T, S", [(200, 12, 25), (208, 31, 64), (209, 33, 65), (223, 1, 128), (257, 40, 130),
+@pytest.mark.parametrize("N, T, S", [(500, 12, 25), (200, 12, 45), (208, 31, 64), (209, 33, 65), (223, 1, 128), (257, 40, 130),
                                      (224, 13, 200)])
 def test_matches_the_gather_projector(N, T, S):
     g = torch.Generator(device="cuda").manual_seed(N)
@@ -61,7 +61,7 @@ def test_several_chunks_of_angles_and_same_result_twice():
 
 
 def test_against_fp64(oracle, built_lib):
-    N, T, S = 225, 40, 32
+    N, T, S = 225, 40, 48
     th = (syn.angles(T) + 0.21).astype(np.float32)
     x = np.random.default_rng(5).random((S, N, N), dtype=np.float32)
     got, ref = both(N, th, torch.from_numpy(x).cuda())
@@ -71,7 +71,7 @@ def test_against_fp64(oracle, built_lib):
 
 def test_scales_of_slices_and_tiles():
     """Every tile of a slice has its own power-of-two scale: slices and regions of very different magnitude."""
-    N, T, S = 209, 20, 32
+    N, T, S = 209, 20, 48
     x = torch.rand(S, N, N, device="cuda")
     x[0] *= 1e30
     x[1] *= 1e-30
@@ -88,7 +88,7 @@ def test_scales_of_slices_and_tiles():
 
 def test_values_that_are_not_finite_stay_on_their_rays():
     """A matrix product would spread a NaN or infinity over its tile: such a call takes plain gathers."""
-    N, T, S = 209, 20, 32
+    N, T, S = 209, 20, 48
     x = torch.rand(S, N, N, device="cuda")
     x[1, 100, 60] = float("nan")
     x[2, 30, 150] = float("inf")
@@ -101,7 +101,7 @@ def test_values_that_are_not_finite_stay_on_their_rays():
 
 def test_in_the_solver():
     """TV of a batch with the tensor-core projector against the gather projector, through a captured graph."""
-    N, T, S = 209, 60, 32
+    N, T, S = 209, 60, 48
     th = syn.angles(T)
     f = torch.stack([syn.normalised_sinogram(syn.random_ellipses(s, 0.3 * N), N, th, I0=5e3, seed=s, device="cuda")
                      for s in range(S)])
