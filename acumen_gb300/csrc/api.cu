@@ -380,6 +380,20 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     return ACU_OK;
 }
 
+// Whether a small batch is projected by the single-slice kernel: on small grids,
+// where 4-slice groups leave most SMs idle, and with a single slice in the second
+// group.  Measured (ms, 4-slice groups / single slices): 65^2 x 90, 4 slices 0.046 /
+// 0.039; 129^2 x 180, 4 slices 0.069 / 0.048, 16 slices 0.098 / 0.090; 199^2 x 60, 8 slices
+// 0.093 / 0.057; 257^2 x 180, 4 slices 0.111 / 0.092, 8 slices 0.132 / 0.141; 399^2 x 360, 4
+// slices 0.26 / 0.27, 6 slices 0.43 / 0.38; 513^2 x 360, 5 slices 0.61 / 0.51, 6 slices
+// equal; 1449^2 x 900, 5 slices 9.97 / 8.62.
+bool project_single(const acu_ctx* c, int S)
+{
+    if (c->opt_lanes != 0 || c->opt_positions != 1 || c->opt_projector != 7) return false;
+    const int N = c->N;
+    return S <= (N < 200 ? 16 : N < 300 ? 6 : 0) || (S == 5 && N <= FX_MAX_SIDE) || (S == 6 && N < 400);
+}
+
 template <typename Real>
 int run_op(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
 {
@@ -387,7 +401,8 @@ int run_op(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     if (S == 0) return ACU_OK;
     if (!in || !out) return set_err(c, ACU_ERR_INVALID, "null array");
     if constexpr (sizeof(Real) == 4) {
-        if (pick_lanes(c, S, false) == 4) return run_op_v<Real, 4>(c, op, S, in, out);
+        if (pick_lanes(c, S, false) == 4 && !(op == OP_RADON && project_single(c, S)))
+            return run_op_v<Real, 4>(c, op, S, in, out);
     }
     return run_op_v<Real, 1>(c, op, S, in, out);
 }
