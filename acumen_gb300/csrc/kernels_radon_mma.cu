@@ -14,18 +14,25 @@
 // a power-of-two scale (per tile and slice for the image, fixed for W).
 // hi hi + hi lo + lo hi is accumulated; the term left out is 2^-24 of a
 // product.  The tensor core truncates when it adds, so a chain in tensor memory
-// is short: hi hi and the small terms have their own columns, and each half
-// tile its own accumulator (8 steps of K = 16); the rest of every sum is added
-// in FP32 with rounding to nearest.
+// is short: one tile (16 steps of K = 16), hi hi and the small terms in columns of their
+// own; the rest of every sum is added in FP32 with rounding to nearest.
 //
 // Blocks walk stretches of tiles along the rays.  A ray that leaves one tile
 // enters the next, so the rows both tiles met are added to in the L2 cache, by bulk
 // reductions in tile order; only the finished rows of a stretch, a third of
 // what the tiles would write one by one, go to memory and are read back.
+// The order is kept by the four warps that send a block's rows: a ray's place in the
+// operand moves from tile to tile, so two tiles' rows of it may be in the hands of two warps, and
+// a bulk operation is known to have arrived only to the thread that issued it.
+// Twice a tile (each group, where there are few) every warp waits for its own and
+// all four meet before they send on: at the first group those of the tile before
+// but its last two groups have arrived, which covers the first two groups, at the third group
+// all of them.
 //
 // Measured at 2049^2 x 1200 angles, 256 slices: 737 ms with the pixel-line
 // gathers, 217 ms with every tile's rows written and read (75 of them the
-// reduction at 80 % of the HBM bandwidth), now 165 ms, 20 of them the reduction.  1025^2 x
+// reduction at 80 % of the HBM bandwidth), now 168 ms, 20 of them the reduction (the
+// meetings of the warps 1.5 ms).  1025^2 x
 // 600, 128 slices 14.7 / 12.0 ms, 64 slices 9.8 / 9.6 ms (23.4 with gathers).
 // What holds the products is shared memory: 14 KB of operands per K step of one
 // block (20 KB of two, which share W) and the stores of W and of the staged rows
@@ -124,7 +131,7 @@ struct Rows {
 
 struct Shared {
     uint64_t w_full[STAGES], w_empty[STAGES], d_full[4], d_empty[4], img_full[PARTS], img_empty[PARTS], sc_full[2], sc_empty[2],
-        rows_full[4], drained;
+        rows_full[4], sent[2], drained;
     Rows rows[4][SLOTS];   // per accumulator
     uint32_t tmem;
 };
@@ -173,6 +180,7 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
             umma::bar_init(&sh.rows_full[i], 1);
             umma::bar_init(&sh.d_empty[i], 4 * R::OUTS);
         }
+        for (int i = 0; i < R::OUTS; ++i) umma::bar_init(&sh.sent[i], 4);
         umma::bar_init(&sh.drained, 1);
         umma::bar_init_fence();
     }
@@ -381,7 +389,8 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
         constexpr int STAGE_STEP = R::OUTS == 1 ? 32 * HALF * 4 : 0;
         const int lines = nt * stretches, slot0 = (warp & 3) * 32 / PITCH;   // a warp's rows belong to two angles
         const size_t plane = (size_t)lines * rows * HALF;
-        unsigned m = 0, b = 0;
+        constexpr int STEPS = NS / 16;   // 16 columns at a time
+        unsigned m = 0, b = 0, met = 0;
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const Stretch w(u, nt, stretches);
         float* const out = P + ((size_t)(w.block * BLK + k) * 2 * lines + u % lines) * rows * HALF;
@@ -389,6 +398,16 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
             ok = umma::bar_wait_warp(&sh.sc_full[b & 1], (b >> 1) & 1);
             const float4* const scale = reinterpret_cast<const float4*>(sm + L::SCALE + ((b & 1) * BLK + k) * SCALE_BYTES);
             for (int g = 0; g < ngroups; ++g, ++m) {
+                // all that the four warps sent has arrived, of five groups and more but the last two groups' (STEPS / 2 pieces each)
+                const bool meet = ngroups < 5 || g == 0 || g == 2;
+                if (ok && meet) {
+                    if (lane < 4) {
+                        if (ngroups < 5) umma::bulk_store_wait<0>();
+                        else umma::bulk_store_wait<STEPS>();
+                    }
+                    __syncwarp();
+                    if (lane == 0) umma::bar_arrive(&sh.sent[k]);
+                }
                 ok = ok && umma::bar_wait_warp(&sh.rows_full[m % ACCS], (m / ACCS) & 1);
                 if (!ok) break;
                 const Rows to = sh.rows[m % ACCS][slot];
@@ -401,11 +420,14 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                 const int from = mine ? __ffs(mine) - 1 : 0, n_rows = lane < 4 ? __popc(mine) : 0;
                 const int to_row = __shfl_sync(0xffffffffu, prow, from);
                 ok = umma::bar_wait_warp(&sh.d_full[m % ACCS], (m / ACCS) & 1);
+                if (ok && meet) {
+                    ok = umma::bar_wait_warp(&sh.sent[k], met++ & 1);
+                    umma::fence_async_global();
+                }
                 if (!ok) break;
                 umma::fence_after();
                 const uint32_t d = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (m % ACCS) * ACC_COLS + k * NS;
-                // 16 columns at a time (with the next ones on their way meanwhile, in more registers, it took 9 % longer)
-                constexpr int STEPS = NS / 16;
+                // with the next columns on their way meanwhile, in more registers, it took 9 % longer
                 float2 v[8], x[8];
                 auto fetch = [&](int i) {
                     umma::tmem_ld16(d + 16 * i, v);
@@ -421,14 +443,8 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
                         if (lane == 0) umma::bar_arrive(&sh.d_empty[m % ACCS]);
                     }
                     if (i % 2 == 0) {
-                        if (lane < 4) {
-                            // what this group sent of the tile before has arrived: as many pieces ago as there are groups
-                            if (i == 0) {
-                                if (ngroups < 5) umma::bulk_store_wait<0>();
-                                else if (g == 0 || g == 2) umma::bulk_store_wait<STEPS>();
-                            }
-                            umma::bulk_store_wait_read<R::OUTS == 1 ? 1 : 0>();   // the staged rows are on their way out no longer
-                        }
+                        // the staged rows are on their way out no longer
+                        if (lane < 4) umma::bulk_store_wait_read<R::OUTS == 1 ? 1 : 0>();
                         __syncwarp();
                     }
                     if (live) {

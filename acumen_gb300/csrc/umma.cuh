@@ -217,6 +217,8 @@ __device__ __forceinline__ void bulk_store_wait()
 {
     asm volatile("cp.async.bulk.wait_group %0;" ::"n"(PENDING) : "memory");
 }
+// bulk operations on global memory that other threads saw done come before those issued from here on
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 // generic-proxy shared-memory writes become visible to MMAs and bulk copies
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

@@ -135,3 +135,20 @@ def test_little_memory():
         torch.cuda.empty_cache()
         assert rel(got, p) < 3e-6 and rel(back, img) < 3e-6
         t.close()
+
+
+# one to six groups of angles along each axis, one block of 64 slices and pairs of them
+@pytest.mark.parametrize("T", [8, 20, 28, 40, 56])
+@pytest.mark.parametrize("N, S", [(500, 25), (513, 128)])
+def test_rows_that_neighbouring_tiles_share_are_added_in_order(N, T, S):
+    """Four warps send the rows of a block and a ray moves among them from tile to tile: a row that was added before the
+    first tile's value was stored, or in another order, would differ from call to call."""
+    t = Tomography(N, syn.angles(T), 25)
+    x = torch.rand(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T))
+    got = t.radon(x)
+    for _ in range(50):
+        assert torch.equal(got, t.radon(x))
+    t.set_option(7, 5)
+    ref = t.radon(x)
+    assert not torch.equal(got, ref) and rel(got, ref) < 3e-6
+    t.close()
