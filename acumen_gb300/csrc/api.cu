@@ -636,18 +636,21 @@ int tv_iterate_v(acu_ctx* c, int nouter)
     }
     if (!run.carried) s.carried_valid = false;
     if (use_graph) {
-        // the key holds every device address the captured iteration uses
-        // outside the solver state, so a work buffer that has grown since
-        // (another call on a larger batch) forces a new capture
-        char key[560];
-        snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p", (int)sizeof(Real), V,
-                 s.G, s.ninner, s.ncg, s.lambda, s.mu, c->opt_filter, c->opt_projector, c->opt_positions,
-                 c->opt_residual, c->g32.d.bp_tma * 100 + c->g32.d.bp_groups * 10 + c->g32.d.bp_param, s.uk.p, s.part.p, c->pairP.p,
-                 c->pairPT.p, c->lineL.p, c->lineA.p, c->mmaT.p, c->mmaP.p, c->mmaF.p, c->bpQ.p,
-                 c->bpS.p);
-        char key2[640];
-        snprintf(key2, sizeof key2, "%s/%d/%zu/%d", key, c->opt_refresh, c->mma_cap, (int)c->bp_room);
-        if (!s.graph || s.graph_key != key2) {
+        // the key names every allocation the captured iteration uses: a buffer that
+        // has grown since (another call on a larger batch, or on fewer slices, whose
+        // filtered bins take twice the room) forces a new capture
+        char head[256];
+        snprintf(head, sizeof head, "%d/%d/%d/%d/%d/%.17g/%.17g/%d/%d/%d/%d/%d/%d/%zu/%d", (int)sizeof(Real), V, s.G, s.ninner,
+                 s.ncg, s.lambda, s.mu, c->opt_filter, c->opt_projector, c->opt_positions, c->opt_residual,
+                 c->g32.d.bp_tma * 100 + c->g32.d.bp_groups * 10 + c->g32.d.bp_param, c->opt_refresh, c->mma_cap,
+                 (int)c->bp_room);
+        std::string key = head;
+        for (const DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp, &s.q, &s.uk, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap,
+                                &s.tmp, &s.bd, &s.dacc, &s.rsold, &s.alpha, &s.beta, &s.delta, &s.part, &c->pairP, &c->pairPT,
+                                &c->lineL, &c->lineA, &c->mmaT, &c->mmaP, &c->mmaF, &c->bpQ, &c->bpS})
+            key += "/" + std::to_string(b->id);
+        if (!s.graph || s.graph_key != key) {
+            s.graph_key.clear();
             for (cudaGraphExec_t* gx : {&s.graph, &s.graph_inc})
                 if (*gx) {
                     cudaGraphExecDestroy(*gx);
@@ -672,7 +675,7 @@ int tv_iterate_v(acu_ctx* c, int nouter)
                     return set_err(c, ACU_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
                 }
             }
-            s.graph_key = key2;
+            s.graph_key = key;
         }
         for (int jo = 0; jo < nouter; ++jo) {
             const int n = s.outer_done + jo + 1;

@@ -3,7 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <string>
 #include <vector>
@@ -15,9 +17,16 @@ namespace acu {
 
 extern thread_local std::string g_last_error;
 
+inline uint64_t next_allocation()
+{
+    static std::atomic<uint64_t> n{0};
+    return ++n;
+}
+
 struct DevBuf {
     void* p = nullptr;
     size_t n = 0;
+    uint64_t id = 0;   // of this allocation, never used again (an address may be), 0: none
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -27,6 +36,7 @@ struct DevBuf {
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
+        id = 0;
     }
     // grow-only; returns a cudaError_t
     cudaError_t ensure(size_t bytes)
@@ -40,6 +50,7 @@ struct DevBuf {
             return e;
         }
         n = bytes;
+        id = next_allocation();
         return cudaSuccess;
     }
     template <typename T>

@@ -276,3 +276,27 @@ def test_batch_in_chunks_matches_one_batch(prob):
     assert rel(tvh, tv_all) < 1e-5 and rel(fbph, fbp_all) < 1e-6
     with pytest.raises(Exception):
         t.set_option(13, -1)
+
+
+def test_graph_is_captured_anew_when_a_buffer_has_moved(built_lib):
+    """Three slices after four keep the solver's images but need a larger buffer for the filtered bins, so the graph that
+    was captured for four refers to one that is gone."""
+    N, T = 513, 300
+    th = syn.angles(T)
+    f = torch.stack([syn.normalised_sinogram(syn.random_ellipses(s, 0.3 * N), N, th, I0=5e3, seed=s, device="cuda")
+                     for s in range(4)])
+    with Tomography(N, th, 25) as t:
+        ref, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+    for graphs_off in (True, False):
+        t = Tomography(N, th, 25)
+        t.radon(torch.zeros(3, N, N, device="cuda"))       # the projector's buffer at its full size
+        t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+        if graphs_off:
+            t.set_option(3, 0)
+            t.tvopt(f[:3], 1, 1, 1, 0.05, 1.0)
+            t.set_option(3, 1)
+        else:
+            t.tv_begin(f[:3], 1, 1, 0.05, 1.0)             # and no iteration, which would capture its own
+        tv, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+        assert torch.equal(tv, ref)
+        t.close()
