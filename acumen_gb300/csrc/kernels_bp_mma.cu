@@ -18,7 +18,8 @@
 //   k_bp_max      largest magnitude of each slice's filtered sinogram
 //   k_bp_bins     lane sinogram -> bins in operand layout [angle][8 slices, hi then lo][bin][8]
 //   k_bp_mma      the products (tiles that meet the mask)
-//   k_bp_rest     zeros in the other tiles; plain gathers if a value was not finite
+//   k_bp_zero     zeros in the other tiles
+//   k_bp_flagged  plain gathers if a value was not finite, NaN if a wait gave up
 #include <cuda.h>
 
 #include <algorithm>
@@ -87,7 +88,8 @@ __device__ __forceinline__ uint64_t desc(uint32_t addr, uint32_t lbo, uint32_t s
 //   8       issues the products
 //   9       loads the bins (one lane), one box per angle
 //   12..    add the chains up in registers (64 slices of one pixel per lane) and write the tile
-// Waits are bounded; one that gives up sets *err, and the tile is written as NaN.
+// Waits are bounded; one that gives up sets *err, and k_bp_flagged then writes
+// NaN: the block leaves its other tiles as they were.
 template <int BLK>
 __global__ void __launch_bounds__(32 * Bp<BLK>::WARPS, 1) k_bp_mma(const __grid_constant__ CUtensorMap bins,
                                                                    const float4* __restrict__ xsc,
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(32 * Bp<BLK>::WARPS, 1) k_bp_mma(const __grid_
             const int x = (tile % nt) * TP + (p & 15), y = (tile / nt) * TP + (p >> 4);
             if (x < N && y < N) {
                 const size_t NN = (size_t)N * N, pix = (size_t)y * N + x;
-                const float cm = ok ? cmask[pix] : __int_as_float(0x7fc00000);
+                const float cm = cmask[pix];
 #pragma unroll
                 for (int i = 0; i < NS / 4; ++i) {
                     const int g = g0 + k * (NS / 4) + i;
@@ -426,19 +428,20 @@ __global__ void __launch_bounds__(PIX) k_bp_zero(const int* __restrict__ list, f
     for (int g = 0; g < G; ++g) img[((size_t)g * N + y) * N + x] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// The image by plain gathers (as k_backproject_exact), done only if *flag is set.
+// The image by plain gathers (as k_backproject_exact) if flag[0] is set; NaN in all of it if flag[1] is.
 __global__ void __launch_bounds__(256) k_bp_flagged(const float* __restrict__ q, const float* __restrict__ cmask,
                                                     const float4* __restrict__ xsc, float* __restrict__ img, int N,
                                                     int T, int G, float mid, const int* __restrict__ flag)
 {
-    if (*flag == 0) return;
+    if (flag[0] == 0 && flag[1] == 0) return;
+    const bool lost = flag[1] != 0;
     const size_t NN = (size_t)N * N, total = NN * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t g = i / NN, pix = i % NN;
         const float dx = (float)(pix % N + 1) - mid, dy = (float)(pix / N + 1) - mid;
         const float cm = cmask[pix];
         Lanes<float, 4> acc{};
-        if (cm != 0.f) {
+        if (cm != 0.f && !lost) {
             for (int t = 0; t < T; ++t) {
                 const float4 x = __ldg(xsc + t);
                 float cell, wh;
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(256) k_bp_flagged(const float* __restrict__ q,
             }
         }
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc.v[v] *= cm;
+        for (int v = 0; v < 4; ++v) acc.v[v] = lost ? __int_as_float(0x7fc00000) : acc.v[v] * cm;
         st_lanes<float, 4>(img + i * 4, acc);
     }
 }
