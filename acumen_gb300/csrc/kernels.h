@@ -103,7 +103,7 @@ int lines_band_rows(int N);
 std::vector<int> lines_angle_order(const float* sc, int T);
 // Projector on the tensor cores (kernels_radon_mma.cu; exact positions):
 // 64-slice blocks of 16 x 16 pixel tiles in operand layout, partial sums of a
-// chunk of angles, two flags (not finite; a wait gave up).
+// chunk of angles, a flag (a wait gave up) and the slices' largest magnitudes.
 struct MmaPlan {
     int nt = 0;        // tiles per side
     int nblk = 0;      // 64-slice blocks of the batch

@@ -19,7 +19,7 @@
 //   k_bp_bins     lane sinogram -> bins in operand layout [angle][8 slices, hi then lo][bin][8]
 //   k_bp_mma      the products (tiles that meet the mask)
 //   k_bp_zero     zeros in the other tiles
-//   k_bp_flagged  plain gathers if a value was not finite, NaN if a wait gave up
+//   k_bp_flagged  plain gathers of slices with a value that is not finite, NaN if a wait gave up
 #include <cuda.h>
 
 #include <algorithm>
@@ -382,7 +382,7 @@ __device__ __forceinline__ int scale_exp(unsigned top)
 // One bin and angle per thread: its 64 slices of block blockIdx.z as eight pieces of hi and eight of lo halves.
 __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, const unsigned* __restrict__ top,
                                                  float* __restrict__ scale, uint4* __restrict__ bins, int N, int T,
-                                                 int G, int g0, int* flag)
+                                                 int G, int g0)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y, k = blockIdx.z;
     if (i >= N) return;
@@ -401,7 +401,6 @@ __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, c
                 if (i == 0 && t == 0) {
                     auto inv = [](unsigned b) { return __int_as_float((scale_exp(b) - 14 + 127) << 23); };
                     reinterpret_cast<float4*>(scale)[g] = make_float4(inv(m.x), inv(m.y), inv(m.z), inv(m.w));
-                    if (max(max(m.x, m.y), max(m.z, m.w)) >= 0x7f800000u) atomicOr(flag, 1);
                 }
             }
             const float f[4] = {v.x, v.y, v.z, v.w};
@@ -428,36 +427,46 @@ __global__ void __launch_bounds__(PIX) k_bp_zero(const int* __restrict__ list, f
     for (int g = 0; g < G; ++g) img[((size_t)g * N + y) * N + x] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// The image by plain gathers (as k_backproject_exact) if flag[0] is set; NaN in all of it if flag[1] is.
+// The slices that held a value that is not finite by plain gathers (as k_backproject_exact): a slice is a column of the
+// product, which spreads such a value over its tiles and no further (one such slice of 256 at
+// 2049^2 x 1200: 8 ms, after 81).  NaN in all of the image if a wait gave up.
 __global__ void __launch_bounds__(256) k_bp_flagged(const float* __restrict__ q, const float* __restrict__ cmask,
                                                     const float4* __restrict__ xsc, float* __restrict__ img, int N,
-                                                    int T, int G, float mid, const int* __restrict__ flag)
+                                                    int T, int G, float mid, const unsigned* __restrict__ top,
+                                                    const int* __restrict__ err)
 {
-    if (flag[0] == 0 && flag[1] == 0) return;
-    const bool lost = flag[1] != 0;
-    const size_t NN = (size_t)N * N, total = NN * G;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t g = i / NN, pix = i % NN;
-        const float dx = (float)(pix % N + 1) - mid, dy = (float)(pix / N + 1) - mid;
-        const float cm = cmask[pix];
-        Lanes<float, 4> acc{};
-        if (cm != 0.f && !lost) {
-            for (int t = 0; t < T; ++t) {
-                const float4 x = __ldg(xsc + t);
-                float cell, wh;
-                exact_coord(x.x, x.y, x.z, x.w, dx, dy, mid, cell, wh);
-                const int y1 = (int)cell;
-                if (y1 > 1 && y1 < N) {
-                    const float* row = q + ((g * T + t) * N + (y1 - 1)) * 4;
-                    const Lanes<float, 4> a = ld_lanes<float, 4>(row), b = ld_lanes<float, 4>(row + 4);
+    const bool lost = *err != 0;
+    bool any = lost;
+    for (int i = threadIdx.x; i < 4 * G; i += 256) any |= top[i] >= 0x7f800000u;
+    if (!__syncthreads_or(any)) return;
+    const size_t NN = (size_t)N * N;
+    for (size_t g = 0; g < G; ++g) {
+        const uint4 m = __ldg(reinterpret_cast<const uint4*>(top) + g);
+        const bool marked[4] = {lost || m.x >= 0x7f800000u, lost || m.y >= 0x7f800000u, lost || m.z >= 0x7f800000u,
+                                lost || m.w >= 0x7f800000u};
+        if (!(marked[0] || marked[1] || marked[2] || marked[3])) continue;
+        for (size_t pix = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pix < NN; pix += (size_t)gridDim.x * blockDim.x) {
+            const float dx = (float)(pix % N + 1) - mid, dy = (float)(pix / N + 1) - mid;
+            const float cm = cmask[pix];
+            Lanes<float, 4> acc{};
+            if (cm != 0.f && !lost) {
+                for (int t = 0; t < T; ++t) {
+                    const float4 x = __ldg(xsc + t);
+                    float cell, wh;
+                    exact_coord(x.x, x.y, x.z, x.w, dx, dy, mid, cell, wh);
+                    const int y1 = (int)cell;
+                    if (y1 > 1 && y1 < N) {
+                        const float* row = q + ((g * T + t) * N + (y1 - 1)) * 4;
+                        const Lanes<float, 4> a = ld_lanes<float, 4>(row), b = ld_lanes<float, 4>(row + 4);
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) acc.v[v] = fmaf(b.v[v], wh, fmaf(a.v[v], 1.f - wh, acc.v[v]));
+                        for (int v = 0; v < 4; ++v) acc.v[v] = fmaf(b.v[v], wh, fmaf(a.v[v], 1.f - wh, acc.v[v]));
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc.v[v] = lost ? __int_as_float(0x7fc00000) : acc.v[v] * cm;
-        st_lanes<float, 4>(img + i * 4, acc);
+            for (int v = 0; v < 4; ++v)
+                if (marked[v]) img[(g * NN + pix) * 4 + v] = lost ? __int_as_float(0x7fc00000) : acc.v[v] * cm;
+        }
     }
 }
 
@@ -485,16 +494,16 @@ bool bins_map(CUtensorMap* map, void* bins, int N, int T, int chunks)
 
 template <int BLK>
 bool bp_pass(const DevGeom<float>& g, int G, int g0, const float* q, void* bins, unsigned* top, float* scale,
-             float* img, int* flags, int sms, cudaStream_t st)
+             float* img, int* err, int sms, cudaStream_t st)
 {
     CUtensorMap map;
     if (!bins_map(&map, bins, g.N, g.T, Bp<BLK>::CHUNKS)) return false;
     const int nt = (g.N + TP - 1) / TP;
     k_bp_bins<<<dim3((g.N + 127) / 128, g.T, BLK), 128, 0, st>>>(reinterpret_cast<const float4*>(q), top, scale,
-                                                                reinterpret_cast<uint4*>(bins), g.N, g.T, G, g0, flags);
+                                                                reinterpret_cast<uint4*>(bins), g.N, g.T, G, g0);
     max_dynamic_smem<k_bp_mma<BLK>>();
     k_bp_mma<BLK><<<std::min(sms, g.n_tiles_in), 32 * Bp<BLK>::WARPS, Bp<BLK>::BARS + sizeof(Shared), st>>>(
-        map, g.xsc_bp, g.tiles_in, g.n_tiles_in, g.cmask, scale, img, g.N, g.T, nt, G, g0, g.mid, flags + 1);
+        map, g.xsc_bp, g.tiles_in, g.n_tiles_in, g.cmask, scale, img, g.N, g.T, nt, G, g0, g.mid, err);
     return true;
 }
 
@@ -532,22 +541,22 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     unsigned* top = scalars;
     float* scale = reinterpret_cast<float*>(scalars + 4 * (size_t)G);
-    int* flags = reinterpret_cast<int*>(scalars + 8 * (size_t)G);   // [0] not finite, [1] a wait gave up
+    int* err = reinterpret_cast<int*>(scalars + 8 * (size_t)G);   // a wait gave up
     cudaMemsetAsync(scalars, 0, bp_mma_scalars(G) * sizeof(unsigned), st);
     k_bp_max<<<dim3((unsigned)std::min<size_t>((npos + 1023) / 1024, 512), G), 256, 0, st>>>(
         reinterpret_cast<const float4*>(q), top, npos);
     if (g.n_tiles_in > 0)
         for (int g0 = 0; g0 < G;) {
             const bool two = G - g0 > NS / 4;
-            if (!(two ? bp_pass<2>(g, G, g0, q, bins, top, scale, img, flags, sms, st)
-                      : bp_pass<1>(g, G, g0, q, bins, top, scale, img, flags, sms, st)))
+            if (!(two ? bp_pass<2>(g, G, g0, q, bins, top, scale, img, err, sms, st)
+                      : bp_pass<1>(g, G, g0, q, bins, top, scale, img, err, sms, st)))
                 return false;
             g0 += (two ? 2 : 1) * (NS / 4);
         }
     const int nt = (g.N + TP - 1) / TP, rest = nt * nt - g.n_tiles_in;
     if (rest > 0)
         k_bp_zero<<<rest, PIX, 0, st>>>(g.tiles_in + g.n_tiles_in, reinterpret_cast<float4*>(img), g.N, nt, G);
-    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, flags);
+    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, top, err);
     return true;
 }
 

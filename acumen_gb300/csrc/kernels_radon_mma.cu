@@ -42,9 +42,8 @@
 //   k_mma_project   tiles -> partial sums P[block][half][stretch][row][32 slices]
 //   k_mma_reduce    P -> sinogram: a ray's partial sums in the order of the
 //                   stretches (fixed, so results do not depend on the schedule)
-//   k_radon_flagged the sinogram by plain gathers if the image held a value that
-//                   is not finite (a matrix product would spread it), or of slices
-//                   of subnormal magnitude
+//   k_radon_flagged by plain gathers the slices that held a value that is not
+//                   finite, and those of subnormal magnitude
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -555,9 +554,9 @@ __global__ void __launch_bounds__(256) k_mma_reduce(const float* __restrict__ P,
 // ([pixel / 8][hi: 64 slices, lo: 64 slices][pixel % 8], of two blocks 128 slices
 // each), then the factors that undo the scales of image and weights.
 __global__ void __launch_bounds__(256) k_mma_tiles(const float4* __restrict__ img, unsigned char* __restrict__ tiles,
-                                                   int N, int nt, int G, int g0, int blk, int* flag)
+                                                   int N, int nt, int G, int g0, int blk, unsigned* top)
 {
-    unsigned* const top = reinterpret_cast<unsigned*>(flag) + 2 + g0 * 4 + blockIdx.y * NS;   // per slice
+    top += g0 * 4 + blockIdx.y * NS;   // the slices' largest magnitudes
     extern __shared__ __align__(16) float s_v[];   // [64][260], then 64 scales
     constexpr int LD = TP * TP + 4;
     float* const s_scale = s_v + NS * LD;
@@ -584,11 +583,8 @@ __global__ void __launch_bounds__(256) k_mma_tiles(const float4* __restrict__ im
         for (int k = 0; k < TP * TP; k += 32) m = max(m, __float_as_uint(s_v[n * LD + k + lane]) & 0x7fffffffu);
         m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0) {
-            if (m >= 0x7f800000u) {
-                atomicOr(flag, 1);
-                m = 0;
-            }
             if (m > top[n]) atomicMax(top + n, m);
+            if (m >= 0x7f800000u) m = 0;
             const int e = m ? max((int)(m >> 23) - 127, -98) : 0;
             s_scale[n] = __int_as_float((14 - e + 127) << 23);
             reinterpret_cast<float*>(out + blk * TILE_OP)[kb * NS + n] = __int_as_float((e - 14 + 127) << 23);
@@ -611,47 +607,69 @@ __global__ void __launch_bounds__(256) k_mma_tiles(const float4* __restrict__ im
     }
 }
 
-// The projection by plain gathers (as k_radon): of all slices if *flag is set, else of the groups with a slice whose
-// values are all below 2^-80 (partial sums in subnormals would be lost).
+// Slices by plain gathers (as k_radon): those that held a value that is not finite (a slice is a column of the product,
+// which spreads such a value over its tiles and no further), and those whose values are all below 2^-80 (partial sums in
+// subnormals would be lost).  Held by the L1 data path; one such slice of 256 at 2049^2 x 1200: 17 ms (168 / 185 ms the
+// projection), 23 ms with eight steps of a ray side by side at all angles.
 __global__ void __launch_bounds__(128) k_radon_flagged(const float* __restrict__ img, const float* __restrict__ sc,
                                                        const float4* __restrict__ xsc, float* __restrict__ sino, int N,
-                                                       int T, int G, float mid, const int* __restrict__ flag)
+                                                       int T, int G, float mid, const unsigned* __restrict__ top)
 {
-    const unsigned* const top = reinterpret_cast<const unsigned*>(flag) + 2;
-    auto wanted = [&](int g) {
-        bool w = *flag != 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w |= top[4 * g + i] - 1u < 0x17800000u - 1u;   // 2^-80
-        return w;
-    };
+    auto marked = [&](int s) { return top[s] >= 0x7f800000u || top[s] - 1u < 0x17800000u - 1u; };   // 2^-80
     bool any = false;
-    for (int i = threadIdx.x; i < G; i += 128) any |= wanted(i);
+    for (int i = threadIdx.x; i < 4 * G; i += 128) any |= marked(i);
     if (!__syncthreads_or(any)) return;
-    const int nb = (N + 127) / 128;
-    for (size_t g = 0; g < G; ++g)
-    for (long long it = wanted((int)g) ? blockIdx.x : (long long)nb * T; it < (long long)nb * T; it += gridDim.x) {
-        const int jy = (int)(it % nb) * 128 + threadIdx.x + 1, t = (int)(it / nb);
-        if (jy > N) continue;
-        const ProjRay<float, true> ray(sc, xsc, t, jy, mid, nullptr);
-        const float* u = img + g * N * N * 4;
-        Lanes<float, 4> acc{};
-        for (int jx = 1; jx <= N; ++jx) {
-            int x1, y1;
-            float wxl, wxh, wyl, wyh;
-            ray.at((float)jx - mid, x1, y1, wxl, wxh, wyl, wyh);
-            if (min(x1, y1) > 1 && max(x1, y1) < N) {
-                const float w11 = wxl * wyl, w21 = wxh * wyl, w12 = wxl * wyh, w22 = wxh * wyh;
-                const float* p = u + ((size_t)(y1 - 1) * N + (x1 - 1)) * 4;
-                const Lanes<float, 4> a = ld_lanes<float, 4>(p), b = ld_lanes<float, 4>(p + 4);
-                const Lanes<float, 4> cc = ld_lanes<float, 4>(p + (size_t)N * 4), d = ld_lanes<float, 4>(p + (size_t)N * 4 + 4);
+    const int nb = (N + 127) / 128, lane = threadIdx.x & 31;
+    for (size_t g = 0; g < G; ++g) {
+    bool m[4];
 #pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    acc.v[v] = fmaf(d.v[v], w22, fmaf(cc.v[v], w12, fmaf(b.v[v], w21, fmaf(a.v[v], w11, acc.v[v]))));
+    for (int v = 0; v < 4; ++v) m[v] = marked((int)g * 4 + v);
+    if (!(m[0] || m[1] || m[2] || m[3])) continue;
+    // eight neighbouring lanes read pixels of the same row or of few: they take eight steps of a ray, or with steeper rays
+    // neighbouring ones, staggered so that a step of theirs stays in a row
+    for (long long it = blockIdx.x; it < (long long)nb * T; it += gridDim.x) {
+        const int t = (int)(it / nb);
+        const float s = sc[2 * t], c = sc[2 * t + 1];
+        const int ns = fabsf(s) < 0.3f ? 8 : 1, kb = ns == 1 ? __float2int_rn((float)lane * (c / s)) : 0;
+        for (int i = 0; i < 32; i += 32 / ns) {
+            const int jy = (int)(it % nb) * 128 + (threadIdx.x & ~31) + 1 + i + lane / ns;
+            const ProjRay<float, true> ray(sc, xsc, t, jy, mid, nullptr);
+            const float* u = img + g * N * N * 4;
+            int lo, hi;
+            valid_steps(s, c, (float)jy - mid, mid, N, lo, hi);
+            if (jy > N || lo > hi) {
+                lo = 0x3fffffff;
+                hi = -0x3fffffff;
             }
-        }
+            const int from = ns == 1 ? __reduce_min_sync(0xffffffffu, lo + kb) : lo + lane % ns;
+            const int to = ns == 1 ? __reduce_max_sync(0xffffffffu, hi + kb) : hi;
+            Lanes<float, 4> acc{};
+#pragma unroll 2
+            for (int k = from; k <= to; k += ns) {
+                const int jx = k - kb;
+                if (jx < lo || jx > hi) continue;
+                int x1, y1;
+                float wxl, wxh, wyl, wyh;
+                ray.at((float)jx - mid, x1, y1, wxl, wxh, wyl, wyh);
+                if (min(x1, y1) > 1 && max(x1, y1) < N) {
+                    const float w11 = wxl * wyl, w21 = wxh * wyl, w12 = wxl * wyh, w22 = wxh * wyh;
+                    const float* p = u + ((size_t)(y1 - 1) * N + (x1 - 1)) * 4;
+                    const Lanes<float, 4> a = ld_lanes<float, 4>(p), b = ld_lanes<float, 4>(p + 4);
+                    const Lanes<float, 4> cc = ld_lanes<float, 4>(p + (size_t)N * 4), d = ld_lanes<float, 4>(p + (size_t)N * 4 + 4);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc.v[v] = acc.v[v] / (float)N;
-        st_lanes<float, 4>(sino + ((g * T + t) * N + (jy - 1)) * 4, acc);
+                    for (int v = 0; v < 4; ++v)
+                        acc.v[v] = fmaf(d.v[v], w22, fmaf(cc.v[v], w12, fmaf(b.v[v], w21, fmaf(a.v[v], w11, acc.v[v]))));
+                }
+            }
+            for (int o = ns / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc.v[v] += __shfl_xor_sync(0xffffffffu, acc.v[v], o);
+            if (lane % ns > 0 || jy > N) continue;
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if (m[v]) sino[((g * T + t) * N + (jy - 1)) * 4 + v] = acc.v[v] / (float)N;
+        }
+    }
     }
 }
 
@@ -769,7 +787,7 @@ MmaPlan mma_plan(const DevGeom<float>& g, int G, size_t cap)
     return p;
 }
 
-size_t mma_flag_words(int G) { return 2 + (size_t)(G * 4 + NS - 1) / NS * NS; }
+size_t mma_flag_words(int G) { return 1 + (size_t)(G * 4 + NS - 1) / NS * NS; }
 
 // Sides whose five-angle chunks of partial sums exceed the cap keep the gather kernels.
 bool mma_fits(int N)
@@ -785,12 +803,13 @@ void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned
     max_dynamic_smem<k_mma_tiles>();
     max_dynamic_smem<k_mma_project<1>>();
     max_dynamic_smem<k_mma_project<2>>();
-    // [0] not finite, [1] a wait gave up, then the slices' largest magnitudes
+    // [0] a wait gave up, then the slices' largest magnitudes
+    unsigned* const top = reinterpret_cast<unsigned*>(flags) + 1;
     cudaMemsetAsync(flags, 0, sizeof(int) * mma_flag_words(G), st);
     for (int b = 0; b < p.nblk; b += p.nb) {
         const int nb = std::min(p.nb, p.nblk - b);
         k_mma_tiles<<<dim3(nt2, nb), 256, NS * (TP * TP + 5) * sizeof(float), st>>>(
-            reinterpret_cast<const float4*>(img), tiles, N, p.nt, G, b * (NS / 4), nb % 2 == 0 ? 2 : 1, flags);
+            reinterpret_cast<const float4*>(img), tiles, N, p.nt, G, b * (NS / 4), nb % 2 == 0 ? 2 : 1, top);
         for (int x = 0; x < 2; ++x) {
             const int first = x ? g.n_groups_x : 0, last = x ? g.n_groups : g.n_groups_x;
             for (int ga = first, gb; ga < last; ga = gb) {
@@ -803,13 +822,13 @@ void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned
                     std::min(g.sms, units), 32 * (blk == 2 ? Roles<2>::WARPS : Roles<1>::WARPS),
                     (blk == 2 ? Smem<2>::BARS : Smem<1>::BARS) + sizeof(Shared), st>>>(
                     tiles, P, g.mma, g.groups + ga, N, p.nt, g.stretches, x == 0, units, gb - ga, row0, rows, g.mid,
-                    flags + 1);
+                    flags);
                 k_mma_reduce<<<dim3((N + 63) / 64, t1 - t0, nb), 256, 0, st>>>(
-                    P, sino, g.mma, N, T, p.nt, g.stretches, G, b * (NS / 4), t0, row0, rows, g.mid, flags + 1);
+                    P, sino, g.mma, N, T, p.nt, g.stretches, G, b * (NS / 4), t0, row0, rows, g.mid, flags);
             }
         }
     }
-    k_radon_flagged<<<g.sms * 8, 128, 0, st>>>(img, g.sc_fp, g.xsc_fp, sino, N, T, G, g.mid, flags);
+    k_radon_flagged<<<g.sms * 8, 128, 0, st>>>(img, g.sc_fp, g.xsc_fp, sino, N, T, G, g.mid, top);
 }
 
 }  // namespace acu

@@ -84,3 +84,22 @@ def test_no_tile_meets_the_mask():
     q = torch.randn(64, 9, 209, device="cuda")
     got, ref = both(209, syn.angles(9), q, wpu=300)
     assert not got.any() and torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("S", [64, 130])
+def test_a_value_that_is_not_finite_changes_no_other_slice(S):
+    N, T = 209, 30
+    q = torch.randn(S, T, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(S))
+    bad = [5, 44]
+    y = q.clone()
+    y[5, 3, 60] = float("nan")
+    y[44, 7, 150] = float("inf")
+    t = Tomography(N, syn.angles(T), 10)
+    clean, got = t.backproject(q), t.backproject(y)
+    others = [s for s in range(S) if s not in bad]
+    assert torch.equal(got[others], clean[others])
+    t.set_option(10, 1)
+    ref = t.backproject(y)[bad]
+    got, m = got[bad], torch.isfinite(ref)
+    assert not m.all() and m.any() and torch.equal(torch.isfinite(got), m) and rel(got[m], ref[m]) < 2e-6
+    t.close()

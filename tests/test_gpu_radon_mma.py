@@ -152,3 +152,23 @@ def test_rows_that_neighbouring_tiles_share_are_added_in_order(N, T, S):
     ref = t.radon(x)
     assert not torch.equal(got, ref) and rel(got, ref) < 3e-6
     t.close()
+
+
+@pytest.mark.parametrize("S", [48, 130])
+def test_a_value_that_is_not_finite_changes_no_other_slice(S):
+    N, T = 209, 20
+    x = torch.rand(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(S))
+    bad = [5, 44]
+    y = x.clone()
+    y[5, 100, 60] = float("nan")
+    y[44, 30, 150] = float("inf")
+    t = Tomography(N, axes(T), 10)
+    clean, got = t.radon(x), t.radon(y)
+    others = [s for s in range(S) if s not in bad]
+    assert torch.equal(got[others], clean[others])
+    assert got[5].isnan().any() and not got[5].isnan().all() and not got[44].isfinite().all()
+    t.set_option(7, 5)
+    ref = t.radon(y)[bad]
+    got, m = got[bad], torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(got), m) and rel(got[m], ref[m]) < 3e-6
+    t.close()
