@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <string>
 #include <vector>
@@ -161,6 +162,29 @@ int pick_lanes(const acu_ctx* c, int S, bool is_double)
     return S >= 4 ? 4 : 1;
 }
 
+// Device memory that a call cannot do without (grow-only).  Where there is none left,
+// the work buffers of the tensor-core operators are given back for it, of which
+// the gathers need none: they are asked for after this, call by call.
+int need(acu_ctx* c, DevBuf& b, size_t bytes)
+{
+    cudaError_t e = b.ensure(bytes);
+    if (e == cudaErrorMemoryAllocation && c->mmaT.n + c->mmaP.n + c->bpQ.n > 0) {
+        cudaGetLastError();
+        for (DevBuf* o : {&c->mmaT, &c->mmaP, &c->bpQ}) o->release();
+        e = b.ensure(bytes);
+    }
+    CK(c, e);
+    return ACU_OK;
+}
+
+// Whether so many more bytes than the buffers hold can be had.
+bool room_for(size_t bytes, std::initializer_list<const DevBuf*> held)
+{
+    size_t freeb = 0, totalb = 0, have = 0;
+    for (const DevBuf* b : held) have += b->n;
+    return cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && bytes <= freeb + have;
+}
+
 // ---- operators in lane layout ---------------------------------------------
 template <typename Real, int V>
 void lanes_filter(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* in, Real* out)
@@ -179,24 +203,29 @@ void lanes_filter(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* in, Rea
 // 513^2 x 20, 45 slices 0.096 / 0.084; 129^2 x 90, 128 slices 0.12 / 0.09.
 constexpr int BP_MMA_MIN_SIDE = 200;
 int bp_mma_min_groups(int N, int T) { return N < 800 && T < 60 ? 16 : N < 300 ? 12 : 10; }
-bool bp_mma(const acu_ctx* c, int G)
+bool bp_mma_wanted(const acu_ctx* c, int G)
 {
-    return c->bp_room && c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma &&
+    return c->opt_positions == 1 && c->g32.d.bp_groups == 0 && !c->g32.d.bp_tma &&
            G >= bp_mma_min_groups(c->N, c->T) && c->N >= BP_MMA_MIN_SIDE;
 }
+bool bp_mma(const acu_ctx* c, int G) { return c->bp_room && bp_mma_wanted(c, G); }
 
-// Work buffers of the single-precision backprojection of G 4-slice groups (grow-only).
+// Work buffers of the single-precision backprojection of G 4-slice groups
+// (grow-only), after all else that the call needs.
 int ensure_backproject_buffers(acu_ctx* c, int G)
 {
-    if (!bp_mma(c, G)) return ACU_OK;
-    const cudaError_t e = c->bpQ.ensure(bp_mma_bins_bytes(c->N, c->T, G));
+    if (!bp_mma_wanted(c, G)) return ACU_OK;
+    const size_t bytes = bp_mma_bins_bytes(c->N, c->T, G);
+    if (!c->bp_room && !room_for(bytes, {&c->bpQ})) return ACU_OK;
+    cudaError_t e = c->bpQ.ensure(bytes);
+    if (e == cudaSuccess) e = c->bpS.ensure(sizeof(unsigned) * bp_mma_scalars(G));
+    c->bp_room = e == cudaSuccess;
     if (e == cudaErrorMemoryAllocation) {   // the gathers need no buffer
         cudaGetLastError();
-        c->bp_room = false;
+        c->bpQ.release();
         return ACU_OK;
     }
     CK(c, e);
-    CK(c, c->bpS.ensure(sizeof(unsigned) * bp_mma_scalars(G)));
     return ACU_OK;
 }
 
@@ -253,40 +282,61 @@ constexpr int PROJ_MMA = 8, MMA_MIN_SIDE = 200;
 // 180, 32 slices 0.36 / 0.29, 48 slices 0.36 / 0.48; 209^2 x 180, 32 slices 0.31 / 0.24,
 // 48 slices 0.32 / 0.35; at 129^2 it gains nothing at any batch that fits a block.
 int mma_min_groups(int N) { return N >= 500 ? 7 : N >= 250 ? 9 : 12; }
+bool mma_wanted(const acu_ctx* c, int G)
+{
+    return c->opt_projector == 7 && c->opt_positions == 1 && G >= mma_min_groups(c->N) && c->N >= MMA_MIN_SIDE && mma_fits(c->N);
+}
 int projector_variant(const acu_ctx* c, int G)
 {
     if (c->opt_projector != 7) return c->opt_projector;
-    if (c->mma_cap > 0 && c->opt_positions == 1 && G >= mma_min_groups(c->N) && c->N >= MMA_MIN_SIDE && mma_fits(c->N))
-        return PROJ_MMA;
+    if (c->mma_cap > 0 && mma_wanted(c, G)) return PROJ_MMA;
     return 8 * ((G + 7) / 8) <= G + G / 8 ? 6 : 5;
 }
 
+// Work buffers of the tensor-core projector.  Where memory is short it takes the
+// angles in smaller chunks, down to an eighth of the plan's partial sums (each
+// chunk reads the tiles again), else mma_cap is 0 and the gathers do without; it is whole
+// again when there is room for it.
+int ensure_mma_buffers(acu_ctx* c, int G)
+{
+    const DevGeom<float>& g = c->g32.d;
+    const MmaPlan whole = mma_plan(g, G, MMA_PART_CAP);
+    if (c->mma_cap == MMA_PART_CAP || room_for(whole.tile_bytes + whole.part_bytes, {&c->mmaT, &c->mmaP}))
+        c->mma_cap = MMA_PART_CAP;
+    while (c->mma_cap > 0) {
+        const MmaPlan p = c->mma_cap == MMA_PART_CAP ? whole : mma_plan(g, G, c->mma_cap);
+        cudaError_t e = c->mmaT.ensure(p.tile_bytes);
+        if (e == cudaSuccess) e = c->mmaP.ensure(p.part_bytes);
+        if (e == cudaSuccess) e = c->mmaF.ensure(sizeof(int) * mma_flag_words(G));
+        if (e != cudaErrorMemoryAllocation) {
+            CK(c, e);
+            break;
+        }
+        cudaGetLastError();
+        c->mmaT.release();
+        c->mmaP.release();
+        c->mma_cap = p.part_bytes / 2;
+        if (c->mma_cap < whole.part_bytes / 8 || mma_plan(g, G, c->mma_cap).part_bytes == p.part_bytes) c->mma_cap = 0;
+    }
+    return ACU_OK;
+}
+
 // Work buffers of the single-precision 4-slice projector that
-// ACU_OPT_PROJECTOR selects, for G slice groups (grow-only).
+// ACU_OPT_PROJECTOR selects, for G slice groups (grow-only), after all else that the
+// call needs but the backprojection's.
 int ensure_projector_buffers(acu_ctx* c, int G)
 {
     const size_t nimg = (size_t)c->N * c->N * G * 4;
+    if (mma_wanted(c, G)) CKRET(ensure_mma_buffers(c, G));
     const int v = projector_variant(c, G);
     if (v == 0) {
-        CK(c, c->pairP.ensure(sizeof(float) * 2 * nimg));
-        CK(c, c->pairPT.ensure(sizeof(float) * 2 * nimg));
-    } else if (v == PROJ_MMA) {
-        const MmaPlan p = mma_plan(c->g32.d, G, c->mma_cap);
-        cudaError_t e = c->mmaT.ensure(p.tile_bytes);
-        if (e == cudaSuccess) e = c->mmaP.ensure(p.part_bytes);
-        if (e == cudaErrorMemoryAllocation) {   // smaller chunks, then the gathers
-            cudaGetLastError();
-            c->mmaT.release();
-            c->mma_cap = c->mma_cap > ((size_t)1 << 30) ? c->mma_cap / 2 : 0;
-            return ensure_projector_buffers(c, G);
-        }
-        CK(c, e);
-        CK(c, c->mmaF.ensure(sizeof(int) * mma_flag_words(G)));
+        CKRET(need(c, c->pairP, sizeof(float) * 2 * nimg));
+        CKRET(need(c, c->pairPT, sizeof(float) * 2 * nimg));
     } else if (v == 6) {
-        CK(c, c->lineL.ensure(sizeof(float) * lines_image_floats(c->N, G)));
-        CK(c, c->lineA.ensure(sizeof(float) * lines_sums_floats(c->N, c->T, G)));
-    } else {
-        CK(c, c->pairPT.ensure(sizeof(float) * nimg));
+        CKRET(need(c, c->lineL, sizeof(float) * lines_image_floats(c->N, G)));
+        CKRET(need(c, c->lineA, sizeof(float) * lines_sums_floats(c->N, c->T, G)));
+    } else if (v != PROJ_MMA) {
+        CKRET(need(c, c->pairPT, sizeof(float) * nimg));
     }
     return ACU_OK;
 }
@@ -321,16 +371,16 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     const Real* lin = in;
     Real* lout = out;
     if constexpr (V > 1) {
-        CK(c, c->w_in.ensure(sizeof(Real) * nin * G * V));
-        CK(c, c->w_out.ensure(sizeof(Real) * nout * G * V));
+        CKRET(need(c, c->w_in, sizeof(Real) * nin * G * V));
+        CKRET(need(c, c->w_out, sizeof(Real) * nout * G * V));
         launch_to_lanes<Real, V>(in, c->w_in.template as<Real>(), S, nin, c->stream);
         lin = c->w_in.template as<Real>();
         lout = c->w_out.template as<Real>();
     }
     switch (op) {
     case OP_IRADON:
+        CKRET(need(c, c->w_q, sizeof(Real) * q_size<Real, V>(nsino, G)));
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
-        CK(c, c->w_q.ensure(sizeof(Real) * q_size<Real, V>(nsino, G)));
         lanes_iradon<Real, V>(c, g, G, lin, c->w_q.template as<Real>(), lout);
         break;
     case OP_RADON:
@@ -338,7 +388,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
             CKRET(ensure_projector_buffers(c, G));
             radon_quads(c, g, G, lin, lout);
         } else if constexpr (V == 1 && sizeof(Real) == 4) {
-            CK(c, c->pairPT.ensure(sizeof(float) * std::max(nimg * G, pair_image_floats(N, G))));
+            CKRET(need(c, c->pairPT, sizeof(float) * std::max(nimg * G, pair_image_floats(N, G))));
             launch_radon_v1_fast(g, G, lin, c->pairPT.template as<float>(), lout, c->stream);
         } else {
             launch_radon<Real, V>(g, G, lin, lout, c->stream);
@@ -359,7 +409,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
         if constexpr (V == 1 && sizeof(Real) == 4) {
             if (g.exact) {
                 const int at_once = pair_slices(8 * nsino, G);
-                CK(c, c->w_q.ensure(sizeof(float2) * nsino * at_once));
+                CKRET(need(c, c->w_q, sizeof(float2) * nsino * at_once));
                 float2* const q = c->w_q.template as<float2>();
                 for (int s = 0; s < G; s += at_once) {
                     const int n = std::min(at_once, G - s);
@@ -416,8 +466,8 @@ int run_op_host(acu_ctx* c, OpKind op, int S, const float* in, float* out)
     const size_t nsino = (size_t)c->T * c->N, nimg = (size_t)c->N * c->N;
     const size_t nin = (op == OP_RADON ? nimg : nsino) * S;
     const size_t nout = (op == OP_RADON || op == OP_FILTER ? nsino : nimg) * S;
-    CK(c, c->w_host_in.ensure(sizeof(float) * nin));
-    CK(c, c->w_host_out.ensure(sizeof(float) * nout));
+    CKRET(need(c, c->w_host_in, sizeof(float) * nin));
+    CKRET(need(c, c->w_host_out, sizeof(float) * nout));
     CK(c, cudaMemcpyAsync(c->w_host_in.p, in, sizeof(float) * nin, cudaMemcpyHostToDevice, c->stream));
     CKRET(run_op<float>(c, op, S, c->w_host_in.template as<float>(), c->w_host_out.template as<float>()));
     CK(c, cudaMemcpyAsync(out, c->w_host_out.p, sizeof(float) * nout, cudaMemcpyDeviceToHost, c->stream));
@@ -537,6 +587,8 @@ struct TvRun {
     }
 };
 
+bool carries(const acu_ctx* c) { return c->opt_residual == 2 && c->opt_refresh != 1; }
+
 template <typename Real, int V>
 TvRun<Real, V> make_run(acu_ctx* c, TvState<Real>& s)
 {
@@ -549,7 +601,7 @@ TvRun<Real, V> make_run(acu_ctx* c, TvState<Real>& s)
     run.verbose = c->opt_verbose != 0;
     run.merged = c->opt_residual != 0;
     run.refresh = c->opt_refresh;
-    run.carried = c->opt_residual == 2 && c->opt_refresh != 1;
+    run.carried = carries(c);
     run.sc = TvScalars{s.rsold.template as<double>(), s.alpha.template as<double>(), s.beta.template as<double>(),
                        s.delta.template as<double>(), s.part.template as<double>(), s.nblk};
     return run;
@@ -565,21 +617,23 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     TvState<Real>& s = tvstate<Real>(c);
     const int N = c->N, T = c->T, G = (S + V - 1) / V;
     const size_t nimg = (size_t)N * N * G * V, nsino = (size_t)T * N * G * V;
-    for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CK(c, b->ensure(sizeof(Real) * nsino));
-    CK(c, s.q.ensure(sizeof(Real) * q_size<Real, V>((size_t)T * N, G)));
+    for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CKRET(need(c, *b, sizeof(Real) * nsino));
+    CKRET(need(c, s.q, sizeof(Real) * q_size<Real, V>((size_t)T * N, G)));
     for (DevBuf* b : {&s.uk, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap, &s.tmp})
-        CK(c, b->ensure(sizeof(Real) * nimg));
-    if (c->opt_verbose) CK(c, s.ukp.ensure(sizeof(Real) * nimg));
+        CKRET(need(c, *b, sizeof(Real) * nimg));
+    if (c->opt_verbose) CKRET(need(c, s.ukp, sizeof(Real) * nimg));
+    if (carries(c))
+        for (DevBuf* b : {&s.bd, &s.dacc}) CKRET(need(c, *b, sizeof(Real) * nimg));
+    const int Sp = G * V;
+    s.nblk = (int)std::min<size_t>(((size_t)N * N + 255) / 256, 512);
+    for (DevBuf* b : {&s.rsold, &s.alpha, &s.beta, &s.delta}) CKRET(need(c, *b, sizeof(double) * Sp));
+    CKRET(need(c, s.part, sizeof(double) * (size_t)s.nblk * Sp));
     if constexpr (V == 4 && sizeof(Real) == 4) {
         CKRET(ensure_projector_buffers(c, G));
         CKRET(ensure_backproject_buffers(c, G));
     } else if constexpr (sizeof(Real) == 4) {
-        CK(c, c->pairPT.ensure(sizeof(float) * std::max(nimg, pair_image_floats(N, G))));
+        CKRET(need(c, c->pairPT, sizeof(float) * std::max(nimg, pair_image_floats(N, G))));
     }
-    const int Sp = G * V;
-    s.nblk = (int)std::min<size_t>(((size_t)N * N + 255) / 256, 512);
-    for (DevBuf* b : {&s.rsold, &s.alpha, &s.beta, &s.delta}) CK(c, b->ensure(sizeof(double) * Sp));
-    CK(c, s.part.ensure(sizeof(double) * (size_t)s.nblk * Sp));
     s.S = S; s.G = G; s.V = V; s.ninner = ninner; s.ncg = ncg; s.lambda = lambda; s.mu = mu;
     s.outer_done = 0;
     s.active = true;
@@ -602,7 +656,6 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     s.carried_valid = false;
     if (run.carried) {
         // fk = f: bd = iradon(f - radon(uk)), dacc = iradon(fk - f) = 0
-        for (DevBuf* b : {&s.bd, &s.dacc}) CK(c, b->ensure(sizeof(Real) * nimg));
         TvEw<Real, V>::diff(nsino, s.f.template as<Real>(), s.ruk.template as<Real>(), s.rp.template as<Real>(), st);
         run.iradon(s.rp.template as<Real>(), s.bd.template as<Real>());
         CK(c, cudaMemsetAsync(s.dacc.p, 0, sizeof(Real) * nimg, st));
@@ -621,16 +674,16 @@ int tv_iterate_v(acu_ctx* c, int nouter)
     cudaStream_t st = c->stream;
     const int S = s.S, Sp = s.G * V;
     const bool use_graph = c->opt_graph != 0 && !run.verbose;
-    // the projector option may have changed since acu_tv_begin
+    // the projector and the residual options may have changed since acu_tv_begin:
+    // the carried backprojections start from the current iterate, and lapse when
+    // not carried
+    if (run.carried)
+        for (DevBuf* b : {&s.bd, &s.dacc}) CKRET(need(c, *b, sizeof(Real) * c->N * c->N * s.G * V));
     if constexpr (V == 4 && sizeof(Real) == 4) {
         CKRET(ensure_projector_buffers(c, s.G));
         CKRET(ensure_backproject_buffers(c, s.G));
     }
-    // the residual options may have changed too: the carried backprojections
-    // start from the current iterate, and lapse when not carried
     if (run.carried && !s.carried_valid) {
-        const size_t nimg = (size_t)c->N * c->N * s.G * V;
-        for (DevBuf* b : {&s.bd, &s.dacc}) CK(c, b->ensure(sizeof(Real) * nimg));
         run.carried_refresh();
         s.carried_valid = true;
     }
@@ -777,7 +830,7 @@ int tv_chunk(acu_ctx* c, int S, bool host_io)
     // chunk of it: count the larger (pixel-line) buffers then
     const int proj = c->opt_projector == 7 ? 6 : c->opt_projector;
     size_t per = sizeof(Real) * (5 * T * N + 10 * N * N);
-    if (c->opt_residual == 2 && c->opt_refresh != 1) per += sizeof(Real) * 2 * N * N;   // bd, dacc
+    if (carries(c)) per += sizeof(Real) * 2 * N * N;   // bd, dacc
     if (sizeof(Real) == 4)
         per += sizeof(float) * (proj == 0 ? 4 * N * N : proj == 6 ? N * N + T * N : N * N);
     if (host_io) per += sizeof(float) * (T * N + 2 * N * N);
@@ -835,12 +888,12 @@ int tv_plain(acu_ctx* c, int S, const float* d_f, int ninner, int nouter, int nc
     TvState<float>& s = c->tv32;
     const int N = c->N, T = c->T;
     const size_t nimg = (size_t)N * N, nsino = (size_t)T * N;
-    for (DevBuf* b : {&s.fk, &s.ruk, &s.rp, &s.q}) CK(c, b->ensure(sizeof(float) * nsino));
+    for (DevBuf* b : {&s.fk, &s.ruk, &s.rp, &s.q}) CKRET(need(c, *b, sizeof(float) * nsino));
     for (DevBuf* b : {&s.uk, &s.ukp, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap, &s.tmp})
-        CK(c, b->ensure(sizeof(float) * nimg));
+        CKRET(need(c, *b, sizeof(float) * nimg));
     const int nblk = (int)std::min<size_t>((nimg + 255) / 256, 512);
-    for (DevBuf* b : {&s.rsold, &s.alpha, &s.beta, &s.delta}) CK(c, b->ensure(sizeof(double) * 1));
-    CK(c, s.part.ensure(sizeof(double) * (size_t)nblk));
+    for (DevBuf* b : {&s.rsold, &s.alpha, &s.beta, &s.delta}) CKRET(need(c, *b, sizeof(double) * 1));
+    CKRET(need(c, s.part, sizeof(double) * (size_t)nblk));
     TvScalars sc{s.rsold.template as<double>(), s.alpha.template as<double>(), s.beta.template as<double>(), s.delta.template as<double>(),
                  s.part.template as<double>(), nblk};
     cudaStream_t st = c->stream;
@@ -919,8 +972,8 @@ int tv_host(acu_ctx* c, bool plain, int S, const float* f, int ninner, int noute
     for (int s0 = 0; s0 < S; s0 += chunk) {
         const int Sc = std::min(chunk, S - s0);
         const size_t nsino = sino1 * Sc, nimg = img1 * Sc;
-        CK(c, c->w_host_in.ensure(sizeof(float) * nsino));
-        CK(c, c->w_host_out.ensure(sizeof(float) * nimg * (fbp ? 2 : 1)));
+        CKRET(need(c, c->w_host_in, sizeof(float) * nsino));
+        CKRET(need(c, c->w_host_out, sizeof(float) * nimg * (fbp ? 2 : 1)));
         float* d_tv = c->w_host_out.template as<float>();
         float* d_fbp = fbp ? d_tv + nimg : nullptr;
         CK(c, cudaMemcpyAsync(c->w_host_in.p, f + s0 * sino1, sizeof(float) * nsino, cudaMemcpyHostToDevice,
@@ -954,9 +1007,9 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     const int N = c->N, T = c->T;
     const size_t nsino = (size_t)T * N, nimg = (size_t)N * N;
     const int nblk = (int)std::min<size_t>((nimg + 255) / 256, 512);
-    CK(c, c->w_in.ensure(sizeof(Real) * nsino * S));      // residual
-    CK(c, c->w_out.ensure(sizeof(Real) * nsino * S));     // offset derivative of the projector
-    CK(c, c->w_part.ensure(sizeof(double) * ((size_t)2 * nblk * S + 2 * S)));
+    CKRET(need(c, c->w_in, sizeof(Real) * nsino * S));      // residual
+    CKRET(need(c, c->w_out, sizeof(Real) * nsino * S));     // offset derivative of the projector
+    CKRET(need(c, c->w_part, sizeof(double) * ((size_t)2 * nblk * S + 2 * S)));
     Real* r = c->w_in.template as<Real>();
     Real* D = c->w_out.template as<Real>();
     double* part = c->w_part.template as<double>();
@@ -967,7 +1020,7 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     if constexpr (sizeof(Real) == 4) fused = g.exact != 0;
     if constexpr (sizeof(Real) == 4) {
         if (fused) {
-            CK(c, c->pairPT.ensure(sizeof(float) * pair_image_floats(N, S)));
+            CKRET(need(c, c->pairPT, sizeof(float) * pair_image_floats(N, S)));
             launch_ray_off(g, S, d_u, c->pairPT.template as<float>(), d_off, r, d_grad_off ? D : nullptr, st);
         }
     }
@@ -978,7 +1031,7 @@ int tv_loss_grad(acu_ctx* c, int S, const Real* d_u, const Real* d_off, const Re
     if (!gu) {
         // loss only: the TV term's kernel still needs a gradient buffer to add
         // into, but the adjoint of the data term is not needed
-        CK(c, c->w_q.ensure(sizeof(Real) * nimg * S));
+        CKRET(need(c, c->w_q, sizeof(Real) * nimg * S));
         gu = c->w_q.template as<Real>();
         CK(c, cudaMemsetAsync(gu, 0, sizeof(Real) * nimg * S, st));
     } else {

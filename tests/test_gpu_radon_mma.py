@@ -172,3 +172,52 @@ def test_a_value_that_is_not_finite_changes_no_other_slice(S):
     got, m = got[bad], torch.isfinite(ref)
     assert torch.equal(torch.isfinite(got), m) and rel(got[m], ref[m]) < 3e-6
     t.close()
+
+
+def test_less_and_less_memory_and_enough_again():
+    """With a little less room than its buffers took the projector does the angles in smaller chunks, with the same bits;
+    with what the pixel-line gathers need it is them; either way it is whole again once there is room.  Its buffers
+    give way to what another call needs."""
+    N, T, S = 513, 180, 64
+    th = syn.angles(T)
+    x = torch.rand(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+
+    def fresh(variant):
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        t = Tomography(N, th, 25)
+        t.set_option(7, variant)
+        out = t.radon(x)
+        torch.cuda.synchronize()
+        taken = free - torch.cuda.mem_get_info()[0]
+        t.close()
+        return out, taken
+
+    whole, most = fresh(7)
+    lines, least = fresh(6)          # either counts the result's own memory
+    assert not torch.equal(whole, lines) and most - least > 64 << 20
+    for room, want in ((most - (16 << 20), whole), (least + (16 << 20), lines)):
+        torch.cuda.empty_cache()
+        t = Tomography(N, th, 25)
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+        got = t.radon(x)
+        del hold
+        torch.cuda.empty_cache()
+        assert torch.equal(got, want)
+        assert torch.equal(t.radon(x), whole)
+        t.close()
+
+    # filtering 256 slices needs 98 MB more than the projection left: 32 are free, its buffers hold the others
+    y = torch.rand(256, T, N, device="cuda")
+    with Tomography(N, th, 25) as t:
+        ref = t.filter(y)
+        t.filter(y)                  # leaves torch the memory of another result
+    t = Tomography(N, th, 25)
+    t.radon(x)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8, device="cuda")
+    got = t.filter(y)
+    del hold
+    torch.cuda.empty_cache()
+    assert torch.equal(got, ref)
+    assert torch.equal(t.radon(x), whole)
+    t.close()
