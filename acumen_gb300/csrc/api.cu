@@ -238,20 +238,31 @@ void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q,
     launch_backproject<Real, V>(g, G, q, img, c->stream);
 }
 
-// Elements of the filtered sinogram's buffer (nsino each, G groups).  Single
-// slices are backprojected from pairs (bin, next bin), some slices at a time.
+// Whether single slices are filtered into pairs (bin, next bin), some slices at a time.
 template <typename Real, int V>
-size_t q_size(size_t nsino, int G)
+bool filters_pairs(const acu_ctx* c, const DevGeom<Real>& g)
 {
-    const size_t all = nsino * G * V;
-    return V == 1 && sizeof(Real) == 4 ? std::max(all, 2 * nsino * pair_slices(8 * nsino, G)) : all;
+    return V == 1 && sizeof(Real) == 4 && g.exact && c->opt_filter == 0 && g.fft_L > 0 && fft_fits<Real>(g.fft_L);
+}
+
+// Elements of the filtered sinogram's buffer (nsino each, G groups).
+template <typename Real, int V>
+size_t q_size(const acu_ctx* c, const DevGeom<Real>& g, size_t nsino, int G)
+{
+    return filters_pairs<Real, V>(c, g) ? 2 * nsino * pair_slices(8 * nsino, G) : nsino * G * V;
+}
+
+// The single-slice projector's buffer: pairs of images, or their transposes.
+int ensure_single_buffer(acu_ctx* c, int S)
+{
+    return need(c, c->pairPT, sizeof(float) * (radon_v1_pairs(c->g32.d) ? pair_image_floats(c->N, S) : (size_t)c->N * c->N * S));
 }
 
 template <typename Real, int V>
 void lanes_iradon(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* sino, Real* q, Real* img)
 {
     if constexpr (V == 1 && sizeof(Real) == 4) {
-        if (g.exact && c->opt_filter == 0 && g.fft_L > 0 && fft_fits<Real>(g.fft_L)) {
+        if (filters_pairs<Real, V>(c, g)) {
             const size_t nsino = (size_t)g.T * g.N, nimg = (size_t)g.N * g.N;
             const int at_once = pair_slices(8 * nsino, G);
             for (int s = 0; s < G; s += at_once) {
@@ -379,7 +390,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
     }
     switch (op) {
     case OP_IRADON:
-        CKRET(need(c, c->w_q, sizeof(Real) * q_size<Real, V>(nsino, G)));
+        CKRET(need(c, c->w_q, sizeof(Real) * q_size<Real, V>(c, g, nsino, G)));
         if constexpr (V == 4 && sizeof(Real) == 4) CKRET(ensure_backproject_buffers(c, G));
         lanes_iradon<Real, V>(c, g, G, lin, c->w_q.template as<Real>(), lout);
         break;
@@ -388,7 +399,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
             CKRET(ensure_projector_buffers(c, G));
             radon_quads(c, g, G, lin, lout);
         } else if constexpr (V == 1 && sizeof(Real) == 4) {
-            CKRET(need(c, c->pairPT, sizeof(float) * std::max(nimg * G, pair_image_floats(N, G))));
+            CKRET(ensure_single_buffer(c, G));
             launch_radon_v1_fast(g, G, lin, c->pairPT.template as<float>(), lout, c->stream);
         } else {
             launch_radon<Real, V>(g, G, lin, lout, c->stream);
@@ -618,7 +629,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
     const int N = c->N, T = c->T, G = (S + V - 1) / V;
     const size_t nimg = (size_t)N * N * G * V, nsino = (size_t)T * N * G * V;
     for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CKRET(need(c, *b, sizeof(Real) * nsino));
-    CKRET(need(c, s.q, sizeof(Real) * q_size<Real, V>((size_t)T * N, G)));
+    CKRET(need(c, s.q, sizeof(Real) * q_size<Real, V>(c, geomset<Real>(c).d, (size_t)T * N, G)));
     for (DevBuf* b : {&s.uk, &s.dx, &s.dy, &s.bx, &s.by, &s.rhs, &s.r, &s.p, &s.Ap, &s.tmp})
         CKRET(need(c, *b, sizeof(Real) * nimg));
     if (c->opt_verbose) CKRET(need(c, s.ukp, sizeof(Real) * nimg));
@@ -632,7 +643,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
         CKRET(ensure_projector_buffers(c, G));
         CKRET(ensure_backproject_buffers(c, G));
     } else if constexpr (sizeof(Real) == 4) {
-        CKRET(need(c, c->pairPT, sizeof(float) * std::max(nimg, pair_image_floats(N, G))));
+        CKRET(ensure_single_buffer(c, G));
     }
     s.S = S; s.G = G; s.V = V; s.ninner = ninner; s.ncg = ncg; s.lambda = lambda; s.mu = mu;
     s.outer_done = 0;
@@ -674,14 +685,17 @@ int tv_iterate_v(acu_ctx* c, int nouter)
     cudaStream_t st = c->stream;
     const int S = s.S, Sp = s.G * V;
     const bool use_graph = c->opt_graph != 0 && !run.verbose;
-    // the projector and the residual options may have changed since acu_tv_begin:
+    // the projector, filter, position and residual options may have changed since acu_tv_begin:
     // the carried backprojections start from the current iterate, and lapse when
     // not carried
     if (run.carried)
         for (DevBuf* b : {&s.bd, &s.dacc}) CKRET(need(c, *b, sizeof(Real) * c->N * c->N * s.G * V));
+    CKRET(need(c, s.q, sizeof(Real) * q_size<Real, V>(c, *run.g, (size_t)c->T * c->N, s.G)));
     if constexpr (V == 4 && sizeof(Real) == 4) {
         CKRET(ensure_projector_buffers(c, s.G));
         CKRET(ensure_backproject_buffers(c, s.G));
+    } else if constexpr (sizeof(Real) == 4) {
+        CKRET(ensure_single_buffer(c, s.G));
     }
     if (run.carried && !s.carried_valid) {
         run.carried_refresh();

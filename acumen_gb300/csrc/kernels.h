@@ -128,8 +128,6 @@ size_t bp_mma_bins_bytes(int N, int T, int G);
 size_t bp_mma_scalars(int G);
 bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
                             cudaStream_t st);
-// The staggered projector for one slice per thread (plain layout); IT is a
-// work buffer of N * N floats per slice and no less than pair_image_floats.
 // Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
 // (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
 // the derivative with respect to them or null; launch_backproject_fx: q as pairs
@@ -151,6 +149,9 @@ template <int V>
 void launch_adjoint_fx(const DevGeom<float>& g, int G, const float* sino, const float* off, float* img, cudaStream_t st);
 void launch_pairs(const float* q, float2* out, int N, size_t n, cudaStream_t st);
 void launch_transpose_v1(int N, int S, const float* img, float* IT, cudaStream_t st);
+// The single-slice projector: through pairs (IT of pair_image_floats floats), else along
+// staggered rays through the image and its transpose (IT of N * N floats per slice).
+inline bool radon_v1_pairs(const DevGeom<float>& g) { return g.exact && g.N <= FX_MAX_SIDE; }
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st);
 template <typename Real, int V>
 void launch_radon_adjoint(const DevGeom<Real>& g, int G, const Real* sino, Real* img, cudaStream_t st);

@@ -878,7 +878,7 @@ void launch_transpose_v1(int N, int S, const float* img, float* IT, cudaStream_t
 
 void launch_radon_v1_fast(const DevGeom<float>& g, int S, const float* img, float* IT, float* sino, cudaStream_t st)
 {
-    if (g.exact && g.N <= FX_MAX_SIDE) return launch_radon_fx(g, S, img, IT, sino, st);
+    if (radon_v1_pairs(g)) return launch_radon_fx(g, S, img, IT, sino, st);
     launch_transpose_v1(g.N, S, img, IT, st);
     dim3 blk(32, 4), grd((g.N + 127) / 128, g.T, S);
     if (g.exact)

@@ -132,3 +132,40 @@ def test_more_slices_than_a_buffer_of_pairs():
         assert torch.equal(p[s], one[k][0][0]) and torch.equal(r[s], one[k][1][0]) and torch.equal(b[s], one[k][2][0])
         assert loss[s] == one[k][3][0][0] and torch.equal(gu[s], one[k][3][1][0]) and torch.equal(go[s], one[k][3][2][0])
     t.close()
+
+
+# the reference's positions, and a side beyond the fixed-point kernels'
+@pytest.mark.parametrize("N, positions", [(2049, 0), (4200, 1)])
+def test_pairs_take_memory_only_where_they_are_used(N, positions):
+    x = torch.rand(1, N, N, device="cuda")
+    with Tomography(33, axes(9), 2) as t:
+        t.radon(x[:, :33, :33])              # the library's code is loaded
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    t = Tomography(N, axes(9), 2)
+    t.set_option(8, positions)
+    y = t.radon(x)
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert taken < 2 * 4 * N * N + 24e6      # the mask and a transposed image; the sinogram and tables are small
+    assert rel(y, t.radon(x.repeat(4, 1, 1))[:1]) < 3e-6
+    t.close()
+
+
+def test_buffers_follow_options_changed_between_the_solvers_steps():
+    """Other positions and another filter need other buffers for one slice."""
+    N, T = 257, 90
+    th = syn.angles(T)
+    f = syn.normalised_sinogram(syn.random_ellipses(2, 0.3 * N), N, th, I0=5e3, seed=2, device="cuda")[None]
+    for first, then in (((8, 0), (8, 1)), ((1, 1), (1, 0))):
+        t = Tomography(N, th, 12)
+        t.set_option(*first)
+        t.tv_begin(f, 1, 3, 0.05, 1.0)
+        t.set_option(*then)
+        t.tv_iterate(2)
+        u = t.tv_end()
+        t.close()
+        with Tomography(N, th, 12) as t:
+            ref, _ = t.tvopt(f, 1, 2, 3, 0.05, 1.0)
+            mask = t.backproject(torch.ones(1, T, N, device="cuda"))[0] != 0
+        # TV with either stays within 1e-4 of FP64 inside the mask (test_gpu_tv)
+        assert rel(u[:, mask], ref[:, mask]) < 2e-4
