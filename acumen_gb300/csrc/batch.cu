@@ -627,7 +627,13 @@ struct acu_batch {
     std::vector<int> order;           // execution order (largest work first) -> caller index
     BatchDev dev;
     DevBuf d_pd, d_sc_bp, d_sc_fp, d_xsc_bp, d_xsc_fp, d_fx_fp, d_cm, d_fh, d_fhx, d_tw, d_counter;
-    DevBuf f, fk, ruk, rp, q, uk, dx, dy, bx, by, rhs, r, p, Ap, tmp, part, rsold, alpha, beta;
+    DevBuf f, fk, ruk, rp, uk, dx, dy, bx, by, r, p, part, rsold, alpha, beta;
+    // One buffer in turns: images that pass from one step to the next (tmp, rhs, Ap), the
+    // projector's pairs (or transposes) of images in all of it, and the filtered bins (q)
+    // in all but tmp, which the backprojection writes.  No image but tmp is
+    // read after an operator has run.
+    DevBuf work;
+    float *tmp = nullptr, *rhs = nullptr, *Ap = nullptr, *q = nullptr;
     DevBuf io_in, io_out;
     cudaGraphExec_t graph = nullptr, graph_inc = nullptr;
     std::string graph_key;
@@ -662,22 +668,22 @@ void batch_outer(acu_batch* b, cudaStream_t st, int ninner, int ncg, float lambd
     auto F = [](DevBuf& x) { return x.as<float>(); };
     auto D = [](DevBuf& x) { return x.as<double>(); };
     auto iradon = [&](const float* s, float* img) {
-        batch_filter(d, s, F(b->q), st);
-        batch_backproject(d, F(b->q), img, 1, st);
+        batch_filter(d, s, b->q, st);
+        batch_backproject(d, b->q, img, 1, st);
     };
     for (int ji = 1; ji <= ninner; ++ji) {
         if (ji > 1 && !carry) batch_radon(d, F(b->uk), F(b->ruk), 0, st);
         batch_diff(d, F(b->fk), F(b->ruk), F(b->rp), st);
-        iradon(F(b->rp), F(b->tmp));
-        batch_rhs(d, mu, lambda, F(b->tmp), F(b->dx), F(b->bx), F(b->dy), F(b->by), F(b->rhs), st);
-        batch_resid(d, mu, lambda, F(b->rhs), nullptr, F(b->uk), F(b->r), F(b->p), D(b->part), st);
+        iradon(F(b->rp), b->tmp);
+        batch_rhs(d, mu, lambda, b->tmp, F(b->dx), F(b->bx), F(b->dy), F(b->by), b->rhs, st);
+        batch_resid(d, mu, lambda, b->rhs, nullptr, F(b->uk), F(b->r), F(b->p), D(b->part), st);
         batch_finalize(d, 0, D(b->part), D(b->rsold), D(b->alpha), D(b->beta), st);
         for (int k = 0; k < ncg; ++k) {
             batch_radon(d, F(b->p), F(b->rp), 0, st);
-            iradon(F(b->rp), F(b->tmp));
-            batch_apply(d, mu, lambda, F(b->tmp), F(b->p), F(b->Ap), D(b->part), st);
+            iradon(F(b->rp), b->tmp);
+            batch_apply(d, mu, lambda, b->tmp, F(b->p), b->Ap, D(b->part), st);
             batch_finalize(d, 1, D(b->part), D(b->rsold), D(b->alpha), D(b->beta), st);
-            batch_update(d, F(b->p), F(b->Ap), F(b->uk), F(b->r), D(b->alpha), D(b->part), st);
+            batch_update(d, F(b->p), b->Ap, F(b->uk), F(b->r), D(b->alpha), D(b->part), st);
             if (carry) batch_sino_axpy(d, D(b->alpha), F(b->rp), F(b->ruk), st);
             batch_finalize(d, 2, D(b->part), D(b->rsold), D(b->alpha), D(b->beta), st);
             batch_pupdate(d, F(b->r), F(b->p), D(b->beta), st);
@@ -910,11 +916,15 @@ int ensure_state(acu_batch* b)
     acu_ctx* c = b->ctx;
     const size_t ni = sizeof(float) * (size_t)b->dev.img_total, ns = sizeof(float) * (size_t)b->dev.sino_total;
     for (DevBuf* x : {&b->f, &b->fk, &b->ruk, &b->rp}) CK(c, x->ensure(ns));
-    for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->rhs, &b->r, &b->p, &b->Ap, &b->tmp})
-        CK(c, x->ensure(ni));
-    // one buffer, at exact positions for pairs: the projector's of the images and their transposes, or the filtered bins'
-    CK(c, b->q.ensure(std::max(4 * ni, 2 * ns)));
-    b->dev.IT = b->q.as<float>();
+    for (DevBuf* x : {&b->uk, &b->dx, &b->dy, &b->bx, &b->by, &b->r, &b->p}) CK(c, x->ensure(ni));
+    // at exact positions: pairs of the images, of their transposes and of the filtered bins
+    const bool pairs = b->dev.exact != 0;
+    const size_t n = ((size_t)b->dev.img_total + 63) / 64 * 64, sino = (size_t)b->dev.sino_total;
+    CK(c, b->work.ensure(sizeof(float) * (n + std::max((pairs ? 3 : 2) * n, (pairs ? 2 : 1) * sino))));
+    b->tmp = b->work.as<float>();
+    b->rhs = b->q = b->tmp + n;
+    b->Ap = b->rhs + n;
+    b->dev.IT = b->tmp;
     CK(c, b->part.ensure(sizeof(double) * (size_t)b->dev.n_ew));
     for (DevBuf* x : {&b->rsold, &b->alpha, &b->beta}) CK(c, x->ensure(sizeof(double) * b->nprob));
     return ACU_OK;
@@ -925,7 +935,7 @@ int tune_all(acu_batch* b)
     if (b->tuned) return ACU_OK;
     CKRET(ensure_state(b));
     CK(b->ctx, cudaMemsetAsync(b->uk.p, 0, sizeof(float) * b->dev.img_total, b->ctx->stream));
-    CK(b->ctx, cudaMemsetAsync(b->q.p, 0, 2 * sizeof(float) * b->dev.sino_total, b->ctx->stream));
+    CK(b->ctx, cudaMemsetAsync(b->work.p, 0, b->work.n, b->ctx->stream));
     // the backprojection work list must match the tile height while timing
     cudaStream_t st = b->ctx->stream;
     cudaEvent_t e0, e1;
@@ -935,9 +945,9 @@ int tune_all(acu_batch* b)
     int br = 8;
     for (int rr : {4, 8, 16}) {
         CKRET(set_bp_rows(b, rr));
-        batch_backproject(b->dev, b->q.as<float>(), b->tmp.as<float>(), 1, st);
+        batch_backproject(b->dev, b->q, b->tmp, 1, st);
         CK(b->ctx, cudaEventRecord(e0, st));
-        batch_backproject(b->dev, b->q.as<float>(), b->tmp.as<float>(), 1, st);
+        batch_backproject(b->dev, b->q, b->tmp, 1, st);
         CK(b->ctx, cudaEventRecord(e1, st));
         CK(b->ctx, cudaEventSynchronize(e1));
         float ms = 0;
@@ -962,17 +972,17 @@ int batch_solve(acu_batch* b, const float* d_f_exec, int ninner, int nouter, int
     const BatchDev& d = b->dev;
     auto F = [](DevBuf& x) { return x.as<float>(); };
     CK(c, cudaMemcpyAsync(b->f.p, d_f_exec, sizeof(float) * d.sino_total, cudaMemcpyDeviceToDevice, st));
-    batch_filter(d, F(b->f), F(b->q), st);
-    batch_backproject(d, F(b->q), F(b->uk), 1, st);
+    batch_filter(d, F(b->f), b->q, st);
+    batch_backproject(d, b->q, F(b->uk), 1, st);
     if (d_fbp_exec) CK(c, cudaMemcpyAsync(d_fbp_exec, b->uk.p, sizeof(float) * d.img_total, cudaMemcpyDeviceToDevice, st));
     for (DevBuf* x : {&b->dx, &b->dy, &b->bx, &b->by}) CK(c, cudaMemsetAsync(x->p, 0, sizeof(float) * d.img_total, st));
     CK(c, cudaMemcpyAsync(b->fk.p, b->f.p, sizeof(float) * d.sino_total, cudaMemcpyDeviceToDevice, st));
     batch_radon(d, F(b->uk), F(b->ruk), 0, st);
     CKLAUNCH(c);
     if (nouter > 0) {
-        char key[160];
-        snprintf(key, sizeof key, "%d/%d/%.9g/%.9g/%d/%d/%d/%d", ninner, ncg, (double)lambda, (double)mu,
-                 d.radon_warps, d.bp_rows, d.exact, b->refresh);
+        char key[192];   // the work buffer grows with the positions' option, the others once and for all
+        snprintf(key, sizeof key, "%d/%d/%.9g/%.9g/%d/%d/%d/%d/%llu", ninner, ncg, (double)lambda, (double)mu,
+                 d.radon_warps, d.bp_rows, d.exact, b->refresh, (unsigned long long)b->work.id);
         if (!b->graph || b->graph_key != key) {
             for (cudaGraphExec_t* gx : {&b->graph, &b->graph_inc})
                 if (*gx) {
@@ -1050,8 +1060,8 @@ int acu_batch_op(acu_batch* b, int op, const float* in, float* out)
     if (op == 0) {
         batch_radon(b->dev, din, dout, 0, c->stream);
     } else {
-        batch_filter(b->dev, din, b->q.as<float>(), c->stream);
-        batch_backproject(b->dev, b->q.as<float>(), dout, 1, c->stream);
+        batch_filter(b->dev, din, b->q, c->stream);
+        batch_backproject(b->dev, b->q, dout, 1, c->stream);
     }
     CKLAUNCH(c);
     CKRET(repack(b, dout, out, op == 0, false, cudaMemcpyDeviceToHost));

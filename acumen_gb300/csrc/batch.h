@@ -42,7 +42,7 @@ struct BatchDev {
     const float2* tw = nullptr;   // twiddles of the largest L (Lmax entries)
     int Lmax = 0;
     long long n_radon = 0, n_bp = 0, n_fft = 0, n_ew = 0, n_tr = 0;   // item totals
-    float* IT = nullptr;          // work buffer: transposed images, or pairs of both (4 img_total floats)
+    float* IT = nullptr;          // work buffer: transposed images (img_total floats), or pairs of both (4 times that)
     long long img_total = 0, sino_total = 0;
     int* counter = nullptr;       // work counters (one per persistent kernel)
     int radon_warps = 4;          // autotuned: warps per projector block

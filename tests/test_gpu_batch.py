@@ -121,3 +121,49 @@ def test_batch_at_uneven_batch_sizes_vs_fp64_oracle(oracle, built_lib):
         mask = oracle.cmask(N, T, 100, 64) > 0
         assert rel(fbp[i], ref_fbp) < 1e-5, i
         assert rel(tv[i], ref_tv, mask) < 1e-4, i
+
+
+# an odd number of pixels in all; many more angles than pixels and the other way round
+@pytest.mark.parametrize("spec", [[(33, 257), (64, 300), (40, 180)], [(130, 9), (97, 7)]])
+def test_steps_share_one_buffer(oracle, built_lib, spec):
+    """The projector's pairs, the filtered bins and the solver's passing images take turns in one buffer, which grows when
+    the positions' option is changed; graphs of either follow it."""
+    sinos = [syn.analytic_sinogram(syn.random_ellipses(20 + i, 0.3 * N), N, syn.angles(T)).numpy().astype(np.float32)
+             for i, (N, T) in enumerate(spec)]
+
+    def solve(b, nouter=2):
+        return b.tvopt(sinos, 2, nouter, 3, 0.05, 1.0)
+
+    fresh = []
+    for positions in (0, 1):
+        b = RaggedBatch([N for N, _ in spec], [syn.angles(T) for _, T in spec], 4)
+        b.set_option(8, positions)
+        fresh.append(solve(b))
+        b.close()
+    for i, (N, T) in enumerate(spec):
+        ref_tv, ref_fbp = oracle.tvopt(sinos[i].astype(np.float64), syn.angles(T), 4, 2, 2, 3, 0.05, 1.0, prec=64)
+        mask = oracle.cmask(N, T, 4, 64) > 0
+        assert rel(fresh[1][0][i], ref_tv, mask) < 1e-4 and rel(fresh[1][1][i], ref_fbp) < 1e-5
+    b = RaggedBatch([N for N, _ in spec], [syn.angles(T) for _, T in spec], 4)
+    for positions, nouter in ((0, 2), (1, 0), (0, 2), (1, 2), (0, 2)):
+        b.set_option(8, positions)
+        tv, fbp = solve(b, nouter)
+        for got, want in zip(tv + fbp, (fresh[positions][0] if nouter else fresh[positions][1]) + fresh[positions][1]):
+            np.testing.assert_array_equal(got, want)
+
+
+def test_memory_of_a_batch():
+    """Four images' worth of pairs take the place of what does not live at the same time."""
+    import torch
+    N, T, P = 1025, 600, 4
+    b = RaggedBatch([N] * P, [syn.angles(T)] * P, 50)
+    b.tvopt([np.zeros((T, N), np.float32)] * P, 1, 1, 1, 0.05, 1.0)   # the library's code is loaded
+    b.close()
+    free = torch.cuda.mem_get_info()[0]
+    b = RaggedBatch([N] * P, [syn.angles(T)] * P, 50)
+    b.tvopt([np.zeros((T, N), np.float32)] * P, 1, 1, 1, 0.05, 1.0)
+    taken = free - torch.cuda.mem_get_info()[0]
+    images, sinos = 4 * P * N * N, 4 * P * T * N
+    # masks, results (2), 7 images that live on, 4 in turns; inputs, 4 sinograms that live on
+    assert taken < 14 * images + 5 * sinos + 32e6
+    b.close()
