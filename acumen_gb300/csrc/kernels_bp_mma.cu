@@ -379,14 +379,16 @@ __device__ __forceinline__ int scale_exp(unsigned top)
     return top && top < 0x7f800000u ? max((int)(top >> 23) - 127, -98) : 0;
 }
 
-// One bin and angle per thread: its 64 slices of block blockIdx.z as eight pieces of hi and eight of lo halves.
+// One bin and angle per thread (grid.x: 128 bins of every angle, of which there may be more than a grid has
+// rows): its 64 slices of block blockIdx.y as eight pieces of hi and eight of lo halves.
 __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, const unsigned* __restrict__ top,
                                                  float* __restrict__ scale, uint4* __restrict__ bins, int N, int T,
                                                  int G, int g0)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y, k = blockIdx.z;
+    const int nb = (N + 127) / 128, t = blockIdx.x / nb, k = blockIdx.y;
+    const int i = (blockIdx.x - t * nb) * 128 + threadIdx.x;
     if (i >= N) return;
-    uint4* const out = bins + (size_t)t * gridDim.z * (2 * NS / 8) * N + i;
+    uint4* const out = bins + (size_t)t * gridDim.y * (2 * NS / 8) * N + i;
 #pragma unroll 2
     for (int c = 0; c < NS / 8; ++c) {
         __align__(16) __half hi[8], lo[8];
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, c
             }
         }
         out[(size_t)(k * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(hi);
-        out[(size_t)((gridDim.z + k) * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(lo);
+        out[(size_t)((gridDim.y + k) * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(lo);
     }
 }
 
@@ -499,7 +501,7 @@ bool bp_pass(const DevGeom<float>& g, int G, int g0, const float* q, void* bins,
     CUtensorMap map;
     if (!bins_map(&map, bins, g.N, g.T, Bp<BLK>::CHUNKS)) return false;
     const int nt = (g.N + TP - 1) / TP;
-    k_bp_bins<<<dim3((g.N + 127) / 128, g.T, BLK), 128, 0, st>>>(reinterpret_cast<const float4*>(q), top, scale,
+    k_bp_bins<<<dim3((g.N + 127) / 128 * g.T, BLK), 128, 0, st>>>(reinterpret_cast<const float4*>(q), top, scale,
                                                                 reinterpret_cast<uint4*>(bins), g.N, g.T, G, g0);
     max_dynamic_smem<k_bp_mma<BLK>>();
     k_bp_mma<BLK><<<std::min(sms, g.n_tiles_in), 32 * Bp<BLK>::WARPS, Bp<BLK>::BARS + sizeof(Shared), st>>>(
