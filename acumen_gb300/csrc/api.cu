@@ -173,6 +173,7 @@ int need(acu_ctx* c, DevBuf& b, size_t bytes)
         for (DevBuf* o : {&c->mmaT, &c->mmaP, &c->bpQ}) o->release();
         e = b.ensure(bytes);
     }
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported here, not by the next call's launches
     CK(c, e);
     return ACU_OK;
 }
@@ -626,6 +627,7 @@ int tv_begin_v(acu_ctx* c, int S, const Real* d_f, int ninner, int ncg, double l
 {
     CKRET(ensure_geom<Real>(c));
     TvState<Real>& s = tvstate<Real>(c);
+    s.active = false;   // until all its buffers are there: one that cannot grow is gone
     const int N = c->N, T = c->T, G = (S + V - 1) / V;
     const size_t nimg = (size_t)N * N * G * V, nsino = (size_t)T * N * G * V;
     for (DevBuf* b : {&s.f, &s.fk, &s.ruk, &s.rp}) CKRET(need(c, *b, sizeof(Real) * nsino));

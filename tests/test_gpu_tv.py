@@ -300,3 +300,26 @@ def test_graph_is_captured_anew_when_a_buffer_has_moved(built_lib):
         tv, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
         assert torch.equal(tv, ref)
         t.close()
+
+
+def test_no_problem_is_active_after_a_refused_one(built_lib):
+    """A problem whose memory cannot be had has given up the buffers of the one before."""
+    from acumen_gb300._lib import AcumenError
+    N, T = 257, 90
+    f = torch.rand(400, T, N, device="cuda")
+    t = Tomography(N, syn.angles(T), 12)
+    t.tv_begin(f[:4], 1, 2, 0.05, 1.0)
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(AcumenError):
+        t.tv_begin(f, 1, 2, 0.05, 1.0)       # its images take 106 MB each
+    del hold
+    torch.cuda.empty_cache()
+    with pytest.raises(AcumenError, match="no active TV problem"):
+        t.tv_iterate(1)
+    t.tv_begin(f[:4], 1, 2, 0.05, 1.0)
+    t.tv_iterate(1)
+    with Tomography(N, syn.angles(T), 12) as fresh:
+        ref, _ = fresh.tvopt(f[:4], 1, 1, 2, 0.05, 1.0)
+    assert torch.equal(t.tv_end(), ref)
+    t.close()
