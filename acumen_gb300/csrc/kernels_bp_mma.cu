@@ -19,7 +19,7 @@
 //   k_bp_bins     lane sinogram -> bins in operand layout [angle][8 slices, hi then lo][bin][8]
 //   k_bp_mma      the products (tiles that meet the mask)
 //   k_bp_zero     zeros in the other tiles
-//   k_bp_flagged  plain gathers of slices with a value that is not finite, NaN if a wait gave up
+//   k_bp_flagged  plain gathers of slices with a value that is not finite or a few that dwarf the others, NaN if a wait gave up
 #include <cuda.h>
 
 #include <algorithm>
@@ -380,15 +380,16 @@ __device__ __forceinline__ int scale_exp(unsigned top)
 }
 
 // One bin and angle per thread (grid.x: 128 bins of every angle, of which there may be more than a grid has
-// rows): its 64 slices of block blockIdx.y as eight pieces of hi and eight of lo halves.
+// rows): its 64 slices of block blockIdx.y as eight pieces of hi and eight of lo halves.  A half ends at 2^-24, so a value
+// below 2^-16 of its slice's largest keeps fewer than 23 bits: brief counts those of each slice (one in 10^4 as a rule).
 __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, const unsigned* __restrict__ top,
-                                                 float* __restrict__ scale, uint4* __restrict__ bins, int N, int T,
-                                                 int G, int g0)
+                                                 float* __restrict__ scale, unsigned* __restrict__ brief,
+                                                 uint4* __restrict__ bins, int N, int T, int G, int g0)
 {
     const int nb = (N + 127) / 128, t = blockIdx.x / nb, k = blockIdx.y;
     const int i = (blockIdx.x - t * nb) * 128 + threadIdx.x;
-    if (i >= N) return;
     uint4* const out = bins + (size_t)t * gridDim.y * (2 * NS / 8) * N + i;
+    unsigned long long few = 0;   // slices whose value keeps fewer bits than others
 #pragma unroll 2
     for (int c = 0; c < NS / 8; ++c) {
         __align__(16) __half hi[8], lo[8];
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, c
             const int g = g0 + k * (NS / 4) + 2 * c + e;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             uint4 m = make_uint4(0, 0, 0, 0);
-            if (g < G) {
+            if (g < G && i < N) {
                 v = __ldg(q + ((size_t)g * T + t) * N + i);
                 m = __ldg(reinterpret_cast<const uint4*>(top) + g);
                 if (i == 0 && t == 0) {
@@ -410,12 +411,24 @@ __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, c
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float s = f[j] * __int_as_float((14 - scale_exp(b[j]) + 127) << 23);
+                if (s != 0.f && fabsf(s) < 0.25f) few |= 1ull << (8 * c + 4 * e + j);
                 hi[4 * e + j] = __float2half_rn(s);
                 lo[4 * e + j] = __float2half_rn(s - __half2float(hi[4 * e + j]));
             }
         }
-        out[(size_t)(k * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(hi);
-        out[(size_t)((gridDim.y + k) * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(lo);
+        if (i < N) {
+            out[(size_t)(k * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(hi);
+            out[(size_t)((gridDim.y + k) * (NS / 8) + c) * N] = *reinterpret_cast<const uint4*>(lo);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const unsigned mine = (unsigned)(few >> 32 * h);
+        for (unsigned any = __reduce_or_sync(0xffffffffu, mine); any; any &= any - 1) {
+            const int b = __ffs(any) - 1;
+            const unsigned n = __popc(__ballot_sync(0xffffffffu, mine >> b & 1));
+            if ((threadIdx.x & 31) == 0) atomicAdd(brief + 4 * g0 + k * NS + 32 * h + b, n);
+        }
     }
 }
 
@@ -430,22 +443,25 @@ __global__ void __launch_bounds__(PIX) k_bp_zero(const int* __restrict__ list, f
 }
 
 // The slices that held a value that is not finite by plain gathers (as k_backproject_exact): a slice is a column of the
-// product, which spreads such a value over its tiles and no further (one such slice of 256 at
+// product, which spreads such a value over its tiles and no further; and the slices of which a quarter of the values keep
+// fewer bits than the others, because a few are more than 2^16 times larger (one such slice of 256 at
 // 2049^2 x 1200: 8 ms, after 81).  NaN in all of the image if a wait gave up.
 __global__ void __launch_bounds__(256) k_bp_flagged(const float* __restrict__ q, const float* __restrict__ cmask,
                                                     const float4* __restrict__ xsc, float* __restrict__ img, int N,
                                                     int T, int G, float mid, const unsigned* __restrict__ top,
-                                                    const int* __restrict__ err)
+                                                    const unsigned* __restrict__ brief, const int* __restrict__ err)
 {
     const bool lost = *err != 0;
-    bool any = lost;
-    for (int i = threadIdx.x; i < 4 * G; i += 256) any |= top[i] >= 0x7f800000u;
+    const size_t quarter = (size_t)T * N / 4;
+    auto wanted = [&](int s) { return lost || top[s] >= 0x7f800000u || brief[s] > quarter; };
+    bool any = false;
+    for (int i = threadIdx.x; i < 4 * G; i += 256) any |= wanted(i);
     if (!__syncthreads_or(any)) return;
     const size_t NN = (size_t)N * N;
     for (size_t g = 0; g < G; ++g) {
-        const uint4 m = __ldg(reinterpret_cast<const uint4*>(top) + g);
-        const bool marked[4] = {lost || m.x >= 0x7f800000u, lost || m.y >= 0x7f800000u, lost || m.z >= 0x7f800000u,
-                                lost || m.w >= 0x7f800000u};
+        bool marked[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) marked[v] = wanted((int)g * 4 + v);
         if (!(marked[0] || marked[1] || marked[2] || marked[3])) continue;
         for (size_t pix = blockIdx.x * (size_t)blockDim.x + threadIdx.x; pix < NN; pix += (size_t)gridDim.x * blockDim.x) {
             const float dx = (float)(pix % N + 1) - mid, dy = (float)(pix / N + 1) - mid;
@@ -496,12 +512,12 @@ bool bins_map(CUtensorMap* map, void* bins, int N, int T, int chunks)
 
 template <int BLK>
 bool bp_pass(const DevGeom<float>& g, int G, int g0, const float* q, void* bins, unsigned* top, float* scale,
-             float* img, int* err, int sms, cudaStream_t st)
+             unsigned* brief, float* img, int* err, int sms, cudaStream_t st)
 {
     CUtensorMap map;
     if (!bins_map(&map, bins, g.N, g.T, Bp<BLK>::CHUNKS)) return false;
     const int nt = (g.N + TP - 1) / TP;
-    k_bp_bins<<<dim3((g.N + 127) / 128 * g.T, BLK), 128, 0, st>>>(reinterpret_cast<const float4*>(q), top, scale,
+    k_bp_bins<<<dim3((g.N + 127) / 128 * g.T, BLK), 128, 0, st>>>(reinterpret_cast<const float4*>(q), top, scale, brief,
                                                                 reinterpret_cast<uint4*>(bins), g.N, g.T, G, g0);
     max_dynamic_smem<k_bp_mma<BLK>>();
     k_bp_mma<BLK><<<std::min(sms, g.n_tiles_in), 32 * Bp<BLK>::WARPS, Bp<BLK>::BARS + sizeof(Shared), st>>>(
@@ -532,7 +548,7 @@ size_t bp_mma_bins_bytes(int N, int T, int G)
 {
     return (size_t)T * N * NS * 4 * (G > NS / 4 ? 2 : 1);
 }
-size_t bp_mma_scalars(int G) { return (size_t)8 * G + 8; }
+size_t bp_mma_scalars(int G) { return (size_t)8 * G + (G * 4 + NS - 1) / NS * NS + 1; }
 
 bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
                             cudaStream_t st)
@@ -543,22 +559,23 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     unsigned* top = scalars;
     float* scale = reinterpret_cast<float*>(scalars + 4 * (size_t)G);
-    int* err = reinterpret_cast<int*>(scalars + 8 * (size_t)G);   // a wait gave up
+    unsigned* brief = scalars + 8 * (size_t)G;                     // of whole blocks of 64 slices
+    int* err = reinterpret_cast<int*>(scalars + bp_mma_scalars(G) - 1);   // a wait gave up
     cudaMemsetAsync(scalars, 0, bp_mma_scalars(G) * sizeof(unsigned), st);
     k_bp_max<<<dim3((unsigned)std::min<size_t>((npos + 1023) / 1024, 512), G), 256, 0, st>>>(
         reinterpret_cast<const float4*>(q), top, npos);
     if (g.n_tiles_in > 0)
         for (int g0 = 0; g0 < G;) {
             const bool two = G - g0 > NS / 4;
-            if (!(two ? bp_pass<2>(g, G, g0, q, bins, top, scale, img, err, sms, st)
-                      : bp_pass<1>(g, G, g0, q, bins, top, scale, img, err, sms, st)))
+            if (!(two ? bp_pass<2>(g, G, g0, q, bins, top, scale, brief, img, err, sms, st)
+                      : bp_pass<1>(g, G, g0, q, bins, top, scale, brief, img, err, sms, st)))
                 return false;
             g0 += (two ? 2 : 1) * (NS / 4);
         }
     const int nt = (g.N + TP - 1) / TP, rest = nt * nt - g.n_tiles_in;
     if (rest > 0)
         k_bp_zero<<<rest, PIX, 0, st>>>(g.tiles_in + g.n_tiles_in, reinterpret_cast<float4*>(img), g.N, nt, G);
-    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, top, err);
+    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, top, brief, err);
     return true;
 }
 

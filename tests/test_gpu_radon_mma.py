@@ -221,3 +221,18 @@ def test_less_and_less_memory_and_enough_again():
     assert torch.equal(got, ref)
     assert torch.equal(t.radon(x), whole)
     t.close()
+
+
+@pytest.mark.parametrize("bright", [1e4, 1e6])
+def test_a_bright_pixel_takes_no_bits_from_other_rays(bright):
+    """The scale is a tile's: rays that miss a bright pixel but cross its tile are as accurate as without it."""
+    N, T, S = 209, 20, 48
+    th = axes(T)
+    x = torch.randn(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7))
+    x[5, 100, 60] = bright
+    spot = torch.zeros(4, N, N, device="cuda")
+    spot[:, 100, 60] = 1.0
+    got, ref = both(N, th, x)
+    with Tomography(N, th, 10) as t:
+        away = t.radon(spot)[0] == 0
+    assert rel(got[5][away], ref[5][away]) < 3e-6 and rel(got[5], ref[5]) < 3e-6
