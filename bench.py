@@ -58,63 +58,41 @@ def projector_variant(option, S):
     return 6 if 8 * ((G + 7) // 8) <= G + G // 8 else 5
 
 
-def tensor_projector(option, positions, S, N):
-    """Whether the library projects on the tensor cores (csrc/api.cu projector_variant)."""
-    groups = 7 if N >= 500 else 9 if N >= 250 else 12
-    return option == 7 and positions == 1 and (S + 3) // 4 >= groups and 200 <= N <= 4096
+def kernels_of(call):
+    """Names of the kernels that one call of a library operator launches, from a
+    stream capture of it after a call that has allocated what it needs."""
+    import ctypes
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
 
+    class Node(ctypes.Structure):      # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", ctypes.c_void_p), ("dims", ctypes.c_uint * 7), ("params", ctypes.c_void_p),
+                    ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
 
-def tensor_radon_launches(N, theta, S, sms=152):
-    """Kernels of one projection on the tensor cores (csrc/kernels_radon_mma.cu
-    mma_plan): per pass over slice blocks one layout kernel, per chunk of angle
-    groups a product and a reduction, and the flagged fallback."""
-    import numpy as np
-    nt, nblk = (N + 15) // 16, (S + 63) // 64
-    cost = [-(-nt * q // sms) * -(-nt // q) * (1 + 0.5 * ((6.0 * (-(-nt // q) - 1) + 22) / -(-nt // q)) / 22)
-            for q in range(1, nt + 1)]
-    stretches = 1 + int(np.argmin(cost))
-    a = np.pi * (np.asarray(theta, np.float64) - 90.0) / 180.0
-    c, s = np.abs(np.cos(a).astype(np.float32)), np.abs(np.sin(a).astype(np.float32))
-    nr = np.minimum(25, np.floor(np.float32(17) * (c + s) + np.float32(0.002)).astype(int) + 1)
-    length = -(-nt // stretches)
-    span = np.floor(16 * (length - 1) * np.minimum(c, s) + 0.01).astype(int) + 1 + nr
-    sides = []   # rows of the groups: angles along x, then the others
-    for side in (c >= s, c < s):
-        n, rows, groups, t = nr[side], span[side], [], 0
-        while t < len(n):
-            k = min(5, len(n) - t)
-            k = 4 if k == 5 and n[t + 4] > 24 else k
-            groups.append(int(rows[t:t + k].sum()))
-            t += k
-        sides.append(groups)
+    def ok(rc):
+        if rc != 0:
+            raise RuntimeError(f"CUDA driver call failed: {rc}")
 
-    def chunks(ng):
-        out = []
-        for g in sides:
-            k = -(-len(g) // ng)
-            out += [sum(g[i * len(g) // k:(i + 1) * len(g) // k]) for i in range(k)]
-        return out
-
-    units = nt * stretches
-    nb = min(nblk, 2)
-    if nb == 2 and units < 4 * sms:
-        nb = min(nblk, 2 * -(-4 * sms // units))
-    nb = nb & ~1 if nb > 2 else nb
-    ng = min(sum(map(len, sides)), max(1, (144 << 20) // (256 * 110 * min(sms, units) * min(nb, 2))))
-    while 256 * max(chunks(ng)) * units * nb > 4 << 30 and not (nb <= 2 and ng == 1):
-        nb, ng = (nb - 2, ng) if nb > 2 else (nb, ng - 1)
-    return 1 + -(-nblk // nb) * (1 + 2 * len(chunks(ng)))
-
-
-def iradon_launches(positions, S, N, T=T_ANG):
-    """Kernels of one filtered backprojection: the filter, then the gather
-    kernel, or on the tensor cores (csrc/kernels_bp_mma.cu) the largest
-    magnitudes, layout and product per pass of up to 128 slices, the tiles
-    outside the mask and the flagged fallback."""
-    groups = 16 if N < 800 and T < 60 else 12 if N < 300 else 10
-    if positions != 1 or (S + 3) // 4 < groups or N < 200:
-        return 2
-    return 1 + 1 + 2 * -(-S // 128) + 2
+    call()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        call()
+    graph, n = ctypes.c_void_p(g.raw_cuda_graph()), ctypes.c_size_t()
+    ok(cu.cuGraphGetNodes(graph, None, ctypes.byref(n)))
+    nodes = (ctypes.c_void_p * n.value)()
+    ok(cu.cuGraphGetNodes(graph, nodes, ctypes.byref(n)))
+    names = []
+    for node in nodes:
+        kind, p, name = ctypes.c_int(), Node(), ctypes.c_char_p()
+        ok(cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)))
+        if kind.value != 0:            # CU_GRAPH_NODE_TYPE_KERNEL
+            continue
+        ok(cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), ctypes.byref(p)))
+        ok(cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(p.func)) if p.func else
+           cu.cuKernelGetName(ctypes.byref(name), ctypes.c_void_p(p.kern)))
+        names.append(name.value.decode())
+    return names
 
 
 def radon_launches(variant, N):
@@ -832,9 +810,14 @@ def main():
     n_ew += NINNER * NCG if carried else 0          # the sinogram updates ruk += alpha radon(p)
     n_ew += 1 if carried_res else 0                 # iradon(fk - f) += iradon(f - radon(uk))
     variant = projector_variant(t.get_option(7), S)
-    tensor = tensor_projector(t.get_option(7), t.get_option(8), S, N)
-    per_radon = tensor_radon_launches(N, t.theta, S) if tensor else radon_launches(variant, N)
-    per_iradon = iradon_launches(t.get_option(8), S, N, T)
+    # the solver's operators are the public ones without the two layout conversions of a batch
+    img = torch.rand(S, N, N, device="cuda")
+    radon_names, iradon_names = kernels_of(lambda: t.radon(img)), kernels_of(lambda: t.iradon(f))
+    del img
+    torch.cuda.empty_cache()
+    layout = sum("k_to_lanes" in k or "k_from_lanes" in k for k in radon_names)
+    per_radon, per_iradon = len(radon_names) - layout, len(iradon_names) - layout
+    tensor = any("k_mma_project" in k for k in radon_names)
     kernel_launches = (per_radon * n_radon + per_iradon * n_iradon + n_ew) * args.steps + per_radon * n_full
     if carried_res:   # each refresh: two differences and two backprojections instead of the sum
         kernel_launches += n_full * (2 * per_iradon + 2 - 1)
@@ -945,7 +928,7 @@ def main():
         # the other hot kernel: the backprojection (8 bytes per update at L1 level)
         t_bp = cuda_time(lambda: t.backproject(f), 2)
         line["roofline_backprojection"] = {
-            "kernel": ("k_bp_mma (tensor cores" if iradon_launches(t.get_option(8), S, N, T) > 2 else
+            "kernel": ("k_bp_mma (tensor cores" if any("k_bp_mma" in k for k in iradon_names) else
                        "k_backproject_exact_ct<4, 1> (gathers") + "; tv_hpc.F90:107-123)", "launch_ms": 1000 * t_bp,
             "updates_per_s": N * N * T * S / t_bp,
             "l1_level": l1_level(8.0 * N * N * T * S / t_bp / 1e9, clocks, probe, bytes_per_update=8),
