@@ -6,6 +6,8 @@ Both round each sum to single precision in another order; a sum of up to 3 N
 terms of one sign stays within ~1e-6 of FP64 either way (the bar of
 test_operators_at_the_2049_grid is 5e-6), so they agree to 3e-6 in relative L2.
 """
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -180,6 +182,8 @@ def test_less_and_less_memory_and_enough_again():
     give way to what another call needs."""
     N, T, S = 513, 180, 64
     th = syn.angles(T)
+    gc.collect()
+    torch.cuda.empty_cache()         # so that every tensor here takes memory of its own
     x = torch.rand(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
 
     def fresh(variant):
@@ -196,7 +200,7 @@ def test_less_and_less_memory_and_enough_again():
     whole, most = fresh(7)
     lines, least = fresh(6)          # either counts the result's own memory
     assert not torch.equal(whole, lines) and most - least > 64 << 20
-    for room, want in ((most - (16 << 20), whole), (least + (16 << 20), lines)):
+    for room, want in ((most - (16 << 20), whole), (least + (24 << 20), lines)):
         torch.cuda.empty_cache()
         t = Tomography(N, th, 25)
         hold = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
