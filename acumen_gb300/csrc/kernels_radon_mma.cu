@@ -24,15 +24,13 @@
 // The order is kept by the four warps that send a block's rows: a ray's place in the
 // operand moves from tile to tile, so two tiles' rows of it may be in the hands of two warps, and
 // a bulk operation is known to have arrived only to the thread that issued it.
-// Twice a tile (each group, where there are few) every warp waits for its own and
-// all four meet before they send on: at the first group those of the tile before
-// but its last two groups have arrived, which covers the first two groups, at the third group
-// all of them.
+// Once a tile every warp waits until all that it sent has arrived, and the four meet
+// before the next tile's rows go out.
 //
 // Measured at 2049^2 x 1200 angles, 256 slices: 737 ms with the pixel-line
 // gathers, 217 ms with every tile's rows written and read (75 of them the
 // reduction at 80 % of the HBM bandwidth), now 168 ms, 20 of them the reduction (the
-// meetings of the warps 1.5 ms).  1025^2 x
+// meetings of the warps 1.5 ms, whether for all rows once a tile or at two groups for those two groups old).  1025^2 x
 // 600, 128 slices 14.7 / 12.0 ms, 64 slices 9.8 / 9.6 ms (23.4 with gathers).
 // What holds the products is shared memory: 14 KB of operands per K step of one
 // block (20 KB of two, which share W) and the stores of W and of the staged rows
@@ -397,13 +395,9 @@ __global__ void __launch_bounds__(32 * Roles<BLK>::WARPS, 1) k_mma_project(const
             ok = umma::bar_wait_warp(&sh.sc_full[b & 1], (b >> 1) & 1);
             const float4* const scale = reinterpret_cast<const float4*>(sm + L::SCALE + ((b & 1) * BLK + k) * SCALE_BYTES);
             for (int g = 0; g < ngroups; ++g, ++m) {
-                // all that the four warps sent has arrived, of five groups and more but the last two groups' (STEPS / 2 pieces each)
-                const bool meet = ngroups < 5 || g == 0 || g == 2;
+                const bool meet = g == 0;   // all that the four warps sent of the tile before has arrived
                 if (ok && meet) {
-                    if (lane < 4) {
-                        if (ngroups < 5) umma::bulk_store_wait<0>();
-                        else umma::bulk_store_wait<STEPS>();
-                    }
+                    if (lane < 4) umma::bulk_store_wait();
                     __syncwarp();
                     if (lane == 0) umma::bar_arrive(&sh.sent[k]);
                 }
