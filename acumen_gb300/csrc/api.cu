@@ -833,7 +833,8 @@ int tv_end(acu_ctx* c, Real* d_tv)
 // device memory that is free (plus what the context already holds for the
 // solver), else the largest multiple of 4 that does, capped by
 // ACU_OPT_MAX_BATCH.  Slices are independent, so a batch solved in chunks
-// gives each slice what one batch gives it.
+// gives each slice what one batch gives it, to the rounding of the operators that
+// a batch of that size takes.  The context's tables are there.
 template <typename Real>
 int tv_chunk(acu_ctx* c, int S, bool host_io)
 {
@@ -857,10 +858,19 @@ int tv_chunk(acu_ctx* c, int S, bool host_io)
     for (const DevBuf* b : {&st.f, &st.fk, &st.ruk, &st.rp, &st.q, &st.uk, &st.ukp, &st.dx, &st.dy, &st.bx, &st.by,
                             &st.rhs, &st.r, &st.p, &st.Ap, &st.tmp, &st.bd, &st.dacc})
         held += b->n;
-    // the tensor-core operators' partial sums and bins (of 128 slices) do not grow with the batch
-    size_t reserve = ((size_t)1 << 30) + totalb / 50;
-    if (sizeof(Real) == 4) reserve += (c->opt_projector == 7 ? MMA_PART_CAP : 0) + sizeof(float) * 128 * T * N;
-    const size_t avail = freeb + held > reserve ? freeb + held - reserve : 0;
+    const size_t reserve = ((size_t)1 << 30) + totalb / 50, room = freeb + held > reserve ? freeb + held - reserve : 0;
+    // the tensor-core operators' buffers hardly grow with the batch; where memory is
+    // short they take half of it at most, as the batch can do without them
+    size_t once = 0;
+    if constexpr (sizeof(Real) == 4) {
+        const int G = (S + 3) / 4;
+        if (pick_lanes(c, S, false) == 4 && mma_wanted(c, G)) {
+            const MmaPlan p = mma_plan(c->g32.d, G, MMA_PART_CAP);
+            once += p.tile_bytes + p.part_bytes;
+        }
+        if (pick_lanes(c, S, false) == 4 && bp_mma_wanted(c, G)) once += bp_mma_bins_bytes(c->N, c->T, G);
+    }
+    const size_t avail = room - std::min(once, room / 2);
     long long smax = (long long)(avail / per);
     if (smax >= 4) smax -= smax % 4;
     if (c->opt_max_batch > 0) smax = std::min<long long>(smax, c->opt_max_batch);
@@ -875,6 +885,7 @@ int tv_solve(acu_ctx* c, int S, const Real* d_f, int ninner, int nouter, int ncg
     if (S == 0) return ACU_OK;
     if (!d_f || !d_tv) return set_err(c, ACU_ERR_INVALID, "null array");
     if (nouter < 0) return set_err(c, ACU_ERR_INVALID, "iteration counts must be >= 0");
+    CKRET(ensure_geom<Real>(c));
     const int chunk = tv_chunk<Real>(c, S, false);
     const size_t nsino = (size_t)c->T * c->N, nimg = (size_t)c->N * c->N;
     for (int s0 = 0; s0 < S; s0 += chunk) {
@@ -980,6 +991,7 @@ int tv_host(acu_ctx* c, bool plain, int S, const float* f, int ninner, int noute
     CKRET(check_ctx(c, S));
     if (S == 0) return ACU_OK;
     if (!f || !tv) return set_err(c, ACU_ERR_INVALID, "null array");
+    CKRET(ensure_geom<float>(c));
     // chunks of slices that fit on the device (the per-slice path holds one
     // slice at a time, so only its copies count)
     const int chunk = plain ? std::max(1, std::min(S, c->opt_max_batch > 0 ? c->opt_max_batch : S))

@@ -101,7 +101,8 @@ int acu_set_stream(acu_ctx *ctx, void *cuda_stream);
 #define ACU_OPT_MAX_BATCH 13  /* acu_tvopt / acu_tvopt_dev / acu_tvopt_plain: at most this many slices on
                                  the device at a time (0, default: as many as fit in the free device
                                  memory); larger calls are solved in consecutive chunks of slices, each
-                                 slice as in one batch */
+                                 slice as in one batch to single-precision rounding (the same bits where
+                                 batch and chunk take the same operators, see 7 and 10) */
 #define ACU_OPT_BP_STAGED 14  /* exact single-precision backprojection with the angle table in the launch
                                  parameters: 1 stages each angle's sinogram bins of a 32x8 pixel tile in
                                  shared memory with bulk copies (cp.async.bulk, double-buffered, mbarrier

@@ -323,3 +323,23 @@ def test_no_problem_is_active_after_a_refused_one(built_lib):
         ref, _ = fresh.tvopt(f[:4], 1, 1, 2, 0.05, 1.0)
     assert torch.equal(t.tv_end(), ref)
     t.close()
+
+
+def test_a_small_batch_stays_whole_where_memory_is_short(built_lib):
+    """Room for the tensor-core operators is set aside only as far as the problem takes them: 20 slices of 257^2 need 73 MB."""
+    N, T, S = 257, 90, 20
+    f = torch.stack([syn.normalised_sinogram(syn.random_ellipses(s, 0.3 * N), N, syn.angles(T), I0=5e3, seed=s, device="cuda")
+                     for s in range(S)])
+    with Tomography(N, syn.angles(T), 12) as t:
+        ref, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+    torch.cuda.empty_cache()
+    free, total = torch.cuda.mem_get_info()
+    t = Tomography(N, syn.angles(T), 12)
+    # what the solver leaves to others, and 1 GB
+    hold = torch.empty(free - (1 << 30) - total // 50 - (1 << 30), dtype=torch.uint8, device="cuda")
+    tv, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+    assert torch.equal(tv, ref)
+    t.set_option(13, 1)
+    one, _ = t.tvopt(f, 1, 2, 2, 0.05, 1.0)
+    assert not torch.equal(one, ref)         # slice by slice takes other operators
+    t.close()
