@@ -178,9 +178,16 @@ int need(acu_ctx* c, DevBuf& b, size_t bytes)
     return ACU_OK;
 }
 
-// Whether so many more bytes than the buffers hold can be had.
-bool room_for(size_t bytes, std::initializer_list<const DevBuf*> held)
+// Whether so many more bytes than the buffers hold can be had (not while the
+// caller captures the stream, which allows no allocation).
+bool room_for(acu_ctx* c, size_t bytes, std::initializer_list<const DevBuf*> held)
 {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return false;
     size_t freeb = 0, totalb = 0, have = 0;
     for (const DevBuf* b : held) have += b->n;
     return cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && bytes <= freeb + have;
@@ -217,7 +224,7 @@ int ensure_backproject_buffers(acu_ctx* c, int G)
 {
     if (!bp_mma_wanted(c, G)) return ACU_OK;
     const size_t bytes = bp_mma_bins_bytes(c->N, c->T, G);
-    if (!c->bp_room && !room_for(bytes, {&c->bpQ})) return ACU_OK;
+    if (!c->bp_room && !room_for(c, bytes, {&c->bpQ})) return ACU_OK;
     cudaError_t e = c->bpQ.ensure(bytes);
     if (e == cudaSuccess) e = c->bpS.ensure(sizeof(unsigned) * bp_mma_scalars(G));
     c->bp_room = e == cudaSuccess;
@@ -313,7 +320,7 @@ int ensure_mma_buffers(acu_ctx* c, int G)
 {
     const DevGeom<float>& g = c->g32.d;
     const MmaPlan whole = mma_plan(g, G, MMA_PART_CAP);
-    if (c->mma_cap == MMA_PART_CAP || room_for(whole.tile_bytes + whole.part_bytes, {&c->mmaT, &c->mmaP}))
+    if (c->mma_cap == MMA_PART_CAP || room_for(c, whole.tile_bytes + whole.part_bytes, {&c->mmaT, &c->mmaP}))
         c->mma_cap = MMA_PART_CAP;
     while (c->mma_cap > 0) {
         const MmaPlan p = c->mma_cap == MMA_PART_CAP ? whole : mma_plan(g, G, c->mma_cap);

@@ -240,3 +240,28 @@ def test_a_bright_pixel_takes_no_bits_from_other_rays(bright):
     with Tomography(N, th, 10) as t:
         away = t.radon(spot)[0] == 0
     assert rel(got[5][away], ref[5][away]) < 3e-6 and rel(got[5], ref[5]) < 3e-6
+
+
+def test_capture_of_a_call_that_found_no_memory_before():
+    """The tensor-core projector is not tried again while its stream is captured: it would have to allocate."""
+    N, T, S = 513, 180, 64
+    gc.collect()
+    torch.cuda.empty_cache()
+    x = torch.rand(S, N, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    t = Tomography(N, syn.angles(T), 25)
+    t.set_option(7, 6)
+    lines = t.radon(x)               # with the gathers' buffers
+    t.set_option(7, 7)
+    out = t.radon(x[:4])             # leaves torch a block; the result below takes one of 24 MB
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    got = t.radon(x)
+    del hold, out
+    torch.cuda.empty_cache()
+    assert torch.equal(got, lines)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        got = t.radon(x)
+    g.replay()
+    assert torch.equal(got, lines)
+    assert not torch.equal(t.radon(x), lines)
+    t.close()
