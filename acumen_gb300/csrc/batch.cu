@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(512) k_batch_backproject(const ProbDesc* __res
     }
 }
 
-// Exact positions: the same items, R pixel rows a thread, bins as pairs (fixed.cuh).
+// Exact positions: the same items, R pixel rows a thread, bins as pairs (fixed.cuh).  The tuner may choose tiles of 16
+// or 32 rows: positions are formed for 16 at a time in either.
 template <int R>
 __global__ void __launch_bounds__(512) k_batch_backproject_fx(const ProbDesc* __restrict__ pd, int nprob,
                                                               const float2* __restrict__ q, float* __restrict__ img,
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(512) k_batch_backproject_fx(const ProbDesc* __
                                                               int* counter)
 {
     __shared__ int s_it;
-    __shared__ int4 tab[FX_CHUNK];
+    __shared__ int4 tab[2 * FX_CHUNK];
     for (;;) {
         if (threadIdx.x == 0 && threadIdx.y == 0) s_it = atomicAdd(counter, 1);
         __syncthreads();
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(512) k_batch_backproject_fx(const ProbDesc* __
             cm[r] = x < N && y + r < N ? cmask[d.cm + (size_t)(y + r) * N + x] : 0.f;
             any |= cm[r] != 0.f;
         }
-        if (__syncthreads_or(any)) fx_backproject<R>(q + d.sino, xsc + d.sc / 2, N, d.T, d.mid, x0, y0, tab, v);
+        if (__syncthreads_or(any)) fx_backproject<R, 16>(q + d.sino, xsc + d.sc / 2, N, d.T, d.mid, x0, y0, tab, v);
 #pragma unroll
         for (int r = 0; r < R; ++r)
             if (x < N && y + r < N) img[d.img + (size_t)(y + r) * N + x] = cm[r] != 0.f ? cm[r] * v[r] : 0.f;

@@ -148,27 +148,31 @@ __device__ __forceinline__ float fx_ray(const float2* __restrict__ base, int N, 
 // tapped.  Per angle the position of the tile's middle pixel is formed once per
 // block (split tables, common.cuh) and kept with 26 fraction bits; the pixels'
 // positions follow by additions.  |position - middle| < 32 bins: the tile is at
-// most 32 pixels high.
+// most 32 pixels high.  FH > 0: every FH rows have a middle of their own, so that the
+// bits do not depend on the tile's height.
 constexpr int FX_CHUNK = 256;   // angles whose entries are held in shared memory
 
-template <int R>
+template <int R, int FH = 0>
 __device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, const float4* __restrict__ xsc, int N,
                                                int T, float mid, int x0, int y0, int4* tab, float (&out)[R])
 {
-    const int tid = threadIdx.y * 32 + threadIdx.x, nthreads = 32 * blockDim.y, h = R * blockDim.y / 2;
-    const int lx = (int)threadIdx.x - 16, ly = (int)threadIdx.y * R - h;
+    const int tid = threadIdx.y * 32 + threadIdx.x, nthreads = 32 * blockDim.y, height = R * blockDim.y;
+    const int fh = FH ? FH : height, frame = FH ? (int)threadIdx.y * R / fh : 0;
+    const int lx = (int)threadIdx.x - 16, ly = (int)threadIdx.y * R - frame * fh - fh / 2;
+    const int4* const mine = tab + frame * FX_CHUNK;
 #pragma unroll
     for (int r = 0; r < R; ++r) out[r] = 0.f;
     for (int t0 = 0; t0 < T; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, T - t0);
         __syncthreads();
+        for (int f = 0; f * fh < height; ++f)
         for (int a = tid; a < n; a += nthreads) {
             const float4 x = __ldg(xsc + t0 + a);
             float cell, frac;
-            exact_coord(x.x, x.y, x.z, x.w, (float)(x0 + 16) - mid, (float)(y0 + h) - mid, mid, cell, frac);
+            exact_coord(x.x, x.y, x.z, x.w, (float)(x0 + 16) - mid, (float)(y0 + f * fh + fh / 2) - mid, mid, cell, frac);
             constexpr float ONE = 67108864.f;   // 2^26
             // cell - 1: the pair's index; 4: half of the fraction's last kept bit
-            tab[a] = make_int4((int)(frac * ONE) + 4, (int)(x.x * ONE) + __float2int_rn(x.z * ONE),
+            tab[f * FX_CHUNK + a] = make_int4((int)(frac * ONE) + 4, (int)(x.x * ONE) + __float2int_rn(x.z * ONE),
                                (int)(x.y * ONE) + __float2int_rn(x.w * ONE), (int)cell - 1);
         }
         __syncthreads();
@@ -176,7 +180,7 @@ __device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, con
         // a block's first touch of an angle's bins comes from L2: 32 loads in flight per thread
 #pragma unroll (32 / R)
         for (int a = 0; a < n; ++a, row += N) {
-            const int4 e = tab[a];
+            const int4 e = mine[a];
             int p = e.x + lx * e.y + ly * e.z;
 #pragma unroll
             for (int r = 0; r < R; ++r) {

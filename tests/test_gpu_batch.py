@@ -167,3 +167,24 @@ def test_memory_of_a_batch():
     # masks, results (2), 7 images that live on, 4 in turns; inputs, 4 sinograms that live on
     assert taken < 14 * images + 5 * sinos + 32e6
     b.close()
+
+
+def test_bits_do_not_depend_on_the_tuning():
+    """The tuner picks tiles by timing them, small ones for small batches: a problem's images are the same, bit for bit,
+    alone and in any company."""
+    spec = [(97, 60), (257, 180), (725, 300)]
+    rng = np.random.default_rng(3)
+    sinos = [rng.standard_normal((T, N)).astype(np.float32) for N, T in spec]
+    want = [None] * len(spec)
+    for copies in (1, 2, 8, 40):
+        for pick in ([0], [1], [2], [0, 1], [0, 1, 2]):
+            many = [k for k in pick for _ in range(copies)]
+            b = RaggedBatch([spec[k][0] for k in many], [syn.angles(spec[k][1]) for k in many], 4)
+            img = b.iradon([sinos[k] for k in many])
+            tv, _ = b.tvopt([sinos[k] for k in many], 1, 1, 1, 0.05, 1.0)
+            b.close()
+            for k, a, u in zip(many, img, tv):
+                if want[k] is None:
+                    want[k] = (a, u)
+                np.testing.assert_array_equal(a, want[k][0])
+                np.testing.assert_array_equal(u, want[k][1])
