@@ -132,7 +132,7 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
 // (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
 // the derivative with respect to them or null; launch_backproject_fx: q as pairs
 // (bin, next bin), which the filter writes or launch_pairs makes from
-// n = slices * T * N bins; launch_adjoint_fx: the projector's exact transpose.
+// n = slices * T * N bins; launch_adjoint_fx: the projector's transpose.
 // Their buffers of pairs hold 1 GB at most, as many slices as that takes: slices
 // at once of so many bytes each, and the floats of a projector's buffer.
 inline int pair_slices(size_t bytes, int S)

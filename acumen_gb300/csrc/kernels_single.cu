@@ -1,6 +1,6 @@
 // Kernels that carry one slice per thread at exact positions: projector
 // (tomography/tv_hpc.F90:129-159) with its offset derivative, filtered
-// backprojection's second half (:107-123), and the projector's exact transpose.
+// backprojection's second half (:107-123), and the projector's transpose.
 // Batches share a sample position among four slices or more; here the position
 // is most of the work, so it is kept in fixed point (fixed.cuh).
 #include <algorithm>
@@ -160,7 +160,8 @@ __device__ __forceinline__ void put_image(float* __restrict__ img, Lanes<float, 
     st_lanes<float, V>(img + (g * N * N + (size_t)(py - 1) * N + (px - 1)) * V, acc);
 }
 
-// Exact transpose of the projector, as a gather over the angles: the at most
+// Transpose of the projector (at positions 5e-7 px from its own, but on the
+// rim), as a gather over the angles: the at most
 // three rays whose samples read the pixel, each with the sum of its samples'
 // weights there.  The general kernel (k_radon_adjoint) evaluates the projector at
 // 16 candidate samples per pixel and angle; this one evaluates the nine bilinear

@@ -75,7 +75,8 @@ int acu_set_stream(acu_ctx *ctx, void *cuda_stream);
                                  the batch fills its 32-slice lines to 8/9 or more, else 5; 1 and 3 to
                                  6 give identical results */
 #define ACU_OPT_POSITIONS 8   /* single-precision sample positions: 1 exact (default; coordinates from split
-                                 FP64 angle tables, within ~1e-7 px of FP64, and the FFT filter's spectrum
+                                 FP64 angle tables, within ~1e-7 px of FP64, or in fixed point, single
+                                 slices, ragged batches and the adjoint, within 5e-7 px; the FFT filter's spectrum
                                  from FP64-evaluated taps: the mode that meets relL2 1e-5 FBP / 1e-4 TV
                                  against FP64 at the benchmark sizes), 0 the reference's single-precision
                                  arithmetic (tv_hpc.F90:53-56,113-115,144-146), whose rounding of the
@@ -86,9 +87,10 @@ int acu_set_stream(acu_ctx *ctx, void *cuda_stream);
                                  outer iterations (default; as 1 when radon(uk) is not carried),
                                  1 one backprojection of fk - radon(uk), or 0 the reference's two */
 #define ACU_OPT_BP_GROUPS 10  /* 4-slice groups per backprojection thread: 0 auto (default: exact positions,
-                                 37 slices or more and a side of 200 or more on the tensor cores, the
-                                 same sums to single-precision rounding; else 1 with the angle table in
-                                 the launch parameters, else 2 where the groups divide), 1, 2 or 4; the
+                                 37 slices or more (45 at sides below 300, 61 with fewer than 60 angles
+                                 below 800) and a side of 200 or more on the tensor cores, the same
+                                 sums to single-precision rounding; else 1 with the angle table in the
+                                 launch parameters, else 2 where the groups divide), 1, 2 or 4; the
                                  groups share the angle's table entry and sample position, the sums are
                                  the same for 1, 2 and 4 */
 #define ACU_OPT_RADON_REFRESH 11 /* batched TV: radon(uk) for the Bregman update recomputed every outer
@@ -116,8 +118,9 @@ int acu_get_option(const acu_ctx *ctx, int option, int *value);
  *   the tapered mask.  sino: S*T*N, img: S*N*N.  Also get_slice
  *   (tv_hpc.F90:365-386, fbp_hpc.F90:129-150), which is iradon with copies.
  * acu_radon: tomography/tv_hpc.F90:129-159 (radon) -- bilinear ray sums / N.
- * acu_radon_adjoint: exact transpose of acu_radon (new; not in the reference):
- *   <radon(x), y> = <x, radon_adjoint(y)> up to round-off.
+ * acu_radon_adjoint: transpose of acu_radon (new; not in the reference):
+ *   <radon(x), y> = <x, radon_adjoint(y)> up to round-off and, in single precision at
+ *   exact positions, that of the positions (5e-7 px).
  * acu_filter_dev / acu_backproject_dev: the two halves of iradon
  *   (tv_hpc.F90:93-105 and :107-123).                                         */
 int acu_iradon(acu_ctx *ctx, int nslices, const float *sino, float *img);
