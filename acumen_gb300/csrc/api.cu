@@ -238,10 +238,10 @@ int ensure_backproject_buffers(acu_ctx* c, int G)
 }
 
 template <typename Real, int V>
-void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q, Real* img)
+void lanes_backproject(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* q, bool filtered, Real* img)
 {
     if constexpr (V == 4 && sizeof(Real) == 4) {
-        if (bp_mma(c, G) && launch_backproject_mma(g, G, q, c->bpQ.p, c->bpS.as<unsigned>(), img, c->stream)) return;
+        if (bp_mma(c, G) && launch_backproject_mma(g, G, q, filtered, c->bpQ.p, c->bpS.as<unsigned>(), img, c->stream)) return;
     }
     launch_backproject<Real, V>(g, G, q, img, c->stream);
 }
@@ -282,7 +282,7 @@ void lanes_iradon(acu_ctx* c, const DevGeom<Real>& g, int G, const Real* sino, R
         }
     }
     lanes_filter<Real, V>(c, g, G, sino, q);
-    lanes_backproject<Real, V>(c, g, G, q, img);
+    lanes_backproject<Real, V>(c, g, G, q, true, img);
 }
 
 enum OpKind { OP_IRADON, OP_RADON, OP_RADON_ADJ, OP_FILTER, OP_BACKPROJECT };
@@ -438,7 +438,7 @@ int run_op_v(acu_ctx* c, OpKind op, int S, const Real* in, Real* out)
                 break;
             }
         }
-        lanes_backproject<Real, V>(c, g, G, lin, lout);
+        lanes_backproject<Real, V>(c, g, G, lin, false, lout);
         break;
     }
     CKLAUNCH(c);

@@ -121,13 +121,14 @@ MmaPlan mma_plan(const DevGeom<float>& g, int G, size_t cap);
 void launch_radon_mma(const DevGeom<float>& g, int G, const float* img, unsigned char* tiles, float* P, int* flags,
                       const MmaPlan& p, float* sino, cudaStream_t st);
 // Backprojection on the tensor cores (kernels_bp_mma.cu; exact positions): work
-// buffers of bp_mma_bins_bytes bytes and bp_mma_scalars words.  False if the
+// buffers of bp_mma_bins_bytes bytes and bp_mma_scalars words.  filtered: q comes
+// from this library's filter.  False if the
 // driver has no tensor maps (nothing usable was written).
 int bp_tiles(const float* cmask, int N, std::vector<int>& list);
 size_t bp_mma_bins_bytes(int N, int T, int G);
 size_t bp_mma_scalars(int G);
-bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
-                            cudaStream_t st);
+bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, bool filtered, void* bins, unsigned* scalars,
+                            float* img, cudaStream_t st);
 // Single-slice kernels at exact positions (kernels_single.cu).  launch_radon_fx
 // (sides up to FX_MAX_SIDE); launch_ray_off: with per-angle offsets or null, dsino
 // the derivative with respect to them or null; launch_backproject_fx: q as pairs

@@ -381,7 +381,7 @@ __device__ __forceinline__ int scale_exp(unsigned top)
 
 // One bin and angle per thread (grid.x: 128 bins of every angle, of which there may be more than a grid has
 // rows): its 64 slices of block blockIdx.y as eight pieces of hi and eight of lo halves.  A half ends at 2^-24, so a value
-// below 2^-16 of its slice's largest keeps fewer than 23 bits: brief counts those of each slice (one in 10^4 as a rule).
+// keeps 23 bits down to 2^-16 of its slice's largest and 19 down to 2^-20: brief counts the values below that.
 __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, const unsigned* __restrict__ top,
                                                  float* __restrict__ scale, unsigned* __restrict__ brief,
                                                  uint4* __restrict__ bins, int N, int T, int G, int g0)
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(128) k_bp_bins(const float4* __restrict__ q, c
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float s = f[j] * __int_as_float((14 - scale_exp(b[j]) + 127) << 23);
-                if (s != 0.f && fabsf(s) < 0.25f) few |= 1ull << (8 * c + 4 * e + j);
+                if (s != 0.f && fabsf(s) < 0x1p-6f) few |= 1ull << (8 * c + 4 * e + j);
                 hi[4 * e + j] = __float2half_rn(s);
                 lo[4 * e + j] = __float2half_rn(s - __half2float(hi[4 * e + j]));
             }
@@ -443,17 +443,20 @@ __global__ void __launch_bounds__(PIX) k_bp_zero(const int* __restrict__ list, f
 }
 
 // The slices that held a value that is not finite by plain gathers (as k_backproject_exact): a slice is a column of the
-// product, which spreads such a value over its tiles and no further; and the slices of which a quarter of the values keep
-// fewer bits than the others, because a few are more than 2^16 times larger (one such slice of 256 at
+// product, which spreads such a value over its tiles and no further; and, in bins that no filter of this library
+// made, the slices of which more than half of the values are below 2^-20 of the largest.  (Where a filter did, the row of
+// the largest value holds that value's rounding, some 2^-28 of it in every bin, which is more in every pixel than the
+// 2^-40 lost here; and the filter's tails of a small object alone go below 2^-20.)  (One such slice of 256 at
 // 2049^2 x 1200: 8 ms, after 81).  NaN in all of the image if a wait gave up.
 __global__ void __launch_bounds__(256) k_bp_flagged(const float* __restrict__ q, const float* __restrict__ cmask,
                                                     const float4* __restrict__ xsc, float* __restrict__ img, int N,
                                                     int T, int G, float mid, const unsigned* __restrict__ top,
-                                                    const unsigned* __restrict__ brief, const int* __restrict__ err)
+                                                    const unsigned* __restrict__ brief, bool filtered,
+                                                    const int* __restrict__ err)
 {
     const bool lost = *err != 0;
-    const size_t quarter = (size_t)T * N / 4;
-    auto wanted = [&](int s) { return lost || top[s] >= 0x7f800000u || brief[s] > quarter; };
+    const size_t half = (size_t)T * N / 2;
+    auto wanted = [&](int s) { return lost || top[s] >= 0x7f800000u || (!filtered && brief[s] > half); };
     bool any = false;
     for (int i = threadIdx.x; i < 4 * G; i += 256) any |= wanted(i);
     if (!__syncthreads_or(any)) return;
@@ -550,8 +553,8 @@ size_t bp_mma_bins_bytes(int N, int T, int G)
 }
 size_t bp_mma_scalars(int G) { return (size_t)8 * G + (G * 4 + NS - 1) / NS * NS + 1; }
 
-bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void* bins, unsigned* scalars, float* img,
-                            cudaStream_t st)
+bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, bool filtered, void* bins, unsigned* scalars,
+                            float* img, cudaStream_t st)
 {
     const size_t npos = (size_t)g.T * g.N;
     int sms = 0, dev = 0;
@@ -575,7 +578,7 @@ bool launch_backproject_mma(const DevGeom<float>& g, int G, const float* q, void
     const int nt = (g.N + TP - 1) / TP, rest = nt * nt - g.n_tiles_in;
     if (rest > 0)
         k_bp_zero<<<rest, PIX, 0, st>>>(g.tiles_in + g.n_tiles_in, reinterpret_cast<float4*>(img), g.N, nt, G);
-    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, top, brief, err);
+    k_bp_flagged<<<sms * 8, 256, 0, st>>>(q, g.cmask, g.xsc_bp, img, g.N, g.T, G, g.mid, top, brief, filtered, err);
     return true;
 }
 
