@@ -157,7 +157,7 @@ __device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, con
                                                int T, float mid, int x0, int y0, int4* tab, float (&out)[R])
 {
     const int tid = threadIdx.y * 32 + threadIdx.x, nthreads = 32 * blockDim.y, height = R * blockDim.y;
-    const int fh = FH ? FH : height, frame = FH ? (int)threadIdx.y * R / fh : 0;
+    const int fh = FH ? FH : height, frames = FH ? height / FH : 1, frame = FH ? (int)threadIdx.y * R / fh : 0;
     const int lx = (int)threadIdx.x - 16, ly = (int)threadIdx.y * R - frame * fh - fh / 2;
     const int4* const mine = tab + frame * FX_CHUNK;
 #pragma unroll
@@ -165,7 +165,7 @@ __device__ __forceinline__ void fx_backproject(const float2* __restrict__ q, con
     for (int t0 = 0; t0 < T; t0 += FX_CHUNK) {
         const int n = min(FX_CHUNK, T - t0);
         __syncthreads();
-        for (int f = 0; f * fh < height; ++f)
+        for (int f = 0; f < frames; ++f)
         for (int a = tid; a < n; a += nthreads) {
             const float4 x = __ldg(xsc + t0 + a);
             float cell, frac;
